@@ -79,6 +79,8 @@ struct dm_graph {
   uint64_t idx_units = 0;             // 16-byte units of the whole index
   int32_t idx_maxd = 0;               // largest out-degree with a block
   std::vector<int32_t> up_order;      // motif roots by descending upper degree
+  std::vector<int32_t> udeg;          // undirected degree by rank (census)
+  int32_t n_deg01 = 0;                // vertices of degree 0 or 1: the lowest ranks
   std::vector<void*> pinned;          // host arrays registered with the CUDA driver
   // device copies
   std::mutex mu;

@@ -45,6 +45,9 @@ struct Workspace {
   size_t per_root_cap = 0;
   int32_t* d_parts = nullptr;       // scheduler part words, parallel to the task list
   size_t parts_cap = 0;
+  unsigned char* d_census = nullptr;  // census: sums, vertex list, edge array
+  size_t census_cap = 0;
+  unsigned long long* h_census = nullptr;  // pinned: the sums read back
   uint32_t* d_bits = nullptr;       // motif membership bitmaps, all zero between calls
   size_t bits_cap = 0;
   RootDesc* d_desc = nullptr;       // task list of a call on the clique index
@@ -120,6 +123,10 @@ struct DeviceSlot {
   // cliques) by original id, and the rank -> original id map of the DAG
   float* d_feat[2] = {nullptr, nullptr};
   int32_t* d_orig = nullptr;
+  // census (k = 3, 4 motifs): degrees by rank, and the DAG's in-lists
+  int32_t* d_udeg = nullptr;
+  int32_t *d_in_end = nullptr, *d_in_deg = nullptr;
+  void* d_in = nullptr;
 };
 
 static std::mutex g_dev_mu;
@@ -315,6 +322,7 @@ static void free_workspace(Workspace& w) {
   cudaFree(w.d_bits);
   cudaFree(w.d_desc);
   cudaFree(w.d_params);
+  cudaFree(w.d_census);
   cudaFree(w.d_sched);
   cudaFree(w.d_sroots);
   cudaFree(w.d_sparts);
@@ -329,6 +337,7 @@ static void free_workspace(Workspace& w) {
   w = Workspace();
 }
 
+  if (w.h_census) cudaFreeHost(w.h_census);
 static DeviceSlot* slot_for(dm_graph* g, int dev) {
   for (auto* p : g->dev)
     if (p->device == dev) return reinterpret_cast<DeviceSlot*>(p);
@@ -535,7 +544,7 @@ void release_device_graphs(dm_graph* g) {
       for (void* p : {(void*)s->dg.d_row, (void*)s->dg.d_deg, (void*)s->dg.d_adj, (void*)s->dg.d_orow,
                       (void*)s->dg.d_odeg, (void*)s->dg.d_oadj, (void*)s->d_deg_order, (void*)s->d_up_order,
                       s->d_blocks, (void*)s->d_boff, (void*)s->d_desc_deg, (void*)s->d_feat[0], (void*)s->d_feat[1],
-                      (void*)s->d_orig})
+                      (void*)s->d_orig, (void*)s->d_udeg, (void*)s->d_in_end, (void*)s->d_in_deg, s->d_in})
         gbuf_free(p, dv);
       {
         std::lock_guard<std::mutex> lk(g_dev_mu);
@@ -1173,6 +1182,51 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
   if (!s->dg.has_oriented && (rc = upload_clique_image(g, s, ctx.stream))) return rc;
   if (!s->dg.has_undirected) {
     rc = upload_csr(g, g->row, g->adj, g->n, g->pad_row[0], g->pad_deg[0], g->pad_adj[0], &s->dg.d_row, &s->dg.d_deg,
+// Device arrays of the census: degrees by rank, and for k = 4 the in-lists (laid out on the
+// first call of a device copy). Returns 1 when the device has no room for them.
+static int ensure_census(dm_graph* g, DeviceSlot* s, int k, LaunchCtx& ctx) {
+  const size_t n = (size_t)std::max(g->n, 1);
+  if (!s->d_udeg) {
+    if (g->udeg.empty()) {
+      g->udeg.assign(n, 0);
+      g->n_deg01 = 0;
+      for (int32_t v = 0; v < g->n; ++v) {
+        const int32_t d = (int32_t)(g->row[v + 1] - g->row[v]);
+        g->udeg[g->rank[v]] = d;
+        g->n_deg01 += d < 2;
+      }
+      pin_host(g, g->udeg.data(), sizeof(int32_t) * n);
+    }
+    if (gbuf_alloc(reinterpret_cast<void**>(&s->d_udeg), sizeof(int32_t) * n) != cudaSuccess) {
+      cudaGetLastError();
+      s->d_udeg = nullptr;
+      return 1;
+    }
+    DM_CUDA(cudaMemcpyAsync(s->d_udeg, g->udeg.data(), sizeof(int32_t) * n, cudaMemcpyHostToDevice, ctx.stream));
+  }
+  if (k == 3 || s->d_in) return DM_OK;
+  int32_t *end = nullptr, *deg = nullptr;
+  void* in = nullptr;
+  cudaError_t e = gbuf_alloc(reinterpret_cast<void**>(&end), sizeof(int32_t) * n);
+  if (e == cudaSuccess) e = gbuf_alloc(reinterpret_cast<void**>(&deg), sizeof(int32_t) * n);
+  if (e == cudaSuccess) e = gbuf_alloc(&in, 8 * (size_t)std::max<int64_t>(g->m, 1));
+  const int rc = e == cudaSuccess
+                     ? census_in_lists(GraphView{s->dg.d_orow, s->dg.d_odeg, s->dg.d_oadj, g->n}, end, deg, in,
+                                       reinterpret_cast<int*>(s->ws.d_ctr), ctx)
+                     : 1;
+  if (rc) {
+    cudaGetLastError();
+    gbuf_free(end, ctx.device);
+    gbuf_free(deg, ctx.device);
+    gbuf_free(in, ctx.device);
+    return rc;
+  }
+  s->d_in_end = end;
+  s->d_in_deg = deg;
+  s->d_in = in;
+  return DM_OK;
+}
+
                     &s->dg.d_adj, ctx.stream);
     if (rc) return rc;
     s->dg.has_undirected = true;
@@ -1293,6 +1347,73 @@ int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_
     s->n_up = (int)order.size();
   }
   std::vector<int32_t> roots, parts;
+// k = 3, 4 class counts by the census (census.cu) instead of the enumeration. Returns 1, having
+// counted nothing, when the graph has no complete clique index (roots above 256 out-neighbours,
+// or over the memory budget), so that the caller enumerates.
+static int motif_census(dm_graph* g, int k, const dm_dictionary* dict, const int32_t* cls, const dm_opts* o,
+                        LaunchCtx& ctx, uint64_t* class_counts, dm_stats* st) {
+  std::lock_guard<std::mutex> lk(g->mu);
+  ensure_oriented(g);
+  if (g->max_out_degree > INDEX_MAX_DEGREE) return 1;
+  DeviceSlot* s = slot_for(g, ctx.device);
+  Workspace& ws = s->ws;
+  int rc;
+  if ((rc = prepare_ws(ws, ctx.stream))) return rc;
+  DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
+  if (!s->dg.has_oriented && (rc = upload_clique_image(g, s, ctx.stream))) return rc;
+  if ((rc = ensure_index(g, s, ctx))) return rc;
+  if (s->index_state != 1) return 1;
+  if ((rc = ensure_census(g, s, k, ctx))) return rc;
+  const size_t list_off = (CENSUS_BYTES + 255) / 256 * 256;
+  const size_t up_off = list_off + (k == 4 ? (sizeof(int) * (size_t)g->n + 255) / 256 * 256 : 0);
+  const size_t bytes = up_off + (k == 4 ? sizeof(uint32_t) * g->img_adj_ints : 0);
+  if ((rc = ensure_ws_bytes(reinterpret_cast<void**>(&ws.d_census), &ws.census_cap, bytes))) return rc;
+  if (!ws.h_census) DM_CUDA(cudaMallocHost(&ws.h_census, CENSUS_BYTES));
+  CensusLaunch L;
+  L.g = GraphView{s->dg.d_orow, s->dg.d_odeg, s->dg.d_oadj, g->n};
+  L.k = k;
+  L.blocks = s->d_blocks;
+  L.boff = s->d_boff;
+  L.ud = s->d_udeg;
+  L.order = s->d_deg_order;
+  L.n_wide = 32 < (int)g->cnt_ge.size() ? (int)g->cnt_ge[32] : 0;
+  L.base = g->n_deg01;
+  L.wide_counters = g->max_degree >= 65536;
+  L.in_end = s->d_in_end;
+  L.in_deg = s->d_in_deg;
+  L.in = s->d_in;
+  L.sums = reinterpret_cast<unsigned long long*>(ws.d_census);
+  L.list = reinterpret_cast<int*>(ws.d_census + list_off);
+  L.up = reinterpret_cast<uint32_t*>(ws.d_census + up_off);
+  L2Window l2;
+  if (o && (o->flags & DM_FLAG_L2_PERSIST) && (rc = l2.begin(ctx.device, ctx.stream, s->d_blocks, s->index_bytes)))
+    return rc;
+  DM_CUDA(cudaEventRecord(ws.k0, ctx.stream));
+  if ((rc = census_launch(L, ctx))) return rc;
+  DM_CUDA(cudaEventRecord(ws.k1, ctx.stream));
+  DM_CUDA(cudaMemcpyAsync(ws.h_census, ws.d_census, CENSUS_BYTES, cudaMemcpyDeviceToHost, ctx.stream));
+  DM_CUDA(cudaStreamSynchronize(ctx.stream));
+  uint64_t sums[CENSUS_SUMS], types[6];
+  for (int i = 0; i < CENSUS_SUMS; ++i) sums[i] = ws.h_census[i];
+  census_classes(k, sums, types);
+  std::memset(class_counts, 0, sizeof(uint64_t) * dict->n_classes);
+  for (int t = 0; t < (k == 3 ? 2 : 6); ++t) class_counts[cls[t]] += types[t];
+  if (st) {
+    float kms = 0, pms = 0;
+    cudaEventElapsedTime(&kms, ws.k0, ws.k1);
+    cudaEventElapsedTime(&pms, ws.ev0, ws.k0);
+    std::memset(st, 0, sizeof(*st));
+    st->kernel_ms = kms;
+    st->prep_ms = pms;
+    st->tasks = (uint64_t)g->n;
+    st->mode_used = DM_MODE_BITMAP;
+    st->vwarp_used = 32;
+    st->block = 256;
+    st->kernel_launches = ctx.launches;
+  }
+  return DM_OK;
+}
+
   const int32_t* d_parts_cached = nullptr;
   if (sched == DM_SCHED_PLAIN && world == 1) {
     d_roots = s->d_up_order;
@@ -1303,6 +1424,15 @@ int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_
     int n_in = s->n_up;
     if (world > 1) {
       dm_opts po = *o;
+  // whole-graph counts of k <= 4 need no enumeration; what names its roots, its order, its groups
+  // or its progress (shards, subtree logs, schedules, vwarp, mode, reports, test hooks) keeps it
+  const bool whole = !o || (o->scheduler == DM_SCHED_PLAIN && o->world_size <= 1 && !o->subtree_counts &&
+                            o->vwarp == 0 && o->mode == DM_MODE_AUTO && !o->report && !o->test_flags);
+  int32_t cls[6];
+  if (k <= 4 && whole && census_class(dict, cls)) {
+    rc = motif_census(g, k, dict, cls, o, ctx, class_counts, st);
+    if (rc != 1) return rc;
+  }
       po.scheduler = DM_SCHED_PLAIN;
       for (int32_t v = 0; v < g->n; ++v)
         if (upper(v) > 0) roots.push_back(v);

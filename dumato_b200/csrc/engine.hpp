@@ -175,6 +175,35 @@ struct NearLaunch {
 int near_clique_launch(const NearLaunch& L, LaunchCtx& ctx, int* grid);
 size_t near_clique_warp_ints(int c, int dag_cap, int und_cap);
 
+// Whole-graph census of the connected 3- and 4-vertex classes (census.cu).
+constexpr int CENSUS_SUMS = 9;
+constexpr size_t CENSUS_BYTES = (CENSUS_SUMS + 2) * sizeof(unsigned long long);  // sums and cursors
+struct CensusLaunch {
+  GraphView g;                     // degree-ordered DAG in rank space
+  int k = 3;
+  const void* blocks = nullptr;    // clique index: a block for every root with 2 or more out-neighbours
+  const uint32_t* boff = nullptr;
+  const int32_t* ud = nullptr;     // undirected degree by rank
+  const int32_t* order = nullptr;  // ranks by descending out-degree; n_wide of them with 32 or more
+  int n_wide = 0;
+  int base = 0;                    // ranks below it have degree 0 or 1
+  bool wide_counters = false;      // a degree of 65,536 or more: 32-bit path counters
+  // k = 4: in-lists (census_in_lists), edge array (one word per padded DAG entry) and vertex list
+  const int32_t* in_end = nullptr;
+  const int32_t* in_deg = nullptr;
+  const void* in = nullptr;
+  uint32_t* up = nullptr;
+  int* list = nullptr;
+  unsigned long long* sums = nullptr;  // CENSUS_BYTES, zeroed by the launch
+};
+int census_launch(const CensusLaunch& L, LaunchCtx& ctx);
+// In-lists of the DAG: n end offsets, n lengths, 8 bytes per edge, and one scratch int.
+int census_in_lists(const GraphView& g, int32_t* in_end, int32_t* in_deg, void* in, int* pool, LaunchCtx& ctx);
+// Class of each connected type in the dictionary (false: the table is not constant on a type),
+// and the types' counts from the sums.
+bool census_class(const dm_dictionary* d, int32_t* cls);
+void census_classes(int k, const uint64_t* sums, uint64_t* counts);
+
 // Motif engine (motif.cu).
 struct MotifLaunch {
   GraphView g;                   // undirected CSR, original ids
