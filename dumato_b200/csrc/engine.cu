@@ -319,10 +319,10 @@ static void free_workspace(Workspace& w) {
   cudaFree(w.d_queue);
   cudaFree(w.d_per_root);
   cudaFree(w.d_parts);
+  cudaFree(w.d_census);
   cudaFree(w.d_bits);
   cudaFree(w.d_desc);
   cudaFree(w.d_params);
-  cudaFree(w.d_census);
   cudaFree(w.d_sched);
   cudaFree(w.d_sroots);
   cudaFree(w.d_sparts);
@@ -334,10 +334,10 @@ static void free_workspace(Workspace& w) {
   if (w.h_init) cudaFreeHost(w.h_init);
   if (w.h_hdr) cudaFreeHost(w.h_hdr);
   if (w.h_out) cudaFreeHost(w.h_out);
+  if (w.h_census) cudaFreeHost(w.h_census);
   w = Workspace();
 }
 
-  if (w.h_census) cudaFreeHost(w.h_census);
 static DeviceSlot* slot_for(dm_graph* g, int dev) {
   for (auto* p : g->dev)
     if (p->device == dev) return reinterpret_cast<DeviceSlot*>(p);
@@ -1165,23 +1165,6 @@ int dm_count_cliques_upto(dm_graph* g, int32_t kmax, const dm_opts* o, uint64_t*
   return DM_OK;
 }
 
-int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* count, dm_stats* st) {
-  if (!g || !count) return fail(DM_EINVAL, "dm_count_near_cliques: null argument");
-  if (n < 4 || n > 13) return fail(DM_EINVAL, "dm_count_near_cliques: n must be in [4, 13]");
-  int rc = check_opts(o);
-  if (rc) return rc;
-  LaunchCtx ctx;
-  rc = select_device(o, ctx);
-  if (rc) return rc;
-  std::lock_guard<std::mutex> lk(g->mu);
-  ensure_oriented(g);
-  DeviceSlot* s = slot_for(g, ctx.device);
-  Workspace& ws = s->ws;
-  if ((rc = prepare_ws(ws, ctx.stream))) return rc;
-  DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
-  if (!s->dg.has_oriented && (rc = upload_clique_image(g, s, ctx.stream))) return rc;
-  if (!s->dg.has_undirected) {
-    rc = upload_csr(g, g->row, g->adj, g->n, g->pad_row[0], g->pad_deg[0], g->pad_adj[0], &s->dg.d_row, &s->dg.d_deg,
 // Device arrays of the census: degrees by rank, and for k = 4 the in-lists (laid out on the
 // first call of a device copy). Returns 1 when the device has no room for them.
 static int ensure_census(dm_graph* g, DeviceSlot* s, int k, LaunchCtx& ctx) {
@@ -1227,6 +1210,23 @@ static int ensure_census(dm_graph* g, DeviceSlot* s, int k, LaunchCtx& ctx) {
   return DM_OK;
 }
 
+int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* count, dm_stats* st) {
+  if (!g || !count) return fail(DM_EINVAL, "dm_count_near_cliques: null argument");
+  if (n < 4 || n > 13) return fail(DM_EINVAL, "dm_count_near_cliques: n must be in [4, 13]");
+  int rc = check_opts(o);
+  if (rc) return rc;
+  LaunchCtx ctx;
+  rc = select_device(o, ctx);
+  if (rc) return rc;
+  std::lock_guard<std::mutex> lk(g->mu);
+  ensure_oriented(g);
+  DeviceSlot* s = slot_for(g, ctx.device);
+  Workspace& ws = s->ws;
+  if ((rc = prepare_ws(ws, ctx.stream))) return rc;
+  DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
+  if (!s->dg.has_oriented && (rc = upload_clique_image(g, s, ctx.stream))) return rc;
+  if (!s->dg.has_undirected) {
+    rc = upload_csr(g, g->row, g->adj, g->n, g->pad_row[0], g->pad_deg[0], g->pad_adj[0], &s->dg.d_row, &s->dg.d_deg,
                     &s->dg.d_adj, ctx.stream);
     if (rc) return rc;
     s->dg.has_undirected = true;
@@ -1301,52 +1301,6 @@ static int ensure_census(dm_graph* g, DeviceSlot* s, int k, LaunchCtx& ctx) {
   return DM_OK;
 }
 
-int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_opts* o, uint64_t* class_counts,
-                    dm_stats* st) {
-  if (!g || !dict || !class_counts) return fail(DM_EINVAL, "dm_count_motifs: null argument");
-  if (k < 3 || k > 7) return fail(DM_EINVAL, "dm_count_motifs: k must be in [3, 7]");
-  if (dict->k != k) return fail(DM_EINVAL, "dm_count_motifs: dictionary was built for another k");
-  int rc = check_opts(o);
-  if (rc) return rc;
-  LaunchCtx ctx;
-  rc = select_device(o, ctx);
-  if (rc) return rc;
-  if (o && o->scheduler == DM_SCHED_LEARNED && (rc = ensure_features(g, false))) return rc;
-  std::lock_guard<std::mutex> lk(g->mu);
-  DeviceSlot* s = slot_for(g, ctx.device);
-  Workspace& ws = s->ws;
-  if ((rc = prepare_ws(ws, ctx.stream))) return rc;
-  DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
-  if (!s->dg.has_undirected) {
-    rc = upload_csr(g, g->row, g->adj, g->n, g->pad_row[0], g->pad_deg[0], g->pad_adj[0], &s->dg.d_row,
-                    &s->dg.d_deg, &s->dg.d_adj, ctx.stream);
-    if (rc) return rc;
-    s->dg.has_undirected = true;
-  }
-  auto upper = [&](int32_t v) {
-    const int32_t* b = g->adj.data() + g->row[v];
-    const int32_t* e = g->adj.data() + g->row[v + 1];
-    return (int)(e - std::upper_bound(b, e, v));
-  };
-  const int sched = o ? o->scheduler : DM_SCHED_PLAIN;
-  const int world = (o && o->world_size > 1) ? o->world_size : 1;
-  const int32_t* d_roots = nullptr;
-  int n_roots = 0;
-  if (!s->d_up_order) {
-    std::vector<int32_t>& order = g->up_order;
-    if (order.empty()) {
-      for (int32_t v = 0; v < g->n; ++v)
-        if (upper(v) > 0) order.push_back(v);
-      std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return upper(a) > upper(b); });
-      pin_host(g, order.data(), sizeof(int32_t) * order.size());
-    }
-    DM_CUDA(gbuf_alloc(reinterpret_cast<void**>(&s->d_up_order), sizeof(int32_t) * std::max<size_t>(order.size(), 1)));
-    if (!order.empty())
-      DM_CUDA(cudaMemcpyAsync(s->d_up_order, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice,
-                              ctx.stream));
-    s->n_up = (int)order.size();
-  }
-  std::vector<int32_t> roots, parts;
 // k = 3, 4 class counts by the census (census.cu) instead of the enumeration. Returns 1, having
 // counted nothing, when the graph has no complete clique index (roots above 256 out-neighbours,
 // or over the memory budget), so that the caller enumerates.
@@ -1414,6 +1368,61 @@ static int motif_census(dm_graph* g, int k, const dm_dictionary* dict, const int
   return DM_OK;
 }
 
+int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_opts* o, uint64_t* class_counts,
+                    dm_stats* st) {
+  if (!g || !dict || !class_counts) return fail(DM_EINVAL, "dm_count_motifs: null argument");
+  if (k < 3 || k > 7) return fail(DM_EINVAL, "dm_count_motifs: k must be in [3, 7]");
+  if (dict->k != k) return fail(DM_EINVAL, "dm_count_motifs: dictionary was built for another k");
+  int rc = check_opts(o);
+  if (rc) return rc;
+  LaunchCtx ctx;
+  rc = select_device(o, ctx);
+  if (rc) return rc;
+  // whole-graph counts of k <= 4 need no enumeration; what names its roots, its order, its groups
+  // or its progress (shards, subtree logs, schedules, vwarp, mode, reports, test hooks) keeps it
+  const bool whole = !o || (o->scheduler == DM_SCHED_PLAIN && o->world_size <= 1 && !o->subtree_counts &&
+                            o->vwarp == 0 && o->mode == DM_MODE_AUTO && !o->report && !o->test_flags);
+  int32_t cls[6];
+  if (k <= 4 && whole && census_class(dict, cls)) {
+    rc = motif_census(g, k, dict, cls, o, ctx, class_counts, st);
+    if (rc != 1) return rc;
+  }
+  if (o && o->scheduler == DM_SCHED_LEARNED && (rc = ensure_features(g, false))) return rc;
+  std::lock_guard<std::mutex> lk(g->mu);
+  DeviceSlot* s = slot_for(g, ctx.device);
+  Workspace& ws = s->ws;
+  if ((rc = prepare_ws(ws, ctx.stream))) return rc;
+  DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
+  if (!s->dg.has_undirected) {
+    rc = upload_csr(g, g->row, g->adj, g->n, g->pad_row[0], g->pad_deg[0], g->pad_adj[0], &s->dg.d_row,
+                    &s->dg.d_deg, &s->dg.d_adj, ctx.stream);
+    if (rc) return rc;
+    s->dg.has_undirected = true;
+  }
+  auto upper = [&](int32_t v) {
+    const int32_t* b = g->adj.data() + g->row[v];
+    const int32_t* e = g->adj.data() + g->row[v + 1];
+    return (int)(e - std::upper_bound(b, e, v));
+  };
+  const int sched = o ? o->scheduler : DM_SCHED_PLAIN;
+  const int world = (o && o->world_size > 1) ? o->world_size : 1;
+  const int32_t* d_roots = nullptr;
+  int n_roots = 0;
+  if (!s->d_up_order) {
+    std::vector<int32_t>& order = g->up_order;
+    if (order.empty()) {
+      for (int32_t v = 0; v < g->n; ++v)
+        if (upper(v) > 0) order.push_back(v);
+      std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return upper(a) > upper(b); });
+      pin_host(g, order.data(), sizeof(int32_t) * order.size());
+    }
+    DM_CUDA(gbuf_alloc(reinterpret_cast<void**>(&s->d_up_order), sizeof(int32_t) * std::max<size_t>(order.size(), 1)));
+    if (!order.empty())
+      DM_CUDA(cudaMemcpyAsync(s->d_up_order, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice,
+                              ctx.stream));
+    s->n_up = (int)order.size();
+  }
+  std::vector<int32_t> roots, parts;
   const int32_t* d_parts_cached = nullptr;
   if (sched == DM_SCHED_PLAIN && world == 1) {
     d_roots = s->d_up_order;
@@ -1424,15 +1433,6 @@ static int motif_census(dm_graph* g, int k, const dm_dictionary* dict, const int
     int n_in = s->n_up;
     if (world > 1) {
       dm_opts po = *o;
-  // whole-graph counts of k <= 4 need no enumeration; what names its roots, its order, its groups
-  // or its progress (shards, subtree logs, schedules, vwarp, mode, reports, test hooks) keeps it
-  const bool whole = !o || (o->scheduler == DM_SCHED_PLAIN && o->world_size <= 1 && !o->subtree_counts &&
-                            o->vwarp == 0 && o->mode == DM_MODE_AUTO && !o->report && !o->test_flags);
-  int32_t cls[6];
-  if (k <= 4 && whole && census_class(dict, cls)) {
-    rc = motif_census(g, k, dict, cls, o, ctx, class_counts, st);
-    if (rc != 1) return rc;
-  }
       po.scheduler = DM_SCHED_PLAIN;
       for (int32_t v = 0; v < g->n; ++v)
         if (upper(v) > 0) roots.push_back(v);
