@@ -65,6 +65,7 @@ struct BatchArgs {
 constexpr int BATCH_WARPS = 8;
 constexpr int BATCH_CLIQUE_KMAX = 6;
 constexpr int BATCH_MOTIF_KMAX = 5;
+constexpr int BATCH_HIST = 64;  // classes a motif task counts in shared memory (k = 5 has 34)
 // bitmap rows of up to 2 words: clique roots with out-degree up to 128 take the bitmap path,
 // larger ones the list path. The per-warp shared memory then stays small enough for four
 // blocks per SM (the motif paths, which dominate mixed batches, are latency-bound and want
@@ -73,7 +74,9 @@ constexpr int BATCH_M = 2;
 
 template <int M>
 __host__ __device__ constexpr size_t batch_warp_smem() {
-  const size_t a = (size_t)warp_layout(M).total, b = motif_warp_smem<8>();
+  // (a clique task's words, or a motif task's class counters and its groups' state)
+  const size_t a = (size_t)warp_layout(M).total;
+  const size_t b = sizeof(unsigned long long) * BATCH_HIST + motif_warp_smem<BATCH_MOTIF_KMAX, 8>();
   return ((a > b ? a : b) + 15) / 16 * 16;
 }
 
@@ -97,10 +100,20 @@ template <int K, int W>
 __device__ void batch_motif(const BatchArgs& a, const BatchQuery& q, unsigned char* wsm, int2* arena,
                             uint32_t* bits, int v0, int b, int e, int level, const int* path,
                             unsigned long long& nodes) {
-  MotifShared* ws = reinterpret_cast<MotifShared*>(wsm);
-  MotifGroup* groups = reinterpret_cast<MotifGroup*>(ws + 1);
+  // a sweep adds to every class it meets: the task's own counters in shared memory take those
+  // adds, and the query's counters, which all warps share, one add per class and task
+  unsigned long long* hist = reinterpret_cast<unsigned long long*>(wsm);
+  MotifShared* ws = reinterpret_cast<MotifShared*>(hist + BATCH_HIST);
+  const bool local = q.n_classes <= BATCH_HIST;
+  const int lane = lane_id();
+  for (int c = lane; c < BATCH_HIST; c += 32) hist[c] = 0ull;
+  __syncwarp();
   unsigned long long tn = 0;
-  motif_run_task<K, W>(q.mctx, q.out, ws, groups, arena, bits, v0, b, e, level, path, tn);
+  motif_run_task<K, W>(q.mctx, local ? hist : q.out, ws, arena, bits, v0, b, e, level, path, tn);
+  __syncwarp();
+  if (local)
+    for (int c = lane; c < q.n_classes; c += 32)
+      if (hist[c]) atomicAdd(q.out + c, hist[c]);
   // every lane of a group counted the group's nodes: keep the leaders' counts
   if ((lane_id() & (W - 1)) == 0) nodes += tn;
 }
@@ -606,6 +619,7 @@ int dm_batch_create(const dm_query* queries, int32_t n, const dm_opts* opts, int
       d.mctx.lb.hungry_trigger = d.trigger;
       d.mctx.lb.min_split = 4;
       d.mctx.q2c = d.q2c;
+      d.mctx.sym = queries[i].dict->sym ? 1 : 0;
       d.mctx.maxdeg = d.maxdeg;
       d.mctx.arena_stride = d.arena_stride;
       d.mctx.bit_base = d.vbase;

@@ -82,7 +82,19 @@ static bool connected_small(int k, const Small& s) {
   return seen == (1u << k) - 1;
 }
 
-static void fill_connected(dm_dictionary* d) {
+// The derived fields of a finished table: which classes are connected, and whether the class
+// survives swapping the last two vertices (any table that follows isomorphism does; a hand-made
+// file need not).
+static void finish_tables(dm_dictionary* d) {
+  const int a_off = (d->k - 4) * (d->k - 1) / 2, b_off = (d->k - 3) * d->k / 2, bits = d->k - 2;
+  const int64_t m = (1ll << bits) - 1;
+  d->sym = d->k > 3;
+  for (int64_t q = 0; d->sym && q < d->n_quicks; ++q) {
+    const int64_t a = (q >> a_off) & m, b = (q >> b_off) & m;
+    if ((q >> (b_off + bits)) & 1 || a >= b) continue;
+    const int64_t swapped = q - (a << a_off) - (b << b_off) + (b << a_off) + (a << b_off);
+    d->sym = d->quick_to_class[q] == d->quick_to_class[swapped];
+  }
   d->connected.assign(d->n_classes, 0);
   std::vector<char> done(d->n_classes, 0);
   for (int64_t q = 0; q < d->n_quicks; ++q) {
@@ -146,7 +158,7 @@ int dm_dictionary_generate(int32_t k, dm_dictionary** out) {
   for (int64_t q = 0; q < nq; ++q) d->quick_to_class[q] = rank_of[orbit_of[q]];
   d->class_code.resize(nc);
   for (int32_t r = 0; r < nc; ++r) d->class_code[r] = orbit_code[order[r]];
-  fill_connected(d);
+  finish_tables(d);
   *out = d;
   return DM_OK;
 }
@@ -221,7 +233,7 @@ int dm_dictionary_load_csv(const char* path, dm_dictionary** out) {
       delete d;
       return fail(DM_EFORMAT, std::string("dictionary ") + path + " leaves a quick code unmapped");
     }
-  fill_connected(d);
+  finish_tables(d);
   *out = d;
   return DM_OK;
 }

@@ -95,6 +95,8 @@ struct dm_dictionary {
   std::vector<int32_t> quick_to_class;   // n_quicks
   std::vector<uint64_t> class_code;      // n_classes
   std::vector<uint8_t> connected;        // n_classes
+  bool sym = false;                      // codes that differ only in the order of two non-adjacent
+                                         // last vertices always have the same class
 };
 
 namespace dmb {

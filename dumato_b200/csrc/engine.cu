@@ -1519,6 +1519,7 @@ int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_
   L.nq = QUEUE_SHARDS;
   L.max_donations = ctx.donations_per_warp;
   L.q2c = ws.d_q2c;
+  L.sym = dict->sym ? 1 : 0;
   L.n_classes = dict->n_classes;
   L.hist = ws.d_hist;
   L.arena = ws.d_scratch;

@@ -216,6 +216,7 @@ struct MotifLaunch {
   int nq = 1;
   int max_donations = 16;
   const int32_t* q2c = nullptr;
+  int sym = 0;                   // dm_dictionary::sym
   int n_classes = 0;
   unsigned long long* hist = nullptr;
   void* arena = nullptr;

@@ -379,15 +379,6 @@ __device__ __forceinline__ bool range_maybe_donate(const LBArgs& lb, unsigned lo
   return range_split_donate(lb, range, root, donations_left, busy, ob, oe, cost_tail, min_items, level, path);
 }
 
-// Demand test shared by the donation paths (lane 0): hungry warps outnumber queued tasks by
-// the trigger and the task has run long enough.
-__device__ __forceinline__ bool lb_wants_donation(const LBArgs& lb, const int* donations_left, long long task_start) {
-  if (lb.hungry_trigger <= 0) return false;
-  if (*reinterpret_cast<const volatile int*>(donations_left) <= 0) return false;
-  if (vload(&lb.ctr->hungry) - vload(&lb.ctr->queued) < lb.hungry_trigger) return false;
-  return global_ns() - task_start >= lb.donate_after_ns;
-}
-
 // Enqueues a deep task (lane 0). Returns false when every shard is full.
 __device__ __forceinline__ bool lb_donate_deep(const LBArgs& lb, int root, int level, const int* path, int b, int e) {
   atomicAdd(&lb.ctr->pending, 1);

@@ -35,11 +35,10 @@ __global__ void __launch_bounds__(32 * MOTIF_WARPS, 4) motif_kernel(const __grid
   unsigned char* wbase = smem + sizeof(unsigned long long) * ((a.n_classes + 1) & ~1);
   const int lane = lane_id();
   const int wib = warp_in_block();
-  MotifShared* ws = reinterpret_cast<MotifShared*>(wbase + motif_warp_smem<W>() * wib);
-  MotifGroup* groups = reinterpret_cast<MotifGroup*>(ws + 1);
+  MotifShared* ws = reinterpret_cast<MotifShared*>(wbase + motif_warp_smem<K, W>() * wib);
   const MotifCtx& c = a.c;
   const size_t warp_bit_words = (size_t)c.bit_words * 2 * (32 / W);
-  uint32_t* sbits = reinterpret_cast<uint32_t*>(wbase + motif_warp_smem<W>() * MOTIF_WARPS);
+  uint32_t* sbits = reinterpret_cast<uint32_t*>(wbase + motif_warp_smem<K, W>() * MOTIF_WARPS);
   for (int cl = threadIdx.x; cl < a.n_classes; cl += blockDim.x) bhist[cl] = 0;
   if (a.bits_smem)
     for (size_t i = threadIdx.x; i < warp_bit_words * MOTIF_WARPS; i += blockDim.x) sbits[i] = 0u;
@@ -79,7 +78,7 @@ __global__ void __launch_bounds__(32 * MOTIF_WARPS, 4) motif_kernel(const __grid
       if (!donated && a.parts) part_bounds(__ldg(a.parts + first + ti), bb, ee);
       ++ntasks;
       // block-level class counters, added to the global ones at exit
-      motif_run_task<K, W>(c, bhist, ws, groups, warp_arena, warp_bits, v0, bb, ee, level, path, nodes);
+      motif_run_task<K, W>(c, bhist, ws, warp_arena, warp_bits, v0, bb, ee, level, path, nodes);
     }
     if (lane == 0) lb_done(c.lb, count);
   }
@@ -105,7 +104,7 @@ static int launch_motif(MotifArgs a, LaunchCtx& ctx, int* grid_out) {
   const size_t bits_bytes = (size_t)a.c.bit_words * 2 * (32 / W) * sizeof(uint32_t) * MOTIF_WARPS;
   a.bits_smem = a.bits && a.c.bit_words > 0 && bits_bytes <= MOTIF_SMEM_BITS_MAX ? 1 : 0;
   const size_t smem = sizeof(unsigned long long) * ((a.n_classes + 1) & ~1) +
-                      motif_warp_smem<W>() * MOTIF_WARPS + (a.bits_smem ? bits_bytes : 0);
+                      motif_warp_smem<K, W>() * MOTIF_WARPS + (a.bits_smem ? bits_bytes : 0);
   auto kern = motif_kernel<K, W>;
   static LaunchCache cache;
   int occ = 0;
@@ -140,6 +139,7 @@ int motif_launch(const MotifLaunch& L, LaunchCtx& ctx, int* grid) {
                   L.max_donations, (long long)ctx.donate_after_us * 1000ll, (long long)ctx.timeout_ms * 1000000ll,
                   ctx.test_stall, 4, L.nq};
   a.c.q2c = L.q2c;
+  a.c.sym = L.sym;
   a.c.maxdeg = L.maxdeg;
   a.c.arena_stride = (int)motif_group_stride(L.k, L.maxdeg);
   a.c.per_root = L.per_root;

@@ -19,11 +19,17 @@
 // sorted runs (run 0 = N(v0) above v0, run i = excl(v_i)). E_t is kept sorted by vertex id, so
 // the inherited members are the suffix of E_t after w.
 //
-// Leaves are counted in bulk: at the last internal level, for each w the leaf masks of
-// E_{k-2} are histogrammed without materialising it (inherited members: either a membership
-// probe in N(w) each, or the suffix's mask counts corrected by the members of N(w) above w,
-// whichever side is cheaper; excl(w): |N(w) above v0| - |N(w) cap U_t|, also from the
-// cheaper side), then each non-empty mask bucket adds to one class counter.
+// The last two vertices are counted in bulk (leaf_sweep): once E_{k-3} of a (k-2)-prefix is
+// materialised, no member is expanded. With R_a the number of members of mask a, the pairs
+// (w, x) of members contribute R_a R_b (C(R_a,2) for a = b) subgraphs of masks a, b, of which
+// those joined by an edge are moved to the joined class; and a member w adds its neighbours above
+// v0 that lie outside U_{k-3}. So the sweep only walks the members' rows above v0 once, testing
+// each neighbour against the two bitmaps, and adds to the class counters once per prefix and
+// mask pair. The rows of W members are laid end to end, one entry per lane, so rows shorter than
+// the group waste no lanes. Expanding every member w on its own (its row scanned, its leaf
+// masks looked up and flushed) took 12.6 ms for k = 5 on a Chung-Lu graph of 3,000 vertices and
+// 18,000 edges, 10.4 ms for k = 6 on a random graph of 2,000 / 10,000, 387 ms for a batch of 24
+// graphs; the sweep takes 7.0, 5.2 and 86 ms.
 //
 // Virtual warps (the reference's DM_WCV variant, src/DM_WCV/DuMatoGPU.cu:12-37): with W < 32
 // the groups of a warp take second vertices of the same task from its shared item range and
@@ -57,8 +63,16 @@ struct alignas(16) MotifGroup {
   int runn[MOTIF_KMAX];        // run sizes per level
   unsigned quick[MOTIF_KMAX];  // quick code of the prefix ending at level t
   int spill_lo, spill_hi;      // second vertices split off when the queue was full
-  unsigned mh[64];             // leaf-mask histogram
-  unsigned sh[32];             // masks of E_{k-3}[pos..n): the members still above the current vertex
+};
+
+// Sweep state of one group: class counters of its task, and by mask over E_{k-3} the members swept
+// (rest: those after the swept range), their neighbours outside U, and the joined pairs.
+template <int K>
+struct alignas(16) MotifSweep {
+  static constexpr int MASKS = 1 << (K > 3 ? K - 2 : 2);
+  unsigned swept[MASKS], rest[MASKS], fresh[MASKS];
+  unsigned joined[K > 3 ? MASKS * MASKS : 1];
+  unsigned mh[8];              // k = 3: leaf-mask histogram
 };
 
 // Task state shared by the groups of one warp.
@@ -68,9 +82,9 @@ struct alignas(16) MotifShared {
   int busy;                    // serialises level-0 splits
 };
 
-template <int W>
+template <int K, int W>
 __host__ __device__ constexpr size_t motif_warp_smem() {
-  return sizeof(MotifShared) + sizeof(MotifGroup) * (32 / W);
+  return sizeof(MotifShared) + (sizeof(MotifGroup) + sizeof(MotifSweep<K>)) * (32 / W);
 }
 
 // Everything a motif task needs besides its own (v0, range) or prefix.
@@ -78,6 +92,7 @@ struct MotifCtx {
   GraphView g;                 // undirected CSR, rows sorted
   LBArgs lb;
   const int32_t* q2c;          // quick code -> class
+  int sym;                     // the class does not depend on the order of the last two vertices
   int maxdeg;                  // bound on every degree in g (arena sizing)
   int arena_stride;            // int2 slots per group
   unsigned long long* per_root;  // optional: subgraphs found under each v0 (subtree logger)
@@ -85,18 +100,19 @@ struct MotifCtx {
   int bit_words;               // 32-bit words per bitmap (0 = no bitmaps: binary searches only)
 };
 
-// Membership bitmaps of one group (2 x bit_words words in global memory, all zero between
-// tasks): U holds U_t = N(v_0..v_t) above v0 for the levels materialised on the current path,
-// E holds E_{k-3} (k = 3: E_0). They turn the leaf step and the exclusion test into one probe
-// per neighbour instead of binary searches over the runs.
-__device__ __forceinline__ bool bit_test(const uint32_t* b, int x) { return (b[x >> 5] >> (x & 31)) & 1u; }
+// Membership bitmaps of one group (bit_words pairs of words, all zero between tasks; word 2i of
+// U and word 2i + 1 of E, so that one 8-byte load answers both questions): U holds
+// U_t = N(v_0..v_t) above v0 for the levels materialised on the current path, E holds E_{k-3}.
+// They turn the sweep and the exclusion test into one probe per neighbour instead of binary
+// searches over the runs (k >= 4).
+__device__ __forceinline__ bool bit_test(const uint32_t* b, int x) { return (b[2 * (x >> 5)] >> (x & 31)) & 1u; }
 
 template <int W>
 __device__ __forceinline__ void bits_flip_ids(uint32_t* b, int base, const int32_t* ids, int n, bool set, int gl) {
   for (int i = gl; i < n; i += W) {
     const int x = __ldg(ids + i) - base;
-    if (set) atomicOr(b + (x >> 5), 1u << (x & 31));
-    else atomicAnd(b + (x >> 5), ~(1u << (x & 31)));
+    if (set) atomicOr(b + 2 * (x >> 5), 1u << (x & 31));
+    else atomicAnd(b + 2 * (x >> 5), ~(1u << (x & 31)));
   }
 }
 
@@ -104,8 +120,8 @@ template <int W>
 __device__ __forceinline__ void bits_flip_list(uint32_t* b, int base, const int2* list, int n, bool set, int gl) {
   for (int i = gl; i < n; i += W) {
     const int x = list[i].x - base;
-    if (set) atomicOr(b + (x >> 5), 1u << (x & 31));
-    else atomicAnd(b + (x >> 5), ~(1u << (x & 31)));
+    if (set) atomicOr(b + 2 * (x >> 5), 1u << (x & 31));
+    else atomicAnd(b + 2 * (x >> 5), ~(1u << (x & 31)));
   }
 }
 
@@ -154,33 +170,199 @@ __device__ __forceinline__ void mask_hist(const int2* list, int lo, int hi, unsi
   __syncwarp(gmask);
 }
 
-// Flushes the group's leaf-mask histogram (masks below NMASK) into the class counters.
-template <int W, int NMASK>
-__device__ __forceinline__ void flush_masks(MotifGroup* sg, const int32_t* q2c, unsigned quick_p, int off,
-                                            unsigned long long* hist, unsigned long long& task_cnt, int gl,
-                                            unsigned gmask) {
-  for (int m = gl; m < NMASK; m += W) {
-    const unsigned c = sg->mh[m];
+// Sweeps members [lo, *lim) of the materialised set E = E_{K-3} (n members, sorted by id) of the
+// prefix whose quick code is quick_t: every subgraph with at least one of its last two vertices
+// in the range, the other one after it in E or new, is added to hist. `between` runs after every
+// batch of W members with the next position (group-uniform; it may lower *lim). Returns this
+// lane's share of the subgraphs counted.
+//
+// Bound by instruction issue: a step of about 45 instructions takes W row entries (an owner
+// search by shuffles, one load of the entry, one 8-byte load of both bitmaps, one ballot).
+template <int K, int W, class Between>
+__device__ __forceinline__ unsigned long long leaf_sweep(const MotifCtx& c, unsigned long long* hist, MotifSweep<K>* sw,
+                                                         const int2* E, int n, int lo, const int* lim, int v0,
+                                                         unsigned quick_t, const uint32_t* Ub, const int32_t* E0,
+                                                         int n0, const int2* runs1, size_t rstride, const int* runn,
+                                                         int gl, int gsrc, unsigned gmask, Between&& between) {
+  constexpr int P = K - 2;  // position of the first of the two vertices; the second is at K - 1
+  constexpr int MASKS = MotifSweep<K>::MASKS;
+  unsigned long long counted = 0;
+  auto code = [&](unsigned a, unsigned b) -> unsigned {
+    return quick_t + (P >= 2 ? a << quick_off(P) : 0u) + (b << quick_off(K - 1));
+  };
+  if (!c.sym) {
+    // pairs in id order, one member at a time: the masks of the members after it
+    mask_hist<W>(E, lo, n, sw->rest, gl, gmask);
+  }
+  int i0 = lo;
+  while (i0 < *reinterpret_cast<const volatile int*>(lim)) {
+    const int end = min(*reinterpret_cast<const volatile int*>(lim), i0 + W);
+    const bool valid = i0 + gl < end;
+    int2 wm = make_int2(0, 0);
+    int base = 0, len = 0;
+    if (valid) {
+      wm = E[i0 + gl];
+      const int r = __ldg(c.g.row + wm.x);
+      const int d = __ldg(c.g.deg + wm.x);
+      const int s = lower_bound(c.g.adj + r, 0, d, v0 + 1);
+      base = r + s;
+      len = d - s;
+    }
+    int off = len;
+#pragma unroll
+    for (int o = 1; o < W; o <<= 1) {
+      const int y = __shfl_up_sync(gmask, off, o, W);
+      if (gl >= o) off += y;
+    }
+    const int total = __shfl_sync(gmask, off, W - 1, W);
+    off -= len;
+    unsigned inside = 0;  // this lane's member: its neighbours in U
+    for (int f0 = 0; f0 < total; f0 += W) {
+      const int f = f0 + gl;
+      // owner: the last member whose entries start at or before f
+      int j = 0;
+#pragma unroll
+      for (int h = W / 2; h >= 1; h >>= 1) {
+        const int o = __shfl_sync(gmask, off, j + h, W);
+        j = o <= f ? j + h : j;
+      }
+      const int ob = __shfl_sync(gmask, base, j, W) + (f - __shfl_sync(gmask, off, j, W));
+      const int ow = __shfl_sync(gmask, wm.x, j, W);
+      const int om = __shfl_sync(gmask, wm.y, j, W);
+      bool in_u = false, in_e = false;
+      int x = 0;
+      if (f < total) {
+        x = __ldg(c.g.adj + ob);
+        if (Ub) {
+          const int xb = x - c.bit_base;
+          const uint2 ue = *reinterpret_cast<const uint2*>(Ub + 2 * (xb >> 5));
+          in_u = (ue.x >> (xb & 31)) & 1u;
+          in_e = x > ow && ((ue.y >> (xb & 31)) & 1u);
+        } else {
+          in_u = in_runs(x, E0, n0, runs1, rstride, runn, K - 3);
+          in_e = in_u && x > ow;
+        }
+      }
+      const unsigned bal = __ballot_sync(gmask, in_u) >> gsrc;
+      const int a0 = min(max(off - f0, 0), W), a1 = min(max(off + len - f0, 0), W);
+      const unsigned upto1 = a1 >= 32 ? 0xffffffffu : (1u << a1) - 1u;
+      const unsigned upto0 = a0 >= 32 ? 0xffffffffu : (1u << a0) - 1u;
+      inside += __popc(bal & upto1 & ~upto0);
+      if (in_e) {
+        const int q = lower_bound2(E, i0 + j + 1, n, x);
+        if (q < n) {
+          const int2 y = E[q];
+          if (y.x == x) atomicAdd(&sw->joined[om * MASKS + y.y], 1u);
+        }
+      }
+    }
+    if (valid) {
+      if (len > (int)inside) atomicAdd(&sw->fresh[wm.y], (unsigned)len - inside);
+      atomicAdd(&sw->swept[wm.y], 1u);
+    }
+    __syncwarp(gmask);
+    if (!c.sym) {
+      for (int i = i0; i < end; ++i) {
+        const int m = E[i].y;
+        if (gl == 0) sw->rest[m] -= 1u;
+        __syncwarp(gmask);
+        for (int b = gl; b < MASKS; b += W) {
+          const unsigned t = sw->rest[b];
+          if (t) {
+            atomicAdd(hist + __ldg(c.q2c + code(m, b)), (unsigned long long)t);
+            counted += t;
+          }
+        }
+        __syncwarp(gmask);
+      }
+    }
+    i0 = end;
+    between(end);
+  }
+  if (c.sym && i0 < n) mask_hist<W>(E, i0, n, sw->rest, gl, gmask);
+  __syncwarp(gmask);
+  for (int a = 1; a < MASKS; ++a) {
+    const unsigned ra = sw->swept[a];
+    if (ra == 0) continue;
+    for (int b = gl; b < MASKS; b += W) {
+      unsigned long long pairs = 0;
+      if (c.sym) {
+        const unsigned long long rb = sw->swept[b];
+        if (b == a) pairs = (rb & 1) ? rb * ((rb - 1) >> 1) : (rb >> 1) * (rb - 1);
+        else if (b > a) pairs = (unsigned long long)ra * rb;
+        pairs += (unsigned long long)ra * sw->rest[b];
+      }
+      const unsigned join = sw->joined[a * MASKS + b];
+      if (join) {
+        sw->joined[a * MASKS + b] = 0u;
+        atomicAdd(hist + __ldg(c.q2c + code(a, b | (1 << P))), (unsigned long long)join);
+      }
+      // (a pair joined in the order (a, b) was taken in that order or, with equal classes, in the
+      // other: the difference may be negative here, the class total is not)
+      if (pairs != join) atomicAdd(hist + __ldg(c.q2c + code(a, b)), pairs - join);
+      counted += pairs;
+    }
+    if (gl == 0) {
+      const unsigned fr = sw->fresh[a];
+      if (fr) {
+        sw->fresh[a] = 0u;
+        atomicAdd(hist + __ldg(c.q2c + code(a, 1 << P)), (unsigned long long)fr);
+        counted += fr;
+      }
+    }
+  }
+  __syncwarp(gmask);
+  for (int m = gl; m < MASKS; m += W) sw->swept[m] = sw->rest[m] = 0u;
+  __syncwarp(gmask);
+  return counted;
+}
+
+// k = 3: flushes the group's leaf-mask histogram (masks below 4) into the class counters.
+template <int W>
+__device__ __forceinline__ void flush_masks(unsigned* mh, const int32_t* q2c, unsigned long long* hist,
+                                            unsigned long long& task_cnt, int gl, unsigned gmask) {
+  for (int m = gl; m < 4; m += W) {
+    const unsigned c = mh[m];
     if (c) {
-      sg->mh[m] = 0;
-      const int cls = __ldg(q2c + (quick_p + ((unsigned)m << off)));
-      atomicAdd(hist + cls, (unsigned long long)c);
+      mh[m] = 0;
+      atomicAdd(hist + __ldg(q2c + m), (unsigned long long)c);
       task_cnt += c;
     }
   }
   __syncwarp(gmask);
 }
 
+// The group leader's view of the demand for work: the hungry and queued counters as loaded at the
+// previous check. The loads complete while the group works on, so a check never waits for them.
+struct MotifDemand {
+  int hungry = 0;
+  int queued = 0;
+};
+
+__device__ __forceinline__ void motif_sample(const LBArgs& lb, MotifDemand& dm) {
+  if (lb.hungry_trigger <= 0) return;
+  dm.hungry = vload(&lb.ctr->hungry);
+  dm.queued = vload(&lb.ctr->queued);
+}
+
+// Whether this task should hand work out now, by the previous sample; takes the next one.
+__device__ __forceinline__ bool motif_wanted(const LBArgs& lb, const MotifShared* ws, MotifDemand& dm, long long t_start) {
+  if (lb.hungry_trigger <= 0) return false;
+  const bool wanted = dm.hungry - dm.queued >= lb.hungry_trigger;
+  motif_sample(lb, dm);
+  if (!wanted || *reinterpret_cast<const volatile int*>(&ws->donations_left) <= 0) return false;
+  return global_ns() - t_start >= lb.donate_after_ns;
+}
+
 // Group leader, between two expansions of a task whose lowest own level is `floor` (1 for an
 // item task; L for a donated DFS prefix of level L) and whose deepest materialised level is
-// t: when warps are hungry, hands the upper half of the shallowest level that still has
+// t, when work is wanted: hands the upper half of the shallowest level that still has
 // unexpanded members to the queue. Level 0 is the task's second-vertex range (cost-aware
 // split, shared by the groups); a level s >= 1 goes out as (root, s, path to E_s, position
 // range), the path being the second vertex's index `it` and the index picked at each level
 // 1..s-1.
-__device__ __forceinline__ void motif_try_donate(const LBArgs& lb, MotifShared* ws, MotifGroup* sg, int v0,
-                                                 int floor, int t, int it, int n0, long long t_start) {
-  if (!lb_wants_donation(lb, &ws->donations_left, t_start)) return;
+__device__ __forceinline__ void motif_donate(const LBArgs& lb, MotifShared* ws, MotifGroup* sg, int v0, int floor, int t,
+                                             int it, int n0) {
   if (floor == 1) {
     const unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(&ws->range);
     const int next = (int)(unsigned)cur, end = (int)(unsigned)(cur >> 32);
@@ -188,7 +370,7 @@ __device__ __forceinline__ void motif_try_donate(const LBArgs& lb, MotifShared* 
       // inside a running item even two untaken second vertices are worth handing out
       if (sg->spill_lo >= sg->spill_hi) {
         int ob = 0, oe = 0;
-        if (range_maybe_donate(lb, &ws->range, v0, &ws->donations_left, t_start, &ws->busy, ob, oe, n0, 2)) {
+        if (range_split_donate(lb, &ws->range, v0, &ws->donations_left, &ws->busy, ob, oe, n0, 2, 0, nullptr)) {
           // the queue was full: this group runs the split-off second vertices itself
           sg->spill_lo = ob;
           sg->spill_hi = oe;
@@ -214,6 +396,47 @@ __device__ __forceinline__ void motif_try_donate(const LBArgs& lb, MotifShared* 
   }
 }
 
+// k = 3: the subgraphs (v0, w, x) with w the member of E_0 = N(v0) above v0 at index it.
+template <int W>
+__device__ __forceinline__ void leaf_pairs(const MotifCtx& c, unsigned* mh, const int32_t* E0, int n0, int it, int v0,
+                                           unsigned long long* hist, unsigned long long& task_cnt, int gl,
+                                           unsigned gmask) {
+  const int w = __ldg(E0 + it);
+  const int32_t* Nw = c.g.adj + __ldg(c.g.row + w);
+  const int dw = __ldg(c.g.deg + w);
+  const int start = it + 1, n_inh = n0 - start;
+  const int sw0 = lower_bound(Nw, 0, dw, v0 + 1);
+  const int above = dw - sw0;
+  const int gt = lower_bound(Nw, 0, dw, w + 1);
+  const int dgt = dw - gt;
+  // members of E_0 after w that are adjacent to w: probe each of them in N(w), or each
+  // neighbour above w in E_0, whichever side is cheaper
+  unsigned adj = 0;
+  if ((long long)dgt * ilog2p1(n_inh) < (long long)n_inh * ilog2p1(dw)) {
+    for (int i = gt + gl; i < dw; i += W) adj += contains(E0 + start, n_inh, Nw[i]) ? 1u : 0u;
+  } else {
+    for (int i = start + gl; i < n0; i += W) adj += contains(Nw, dw, __ldg(E0 + i)) ? 1u : 0u;
+  }
+  // new vertices: N(w) above v0 minus N(v0)
+  unsigned inter = 0;
+  if (n0 <= above) {
+    for (int i = gl; i < n0; i += W) inter += contains(Nw, dw, __ldg(E0 + i)) ? 1u : 0u;
+  } else {
+    for (int i = sw0 + gl; i < dw; i += W) inter += contains(E0, n0, Nw[i]) ? 1u : 0u;
+  }
+  for (int o = W / 2; o > 0; o >>= 1) {
+    adj += __shfl_xor_sync(gmask, adj, o);
+    inter += __shfl_xor_sync(gmask, inter, o);
+  }
+  if (gl == 0) {
+    mh[1] = (unsigned)n_inh - adj;
+    mh[2] = (unsigned)above - inter;
+    mh[3] = adj;
+  }
+  __syncwarp(gmask);
+  flush_masks<W>(mh, c.q2c, hist, task_cnt, gl, gmask);
+}
+
 // Runs one task on the calling warp (all 32 lanes). level 0: second vertices [bb, ee) of v0
 // (task_range encoding); level L >= 1: replay path[0..L-1], then expand positions [bb, ee) of
 // E_L (group 0 only). Adds the task's subgraphs to hist (class counters in shared or global
@@ -221,16 +444,17 @@ __device__ __forceinline__ void motif_try_donate(const LBArgs& lb, MotifShared* 
 // lane of a group counts the same nodes; the caller keeps group leaders' counts only).
 template <int K, int W>
 __device__ __forceinline__ void motif_run_task(const MotifCtx& c, unsigned long long* hist, MotifShared* ws,
-                                               MotifGroup* groups, int2* warp_arena, uint32_t* warp_bits, int v0,
-                                               int bb, int ee, int level, const int* path,
-                                               unsigned long long& nodes) {
+                                               int2* warp_arena, uint32_t* warp_bits, int v0, int bb, int ee,
+                                               int level, const int* path, unsigned long long& nodes) {
   static_assert(W == 8 || W == 16 || W == 32, "virtual warp width must be 8, 16 or 32");
   const int lane = lane_id();
   const int gl = lane & (W - 1);
   const int gi = lane / W;
   const unsigned gmask = (W == 32) ? FULL_MASK : (((1u << W) - 1u) << (gi * W));
   const int gsrc = gi * W;  // the group leader's lane
-  MotifGroup* sg = groups + gi;
+  // the warp's words: MotifShared | a MotifGroup per group | a MotifSweep per group
+  MotifGroup* sg = reinterpret_cast<MotifGroup*>(ws + 1) + gi;
+  MotifSweep<K>* sw = reinterpret_cast<MotifSweep<K>*>(reinterpret_cast<MotifGroup*>(ws + 1) + 32 / W) + gi;
   // level t (1..K-3): extension list E_t at ext_at(t); run t at run_at(t) (no pointer
   // tables, so nothing indexed dynamically lives in local memory)
   int2* const arena = warp_arena + (size_t)gi * c.arena_stride;
@@ -243,7 +467,7 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, unsigned long 
   // binary searches it saves)
   const bool use_bits = K >= 4 && warp_bits != nullptr && c.bit_words > 0;
   uint32_t* const Ub = use_bits ? warp_bits + (size_t)gi * 2 * c.bit_words : nullptr;
-  uint32_t* const Eb = use_bits ? Ub + c.bit_words : nullptr;
+  uint32_t* const Eb = use_bits ? Ub + 1 : nullptr;
   int bdepth = 0;  // levels 1..bdepth have their run (and, at level k-3, E) bits set
   unsigned long long task_cnt = 0;
   const long long t_start = global_ns();
@@ -266,11 +490,11 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, unsigned long 
     sg->quick[0] = 0;
     sg->spill_lo = sg->spill_hi = 0;
   }
-  for (int m = gl; m < 64; m += W) sg->mh[m] = 0;
-  if (use_bits) {
-    bits_flip_ids<W>(Ub, c.bit_base, E0, n0, true, gl);
-    if (K == 3) bits_flip_ids<W>(Eb, c.bit_base, E0, n0, true, gl);
-  }
+  for (int m = gl; m < (int)(sizeof(MotifSweep<K>) / sizeof(unsigned)); m += W) reinterpret_cast<unsigned*>(sw)[m] = 0u;
+  if (use_bits) bits_flip_ids<W>(Ub, c.bit_base, E0, n0, true, gl);
+  MotifDemand dm;  // group leader
+  if (gl == 0) motif_sample(c.lb, dm);
+  unsigned long long checked = nodes;
   __syncwarp();
   // drops the bits of levels from..bdepth (the group's lanes, then a group barrier)
   auto drop_levels = [&](int from) {
@@ -299,7 +523,8 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, unsigned long 
           if (sg->spill_lo < sg->spill_hi) it = sg->spill_lo++;
         } else if (sg->spill_lo >= sg->spill_hi) {
           int ob = 0, oe = 0;
-          if (range_maybe_donate(c.lb, &ws->range, v0, &ws->donations_left, t_start, &ws->busy, ob, oe, n0)) {
+          if (motif_wanted(c.lb, ws, dm, t_start) &&
+              range_split_donate(c.lb, &ws->range, v0, &ws->donations_left, &ws->busy, ob, oe, n0, 0, 0, nullptr)) {
             sg->spill_lo = ob;
             sg->spill_hi = oe;
           }
@@ -308,143 +533,42 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, unsigned long 
       it = __shfl_sync(gmask, it, gsrc);
       if (it < 0) break;
     }
-    // prefix (v0, w1); the members of E_0 after w1 are the inherited part
-    int t = 0;
-    int w = __ldg(E0 + it);
-    int wmask = 1;
-    bool bad = false;
-    // depth-first over levels; level t's current vertex is w with mask wmask
-    while (true) {
-      // here the prefix is v_0..v_t plus w = v_{t+1}
-      const int p = t + 1;  // position of w
-      if (p > level) {
-        // nodes at or above a donated prefix's level belong to the donor
-        ++nodes;
-        if (gl == 0 && (nodes & 255) == 0) atomicAdd(&c.lb.ctr->progress, 256ull);
-      }
-      unsigned quick_p = (t == 0) ? 0u : sg->quick[t];
-      if (p >= 2) quick_p += ((unsigned)wmask & ((1u << p) - 1u)) << quick_off(p);
-      const int32_t* Nw = c.g.adj + __ldg(c.g.row + w);
-      const int dw = __ldg(c.g.deg + w);
-      // inherited members: e in E_t with e > w. E_t is sorted by vertex id and w is its
-      // member at position pos[t] - 1 (E_0: index it), so they are the suffix from there.
-      const int2* Et = t == 0 ? nullptr : ext_at(t);
-      const int nE = (t == 0) ? n0 : sg->n[t];
-      const int startE = (t == 0) ? it + 1 : sg->pos[t];
-      if (p == K - 2) {
-        // leaves: histogram the masks of E_{p} without writing it
-        const int leaf_off = quick_off(K - 1);
-        const int n_inh = nE - startE;
-        // a short row is scanned whole (members up to v0 skipped) instead of searched for v0
-        const bool short_row = dw <= 2 * W;
-        const int sw0b = short_row ? 0 : lower_bound(Nw, 0, dw, v0 + 1);
-        int usize = n0;
-        for (int i = 1; i <= t; ++i) usize += sg->runn[i];
-        if (use_bits && dw - sw0b <= 4 * (n_inh + usize) + 128) {
-          // one pass over N(w) above v0: a neighbour outside U_t is a new member of E_{p}
-          // (excl(w)); a neighbour in E_t above w is an inherited member adjacent to w; the
-          // inherited members not adjacent to w come from the suffix's mask counts
-          if (t == 0) {
-            if (gl == 0 && n_inh) atomicAdd(&sg->mh[1], (unsigned)n_inh);
-          } else {
-            for (int m = gl; m < (1 << (K - 2)); m += W) {
-              const unsigned cm = sg->sh[m];
-              if (cm) atomicAdd(&sg->mh[m], cm);
-            }
-          }
+    if constexpr (K == 3) {
+      ++nodes;
+      if (gl == 0 && (nodes & 255) == 0) atomicAdd(&c.lb.ctr->progress, 256ull);
+      leaf_pairs<W>(c, sw->mh, E0, n0, it, v0, hist, task_cnt, gl, gmask);
+    } else {
+      // prefix (v0, w1); the members of E_0 after w1 are the inherited part
+      int t = 0;
+      int w = __ldg(E0 + it);
+      int wmask = 1;
+      bool bad = false;
+      // hands work away when it is wanted (checked every 64 expansions)
+      auto give = [&]() {
+        if (nodes - checked >= 64) {
+          checked = nodes;
+          if (gl == 0 && motif_wanted(c.lb, ws, dm, t_start)) motif_donate(c.lb, ws, sg, v0, floor, t, it, n0);
           __syncwarp(gmask);
-          unsigned ex = 0;
-          for (int i = sw0b + gl; i < dw; i += W) {
-            const int32_t x = Nw[i];
-            if (x <= v0) continue;
-            const int xb = x - c.bit_base;
-            if (!bit_test(Ub, xb)) {
-              ++ex;
-            } else if (x > w && bit_test(Eb, xb)) {
-              const int em = (t == 0) ? 1 : Et[lower_bound2(Et, startE, nE, x)].y;
-              atomicSub(&sg->mh[em], 1u);
-              atomicAdd(&sg->mh[em | (1 << p)], 1u);
-            }
-          }
-          for (int o = W / 2; o > 0; o >>= 1) ex += __shfl_xor_sync(gmask, ex, o);
-          if (gl == 0 && ex) atomicAdd(&sg->mh[1 << p], ex);
-          __syncwarp(gmask);
-          flush_masks<W, (1 << (K - 1))>(sg, c.q2c, quick_p, leaf_off, hist, task_cnt, gl, gmask);
-        } else {
-        const int sw0 = short_row ? lower_bound(Nw, 0, dw, v0 + 1) : sw0b;
-        const int above = dw - sw0;
-        const int gt = lower_bound(Nw, 0, dw, w + 1);
-        const int dgt = dw - gt;
-        // probe each inherited member in N(w), or take the suffix's mask counts and move
-        // the members found in N(w) above w (whichever side is cheaper)
-        if ((long long)dgt * ilog2p1(n_inh) + (1 << (K - 2)) < (long long)n_inh * ilog2p1(dw)) {
-          if (t == 0) {
-            if (gl == 0 && n_inh) atomicAdd(&sg->mh[1], (unsigned)n_inh);
-          } else {
-            for (int m = gl; m < (1 << (K - 2)); m += W) {
-              const unsigned cm = sg->sh[m];
-              if (cm) atomicAdd(&sg->mh[m], cm);
-            }
-          }
-          __syncwarp(gmask);
-          for (int i = gt + gl; i < dw; i += W) {
-            const int32_t x = Nw[i];
-            int em = -1;
-            if (t == 0) {
-              const int j = lower_bound(E0, startE, n0, x);
-              if (j < n0 && __ldg(E0 + j) == x) em = 1;
-            } else {
-              const int j = lower_bound2(Et, startE, nE, x);
-              if (j < nE) {
-                const int2 y = Et[j];
-                if (y.x == x) em = y.y;
-              }
-            }
-            if (em >= 0) {
-              atomicSub(&sg->mh[em], 1u);
-              atomicAdd(&sg->mh[em | (1 << p)], 1u);
-            }
-          }
-        } else {
-          for (int i = startE + gl; i < nE; i += W) {
-            int ev, em;
-            if (t == 0) {
-              ev = __ldg(E0 + i);
-              em = 1;
-            } else {
-              const int2 x = Et[i];
-              ev = x.x;
-              em = x.y;
-            }
-            const int m = em | (contains(Nw, dw, ev) ? (1 << p) : 0);
-            atomicAdd(&sg->mh[m], 1u);
-          }
         }
-        // excl(w) = N(w) above v0 minus U_t
-        unsigned inter = 0;
-        if ((long long)usize <= (long long)above * (t + 1)) {
-          // iterate U_t, probe N(w)
-          for (int i = gl; i < n0; i += W) inter += contains(Nw, dw, __ldg(E0 + i)) ? 1u : 0u;
-          for (int r = 1; r <= t; ++r) {
-            const int2* R = run_at(r);
-            const int nr = sg->runn[r];
-            for (int i = gl; i < nr; i += W) inter += contains(Nw, dw, R[i].x) ? 1u : 0u;
-          }
-        } else {
-          // iterate N(w) above v0, probe the runs
-          for (int i = sw0 + gl; i < dw; i += W)
-            inter += (use_bits ? bit_test(Ub, Nw[i] - c.bit_base)
-                               : in_runs(Nw[i], E0, n0, runs1, rstride, sg->runn, t)) ? 1u : 0u;
+      };
+      // depth-first over levels; level t's current vertex is w with mask wmask
+      while (true) {
+        // here the prefix is v_0..v_t plus w = v_{t+1}
+        const int p = t + 1;  // position of w
+        if (p > level) {
+          // nodes at or above a donated prefix's level belong to the donor
+          ++nodes;
+          if (gl == 0 && (nodes & 255) == 0) atomicAdd(&c.lb.ctr->progress, 256ull);
         }
-        for (int o = W / 2; o > 0; o >>= 1) inter += __shfl_xor_sync(gmask, inter, o);
-        if (gl == 0) {
-          const unsigned ex = (unsigned)above - inter;
-          if (ex) atomicAdd(&sg->mh[1 << p], ex);
-        }
-        __syncwarp(gmask);
-        flush_masks<W, (1 << (K - 1))>(sg, c.q2c, quick_p, leaf_off, hist, task_cnt, gl, gmask);
-        }
-      } else {
+        unsigned quick_p = (t == 0) ? 0u : sg->quick[t];
+        if (p >= 2) quick_p += ((unsigned)wmask & ((1u << p) - 1u)) << quick_off(p);
+        const int32_t* Nw = c.g.adj + __ldg(c.g.row + w);
+        const int dw = __ldg(c.g.deg + w);
+        // inherited members: e in E_t with e > w. E_t is sorted by vertex id and w is its
+        // member at position pos[t] - 1 (E_0: index it), so they are the suffix from there.
+        const int2* Et = t == 0 ? nullptr : ext_at(t);
+        const int nE = (t == 0) ? n0 : sg->n[t];
+        const int startE = (t == 0) ? it + 1 : sg->pos[t];
         // materialise E_{p} = inherited + excl(w), merged by vertex id; excl(w) is also run
         // p. Both parts are sorted and disjoint, so each member's place is its index in its
         // own part plus the number of smaller members of the other part.
@@ -522,47 +646,48 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, unsigned long 
           sg->runn[p] = rn;
           sg->quick[p] = quick_p;
         }
+        __syncwarp(gmask);
+        t = p;  // descend
         if (p == K - 3) {
-          for (int i = gl; i < 32; i += W) sg->sh[i] = 0;
-          __syncwarp(gmask);
-          mask_hist<W>(Ep, first_pos, m, sg->sh, gl, gmask);
+          // the last two vertices in bulk
+          int last = first_pos;
+          task_cnt += leaf_sweep<K, W>(c, hist, sw, Ep, m, first_pos, &sg->lim[p], v0, quick_p, Ub, E0, n0, runs1, rstride,
+                                       sg->runn, gl, gsrc, gmask, [&](int next) {
+                                         const unsigned long long before = nodes;
+                                         nodes += (unsigned long long)(next - last);
+                                         last = next;
+                                         if (gl == 0) {
+                                           sg->pos[p] = next;
+                                           if ((nodes ^ before) >> 8) atomicAdd(&c.lb.ctr->progress, 256ull);
+                                         }
+                                         __syncwarp(gmask);
+                                         give();
+                                       });
         }
-        __syncwarp(gmask);
-        t = p;  // descend; pick the first member below
-      }
-      // give work away when warps are hungry (checked every 16 expansions)
-      if (K >= 4 && (nodes & 15) == 0) {
-        if (gl == 0) motif_try_donate(c.lb, ws, sg, v0, floor, t, it, n0, t_start);
-        __syncwarp(gmask);
-      }
-      // next vertex: advance the deepest level that still has members
-      bool found = false;
-      while (t >= floor) {
-        const int ps = sg->pos[t];
-        if (ps < sg->lim[t]) {
-          const int2 x = ext_at(t)[ps];
-          __syncwarp(gmask);
-          if (gl == 0) {
-            sg->pos[t] = ps + 1;
-            if (t == K - 3) sg->sh[x.y] -= 1u;
+        give();
+        // next vertex: advance the deepest level that still has members
+        bool found = false;
+        while (t >= floor) {
+          const int ps = sg->pos[t];
+          if (ps < sg->lim[t]) {
+            const int2 x = ext_at(t)[ps];
+            __syncwarp(gmask);
+            if (gl == 0) sg->pos[t] = ps + 1;
+            __syncwarp(gmask);
+            w = x.x;
+            wmask = x.y;
+            found = true;
+            break;
           }
-          __syncwarp(gmask);
-          w = x.x;
-          wmask = x.y;
-          found = true;
-          break;
+          --t;
         }
-        --t;
+        if (!found) break;
       }
-      if (!found) break;
+      if (use_bits) drop_levels(1);
+      if (bad) break;
     }
-    if (use_bits) drop_levels(1);
-    if (bad) break;
   }
-  if (use_bits) {
-    bits_flip_ids<W>(Ub, c.bit_base, E0, n0, false, gl);
-    if (K == 3) bits_flip_ids<W>(Eb, c.bit_base, E0, n0, false, gl);
-  }
+  if (use_bits) bits_flip_ids<W>(Ub, c.bit_base, E0, n0, false, gl);
   __syncwarp();
   if (c.per_root) {
     const unsigned long long tsum = warp_sum_u64(task_cnt);

@@ -1,0 +1,61 @@
+"""The motif kernel's bulk count of the last two vertices (GPU) against the enumerating oracle:
+extension sets below, at and above a group's width, rows longer than the group, dense cores
+(joined pairs), donated ranges in the middle of a set, shards and subtree logs. Exact counts."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def graph(dm, kind):
+    rng = np.random.default_rng(17)
+    if kind == "clique":
+        u, v = np.triu_indices(13, 1)
+    elif kind == "wheel":      # a hub whose rows are longer than a group, and a rim
+        u = np.concatenate([np.zeros(45, int), np.arange(1, 45)])
+        v = np.concatenate([np.arange(1, 46), np.arange(2, 46)])
+    elif kind == "star33":
+        u, v = np.zeros(33, int), np.arange(1, 34)
+    else:                      # sparse with a dense core, ids shuffled
+        a, b = np.triu_indices(8, 1)
+        ids = rng.permutation(90)
+        u = np.concatenate([rng.integers(0, 90, 130), ids[a]])
+        v = np.concatenate([rng.integers(0, 90, 130), ids[b]])
+    return dm.Graph.from_edges(u, v)
+
+
+@pytest.mark.parametrize("vwarp", [8, 16, 32])
+@pytest.mark.parametrize("k", [4, 5, 6, 7])
+@pytest.mark.parametrize("kind", ["clique", "wheel", "star33", "core"])
+def test_sweep_vs_oracle(dm, orc, gpu, kind, k, vwarp):
+    if kind in ("wheel", "star33") and k == 7:
+        pytest.skip("too many subgraphs for the oracle")
+    g = graph(dm, kind)
+    og = orc.OracleGraph.from_pairs(*g.edges())
+    d = dm.Dictionary.generate(k)
+    want = orc.motifs(og, k, d.tables()[0], d.n_classes)
+    for flags in (0, dm.TEST_EAGER_DONATION):
+        per = np.zeros(g.info().n_vertices, np.uint64)
+        got, _ = dm.count_motifs(g, k, d, dm.Options(vwarp=vwarp, test_flags=flags, subtree_counts=per))
+        assert np.array_equal(got, want), flags
+        assert int(per.sum()) == int(want.sum())
+    parts = [dm.count_motifs(g, k, d, dm.Options(vwarp=vwarp, rank=r, world_size=3))[0] for r in range(3)]
+    assert np.array_equal(sum(parts), want)
+
+
+@pytest.mark.parametrize("q", [4, 5, 6, 9])
+def test_near_cliques_of_wide_universes(dm, orc, gpu, q):
+    """Edges with more than 256 common neighbours, and rows beyond a warp's shared memory."""
+    rng = np.random.default_rng(q)
+    a, b = np.triu_indices(24, 1)
+    core = [(int(x), int(y)) for x, y in zip(a, b) if rng.random() < 0.8]
+    outer = [(24 + i, int(c)) for i in range(400) for c in rng.choice(24, 9, replace=False)]
+    s, t = np.array(core + outer).T
+    g = dm.Graph.from_edges(s, t)
+    og = orc.OracleGraph.from_pairs(*g.edges())
+    want = orc.near_cliques(og, q)
+    assert dm.count_near_cliques(g, q)[0] == want
+    assert sum(dm.count_near_cliques(g, q, dm.Options(rank=r, world_size=3))[0] for r in range(3)) == want
+    assert dm.count_near_cliques(g, q, dm.Options(threads=256))[0] == want
