@@ -1225,20 +1225,16 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
   if ((rc = prepare_ws(ws, ctx.stream))) return rc;
   DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
   if (!s->dg.has_oriented && (rc = upload_clique_image(g, s, ctx.stream))) return rc;
-  if (!s->dg.has_undirected) {
-    rc = upload_csr(g, g->row, g->adj, g->n, g->pad_row[0], g->pad_deg[0], g->pad_adj[0], &s->dg.d_row, &s->dg.d_deg,
-                    &s->dg.d_adj, ctx.stream);
-    if (rc) return rc;
-    s->dg.has_undirected = true;
-  }
-  if ((rc = ensure_deg_order(g, s, ctx.stream)) || (rc = ensure_orig(g, s, ctx))) return rc;
+  if ((rc = ensure_deg_order(g, s, ctx.stream))) return rc;
+  if ((rc = ensure_census(g, s, 4, ctx))) return rc < 0 ? rc : fail(DM_ENOMEM, "no device memory for the in-lists");
   const int c = n - 2;
   const int need = c - 1;  // out-neighbours a root needs to start a c-clique
   const int world = (o && o->world_size > 1) ? o->world_size : 1;
   int n_roots = need <= g->max_out_degree ? (int)g->cnt_ge[need] : 0;
   const int32_t* d_roots = s->d_deg_order;
+  const int32_t* h_roots = g->deg_order.data();
+  std::vector<int32_t> mine;
   if (world > 1) {
-    std::vector<int32_t> mine;
     for (int i = o->rank; i < n_roots; i += world) mine.push_back(g->deg_order[i]);
     if ((rc = ensure_ws_bytes(reinterpret_cast<void**>(&ws.d_tasks), &ws.tasks_cap,
                               sizeof(int32_t) * (mine.size() + 1))))
@@ -1247,32 +1243,65 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
       DM_CUDA(cudaMemcpyAsync(ws.d_tasks, mine.data(), sizeof(int32_t) * mine.size(), cudaMemcpyHostToDevice,
                               ctx.stream));
     d_roots = ws.d_tasks;
+    h_roots = mine.data();
     n_roots = (int)mine.size();
   }
+  // the items are the roots' out-edges: runs of equal out-degree number them
+  std::vector<NearStep> steps;
+  int64_t items = 0;
+  for (int i = 0; i < n_roots;) {
+    const int32_t d = (int32_t)(g->orow[h_roots[i] + 1] - g->orow[h_roots[i]]);
+    int j = i;
+    if (world == 1) j = (int)std::min<int64_t>(n_roots, g->cnt_ge[d]);
+    else
+      while (j < n_roots && g->orow[h_roots[j] + 1] - g->orow[h_roots[j]] == d) ++j;
+    steps.push_back(NearStep{(int32_t)items, i, d, 0});
+    items += (int64_t)(j - i) * d;
+    i = j;
+  }
+  if ((rc = ensure_ws_bytes(reinterpret_cast<void**>(&ws.d_parts), &ws.parts_cap, sizeof(NearStep) * (steps.size() + 1))))
+    return rc;
+  if (!steps.empty())
+    DM_CUDA(cudaMemcpyAsync(ws.d_parts, steps.data(), sizeof(NearStep) * steps.size(), cudaMemcpyHostToDevice,
+                            ctx.stream));
   NearLaunch L;
   L.dag = GraphView{s->dg.d_orow, s->dg.d_odeg, s->dg.d_oadj, g->n};
-  L.und = GraphView{s->dg.d_row, s->dg.d_deg, s->dg.d_adj, g->n};
-  L.orig = s->d_orig;
+  L.in_end = s->d_in_end;
+  L.in_deg = s->d_in_deg;
+  L.in = s->d_in;
   L.roots = d_roots;
-  L.n_roots = n_roots;
+  L.steps = ws.d_parts;
+  L.n_steps = (int)steps.size();
+  L.n_items = (int)items;
   L.c = c;
   L.ctr = ws.d_ctr;
-  L.queue = ws.d_queue;
-  L.qcap = ws.qcap;
-  L.nq = QUEUE_SHARDS;
-  L.dag_cap = g->max_out_degree + 4;
-  L.und_cap = g->max_degree + 4;
-  const size_t per_warp = near_clique_warp_ints(c, L.dag_cap, L.und_cap) * sizeof(int32_t);
-  ctx.arena_warps = (int)std::min<size_t>((size_t)ctx.num_sms * 64, std::max<size_t>(8, ((size_t)8 << 30) / per_warp));
-  if ((rc = ensure_ws_bytes(&ws.d_scratch, &ws.scratch_cap, per_warp * ctx.arena_warps))) return rc;
-  L.arena = reinterpret_cast<int32_t*>(ws.d_scratch);
-  if ((rc = init_counters(ws, n_roots, ctx.stream))) return rc;
+  if (g->near_rows < 0) {
+    // the largest universe and rows that an edge of this graph can have
+    g->near_list = 0;
+    g->near_rows = 0;
+    for (int32_t r = 0; r < g->n; ++r) {
+      const int d = (int)(g->orow[r + 1] - g->orow[r]);
+      if (d < 1) continue;
+      g->near_list = std::max(g->near_list, g->udeg[r]);
+      g->near_rows = std::max(g->near_rows, (int64_t)near_clique_rows(d, g->udeg[r]));
+    }
+  }
+  ctx.arena_warps = ctx.num_sms * 64;
+  if (g->near_rows > 0) {
+    L.list_cap = g->near_list + 32;
+    L.arena_ints = ((size_t)L.list_cap + (size_t)g->near_rows + 63) / 64 * 64;
+    const size_t per_warp = L.arena_ints * sizeof(int32_t);
+    ctx.arena_warps = (int)std::min<size_t>((size_t)ctx.num_sms * 64, std::max<size_t>(8, ((size_t)8 << 30) / per_warp));
+    if ((rc = ensure_ws_bytes(&ws.d_scratch, &ws.scratch_cap, per_warp * ctx.arena_warps))) return rc;
+    L.arena = reinterpret_cast<int32_t*>(ws.d_scratch);
+  }
+  if ((rc = init_counters(ws, (int)items, ctx.stream))) return rc;
   DM_CUDA(cudaEventRecord(ws.k0, ctx.stream));
   int grid = 0;
   Reporter reporter;
-  if (n_roots > 0) {
+  if (items > 0) {
     if ((rc = near_clique_launch(L, ctx, &grid))) return rc;
-    if ((rc = reporter.start(o, ctx.device, ws.d_ctr, grid * 8, n_roots))) return rc;
+    if ((rc = reporter.start(o, ctx.device, ws.d_ctr, grid * 8, items))) return rc;
   }
   DM_CUDA(cudaEventRecord(ws.k1, ctx.stream));
   DM_CUDA(cudaMemcpyAsync(ws.h_out, ws.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, ctx.stream));

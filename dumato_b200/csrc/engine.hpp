@@ -160,20 +160,25 @@ int clique_index_build(const GraphView& g, const int32_t* roots, int n, void* bl
 // Pattern-aware queries q4..q13 (near_clique.cu): (n-2)-cliques and their common neighbours.
 struct NearLaunch {
   GraphView dag;                   // rank space
-  GraphView und;                   // undirected, original ids
-  const int32_t* orig = nullptr;   // rank -> original id
-  const int32_t* roots = nullptr;
-  int n_roots = 0;
+  const int32_t* in_end = nullptr; // in-lists (census_in_lists)
+  const int32_t* in_deg = nullptr;
+  const void* in = nullptr;
+  const int32_t* roots = nullptr;  // by descending out-degree
+  const void* steps = nullptr;     // NearStep[n_steps]
+  int n_steps = 0;
+  int n_items = 0;                 // out-edges of the roots
   int c = 2;                       // clique size n - 2
   DevCounters* ctr = nullptr;
-  void* queue = nullptr;
-  int qcap = 0;
-  int nq = 1;
-  int32_t* arena = nullptr;        // near_clique_warp_ints ints per warp
-  int dag_cap = 0, und_cap = 0;
+  int32_t* arena = nullptr;        // arena_ints per warp, or null
+  size_t arena_ints = 0;
+  int list_cap = 0;
+};
+// A run of roots of equal out-degree: its first item (out-edge), first root, out-degree.
+struct NearStep {
+  int32_t item, root, deg, pad;
 };
 int near_clique_launch(const NearLaunch& L, LaunchCtx& ctx, int* grid);
-size_t near_clique_warp_ints(int c, int dag_cap, int und_cap);
+size_t near_clique_rows(int d, int deg);  // arena ints (beyond the list) for a root's edges
 
 // Whole-graph census of the connected 3- and 4-vertex classes (census.cu).
 constexpr int CENSUS_SUMS = 9;

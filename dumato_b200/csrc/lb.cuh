@@ -168,6 +168,18 @@ static __device__ __noinline__ bool q_pop(const LBArgs& lb, int home, int& root,
   return false;
 }
 
+// Test hook: waits for test_gate, which nothing sets, until the bounded wait gives up.
+static __device__ __noinline__ void lb_stall(const LBArgs& lb) {
+  const long long ts = global_ns();
+  while (vload(&lb.ctr->test_gate) == 0) {
+    if (global_ns() - ts > lb.timeout_ns) {
+      set_err(lb.ctr, ERR_TIMEOUT);
+      break;
+    }
+    __nanosleep(2000);
+  }
+}
+
 // Lane-0 only. Claims a chunk of roots [first, first+count) from the cursor, or failing
 // that a donated task (count = 1, range [b, e)). Returns false when all work is done or an
 // error was raised. A caller that defers the pending-count decrements of the roots it has
@@ -220,15 +232,7 @@ static __device__ __noinline__ bool lb_next(const LBArgs& lb, int n_roots, int t
     }
     const int pend = vload(&c->pending);
     if (pend <= 0 && lb.test_stall) {
-      // test hook: wait for test_gate, which nothing sets, until the bounded wait gives up
-      const long long ts = global_ns();
-      while (vload(&c->test_gate) == 0) {
-        if (global_ns() - ts > lb.timeout_ns) {
-          set_err(c, ERR_TIMEOUT);
-          break;
-        }
-        __nanosleep(2000);
-      }
+      lb_stall(lb);
       break;
     }
     if (pend <= 0 || vload(&c->err) != 0) break;

@@ -8,11 +8,22 @@
 // of K_n minus one edge - and the count is
 //     q_n = sum over (n-2)-cliques C of  t_C (t_C - 1) / 2,   t_C = |common neighbourhood of C|.
 //
-// Here each (n-2)-clique is found once, from its lowest-ranked vertex, by a warp-cooperative
-// list DFS on the degree-ordered DAG (dm_gpm::extend_intersect), and t_C is the size of the
-// intersection of the members' rows in the undirected CSR (original ids), computed from the
-// shortest row by dm_gpm::extend_intersect / intersect_count. Root tasks are claimed from the
-// shared cursor in runs (lb.cuh); there is no donation in this kernel.
+// Here an (n-2)-clique C is found once on the degree-ordered DAG, from its two lowest-ranked
+// vertices r -> v, and one warp takes each DAG edge. Every other vertex of C and every common
+// neighbour of C lies in N(r) cap N(v), the edge's triangles, so the warp lists that universe
+// (the members of it that r and v both point to first: the candidates for C, ascending), builds
+// one bitmap row over the universe per candidate, and from there only ANDs rows:
+// X = the universe cap the rows of the members chosen so far holds both the candidates left and
+// the common neighbours, and t_C = popc(X & row of the last member), one last member per lane.
+// Edges are numbered by descending out-degree of r, so the heaviest start first, and claimed in
+// runs from a cursor.
+//
+// Bound by the dependent loads of the membership searches that build the rows (one binary search
+// in an out-row per universe vertex and candidate, 32 side by side); the counting is AND + popc
+// from shared memory. Taking a whole root per warp and intersecting undirected adjacency lists
+// for every clique again, as this kernel did before, read whole rows per clique and left the
+// heaviest roots on one warp each: q_6 on an R-MAT graph of 1,377 vertices and 8,000 edges took
+// 7,867 us per call, now 76 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -26,160 +37,172 @@
 namespace dmb {
 
 struct NearArgs {
-  GraphView dag;          // rank-space out-lists
-  GraphView und;          // undirected CSR, original ids
-  const int32_t* orig;    // rank -> original id
-  const int32_t* roots;   // roots (rank space)
-  int n_roots;
+  GraphView dag;            // rank-space out-lists
+  const int32_t* in_end;    // in-lists (census_in_lists)
+  const int32_t* in_deg;
+  const int2* in;
+  const int32_t* roots;     // by descending out-degree
+  const int4* steps;        // (first item, first root, out-degree): runs of equal out-degree
+  int n_steps, n_items;
   LBArgs lb;
-  int32_t* arena;         // per warp: C levels of dag_cap ints, then 2 lists of und_cap ints
-  int dag_cap, und_cap;
+  int32_t* arena;           // per warp: list, rows, sets that do not fit shared memory; or null
+  size_t arena_ints;
+  int list_cap;             // universe vertices an edge can have
 };
 
 constexpr int NEAR_WARPS = 8;
+// shared memory of a warp: universes of up to 256 vertices and 1,024 row words (the rest of the
+// edges, a few around hubs, use the arena)
+constexpr int NEAR_LIST = 256;
+constexpr int NEAR_ROWS = 1024;
+constexpr int NEAR_SETS = 9;  // nested sets X (n = 13 chooses nine members from the candidates)
+constexpr int NEAR_WARP_INTS = NEAR_LIST + NEAR_ROWS + NEAR_SETS * (NEAR_LIST / 32);
 
-// t (t - 1) / 2 for the common neighbourhood of the clique held in members[0..C) (rank space).
-template <int C>
-__device__ unsigned long long near_pairs(const NearArgs& a, const int32_t* members, int32_t* s0, int32_t* s1) {
-  // the member with the shortest undirected row first
-  int best = 0, best_deg = INT_MAX;
-  int32_t ids[C];
-#pragma unroll
-  for (int i = 0; i < C; ++i) {
-    ids[i] = __ldg(a.orig + members[i]);
-    const int dg = __ldg(a.und.deg + ids[i]);
-    if (dg < best_deg) {
-      best_deg = dg;
-      best = i;
+// Adds t (t - 1) / 2 over the cliques that extend the members chosen so far by LEFT more
+// candidates from index `start` on. X: the candidates and common neighbours left (null: the whole
+// universe); sets: room for the sets below. Warp-uniform but for the last member.
+template <int LEFT>
+__device__ __forceinline__ void near_dfs(const uint32_t* rows, int W, int m, const uint32_t* X, uint32_t* sets, int start,
+                                         unsigned long long& total) {
+  const int lane = lane_id();
+  if constexpr (LEFT == 1) {
+    for (int j = start + lane; j < m; j += 32) {
+      if (X && !((X[j >> 5] >> (j & 31)) & 1u)) continue;
+      unsigned t = 0;
+      for (int w = 0; w < W; ++w) t += __popc(rows[j * W + w] & (X ? X[w] : 0xffffffffu));
+      total += (t & 1) ? (unsigned long long)t * ((t - 1) >> 1) : (unsigned long long)(t >> 1) * (t - 1u);
     }
-  }
-  const int32_t* cur = a.und.adj + __ldg(a.und.row + ids[best]);
-  int n = best_deg;
-  int t = 0;
-  int done = 1;
-#pragma unroll
-  for (int i = 0; i < C; ++i) {
-    if (i == best) continue;
-    const int32_t* B = a.und.adj + __ldg(a.und.row + ids[i]);
-    const int nb = __ldg(a.und.deg + ids[i]);
-    if (++done == C) {
-      t = dm_gpm::intersect_count<32>(cur, n, B, nb);
-    } else {
-      int32_t* out = (done & 1) ? s0 : s1;
-      n = dm_gpm::extend_intersect<32>(cur, n, B, nb, out);
+  } else {
+    for (int j = start; j <= m - LEFT; ++j) {
+      if (X && !((X[j >> 5] >> (j & 31)) & 1u)) continue;
+      const uint32_t* Y = rows + (size_t)j * W;
+      if (X) {
+        for (int w = lane; w < W; w += 32) sets[w] = X[w] & Y[w];
+        __syncwarp();
+        Y = sets;
+      }
+      // candidates left above j
+      int left = 0;
+      for (int w = (j + 1) >> 5; w <= (m - 1) >> 5; ++w) {
+        uint32_t b = Y[w];
+        if (w == (j + 1) >> 5) b &= 0xffffffffu << ((j + 1) & 31);
+        if (w == (m - 1) >> 5) b &= 0xffffffffu >> (31 - ((m - 1) & 31));
+        left += __popc(b);
+      }
+      if (left >= LEFT - 1) near_dfs<LEFT - 1>(rows, W, m, Y, X ? sets + W : sets, j + 1, total);
       __syncwarp();
-      cur = out;
-    }
-    if (n == 0) {
-      t = 0;
-      break;
     }
   }
-  return (unsigned long long)t * (unsigned long long)(t > 0 ? t - 1 : 0) / 2ull;
 }
 
 template <int C>
 __global__ void __launch_bounds__(32 * NEAR_WARPS) near_clique_kernel(const __grid_constant__ NearArgs a) {
-  __shared__ int sN[NEAR_WARPS][C > 1 ? C : 2], sPos[NEAR_WARPS][C > 1 ? C : 2];
-  __shared__ int32_t sMem[NEAR_WARPS][C];
+  __shared__ int32_t smem[NEAR_WARPS][NEAR_WARP_INTS];
   const int lane = lane_id();
   const int wib = warp_in_block();
-  const int gw = blockIdx.x * NEAR_WARPS + wib;
   const int total_warps = gridDim.x * NEAR_WARPS;
-  int32_t* base = a.arena + (size_t)gw * ((size_t)C * a.dag_cap + 2 * (size_t)a.und_cap);
-  int32_t* s0 = base + (size_t)C * a.dag_cap;
-  int32_t* s1 = s0 + a.und_cap;
-  int* N = sN[wib];
-  int* Pos = sPos[wib];
-  int32_t* mem = sMem[wib];
-  unsigned long long cnt = 0, ntasks = 0;
+  int32_t* own = smem[wib];
+  int32_t* arena = a.arena ? a.arena + (size_t)(blockIdx.x * NEAR_WARPS + wib) * a.arena_ints : nullptr;
+  DevCounters* ctr = a.lb.ctr;
+  unsigned long long total = 0, ntasks = 0;
   while (true) {
-    int first = 0, count = 0, b = 0, e = -1, ok = 0, level = 0;
-    int path[QPATH];
-    bool donated = false;
-    if (lane == 0) ok = lb_next(a.lb, a.n_roots, total_warps, first, count, b, e, donated, level, path) ? 1 : 0;
-    ok = __shfl_sync(FULL_MASK, ok, 0);
-    if (!ok) break;
+    int first = 0, count = 0;
+    if (lane == 0) {
+      const int left = a.n_items - vload(&ctr->cursor);
+      const int chunk = max(1, min(16, left / (8 * total_warps)));
+      first = left > 0 ? atomicAdd(&ctr->cursor, chunk) : a.n_items;
+      count = min(chunk, a.n_items - first);
+    }
     first = __shfl_sync(FULL_MASK, first, 0);
     count = __shfl_sync(FULL_MASK, count, 0);
+    if (count <= 0) break;
     ntasks += count;
-    for (int ti = 0; ti < count; ++ti) {
-      const int root = __ldg(a.roots + first + ti);
-      if (lane == 0) mem[0] = root;
-      const int32_t* L = a.dag.adj + __ldg(a.dag.row + root);
-      const int d = __ldg(a.dag.deg + root);
+    for (int e = first; e < first + count; ++e) {
+      // item e: out-edge i of root o, found through the runs of roots of equal out-degree
+      int lo = 0, hi = a.n_steps;
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(&a.steps[mid].x) <= e) lo = mid; else hi = mid;
+      }
+      const int4 st = __ldg(a.steps + lo);
+      const int d = st.z;
+      const int o = st.y + (e - st.x) / d, i = (e - st.x) % d;
+      if (d - 1 - i < C - 2) continue;
+      const int r = __ldg(a.roots + o);
+      const int32_t* L = a.dag.adj + __ldg(a.dag.row + r);
+      const int v = __ldg(L + i);
+      const int32_t* B = a.dag.adj + __ldg(a.dag.row + v);
+      const int nb = __ldg(a.dag.deg + v);
+      const int nin = __ldg(a.in_deg + r);
+      int32_t* uni = d + nin <= NEAR_LIST ? own : arena;
+      // candidates: above v, and out-neighbours of both
+      int m = 0;
+      for (int j0 = i + 1; j0 < d; j0 += 32) {
+        const int j = j0 + lane;
+        const int y = j < d ? __ldg(L + j) : 0;
+        m += compact(uni, m, y, j < d && contains(B, nb, y));
+      }
+      if (m < C - 2) continue;
+      // the other common neighbours lie below v: v is in their out-row
+      int u = m;
+      for (int j0 = 0; j0 < i; j0 += 32) {
+        const int j = j0 + lane;
+        const int y = j < i ? __ldg(L + j) : 0;
+        u += compact(uni, u, y, j < i && contains(a.dag.adj + __ldg(a.dag.row + y), __ldg(a.dag.deg + y), v));
+      }
+      const int2* I = a.in + (__ldg(a.in_end + r) - nin);
+      for (int j0 = 0; j0 < nin; j0 += 32) {
+        const int j = j0 + lane;
+        const int y = j < nin ? __ldg(&I[j].x) : 0;
+        u += compact(uni, u, y, j < nin && contains(a.dag.adj + __ldg(a.dag.row + y), __ldg(a.dag.deg + y), v));
+      }
+      __syncwarp();
       if constexpr (C == 2) {
-        for (int i = 0; i < d; ++i) {
-          if (lane == 0) mem[1] = __ldg(L + i);
-          __syncwarp();
-          cnt += near_pairs<C>(a, mem, s0, s1);
-          __syncwarp();
-        }
+        if (lane == 0) total += (u & 1) ? (unsigned long long)u * ((u - 1) >> 1) : (unsigned long long)(u >> 1) * (u - 1);
       } else {
-        // level l (1..C-1) holds the candidates of the (l+1)-th member: level 1 = N+(root)
-        if (lane == 0) {
-          N[1] = d;
-          Pos[1] = 0;
+        const int W = (u + 31) >> 5;
+        const bool small = u <= NEAR_LIST && m * W <= NEAR_ROWS;
+        uint32_t* rows = reinterpret_cast<uint32_t*>(small ? own + NEAR_LIST : arena + a.list_cap);
+        uint32_t* sets = small ? rows + NEAR_ROWS : rows + (size_t)m * W;
+        for (int w = 0; w < W; ++w) {
+          const int q = w * 32 + lane;
+          const int y = q < u ? uni[q] : 0;
+          const int32_t* Ny = a.dag.adj + __ldg(a.dag.row + y);
+          const int ny = __ldg(a.dag.deg + y);
+          for (int j = 0; j < m; ++j) {
+            const int c = uni[j];
+            bool adj = false;
+            if (q < u && y < c) adj = contains(Ny, ny, c);
+            if (q < u && y > c) adj = contains(a.dag.adj + __ldg(a.dag.row + c), __ldg(a.dag.deg + c), y);
+            const unsigned bits = __ballot_sync(FULL_MASK, adj);
+            if (lane == 0) rows[j * W + w] = bits;
+          }
         }
         __syncwarp();
-        int lvl = 1;
-        while (lvl >= 1) {
-          const int pos = Pos[lvl];
-          const int rem = N[lvl] - pos;
-          if (rem < C - lvl) {  // not enough candidates left to complete the clique
-            --lvl;
-            continue;
-          }
-          const int32_t* P = lvl == 1 ? L : base + (size_t)lvl * a.dag_cap;
-          const int v = P[pos];
-          __syncwarp();
-          if (lane == 0) {
-            Pos[lvl] = pos + 1;
-            mem[lvl] = v;
-            if ((pos & 63) == 63) atomicAdd(&a.lb.ctr->progress, 64ull);
-          }
-          __syncwarp();
-          if (lvl == C - 1) {
-            cnt += near_pairs<C>(a, mem, s0, s1);
-            __syncwarp();
-            continue;
-          }
-          const int32_t* B = a.dag.adj + __ldg(a.dag.row + v);
-          const int nb = __ldg(a.dag.deg + v);
-          const int m = dm_gpm::extend_intersect<32>(P + pos + 1, rem - 1, B, nb, base + (size_t)(lvl + 1) * a.dag_cap);
-          __syncwarp();
-          if (lane == 0) {
-            N[lvl + 1] = m;
-            Pos[lvl + 1] = 0;
-          }
-          __syncwarp();
-          ++lvl;
-        }
+        near_dfs<C - 2>(rows, W, m, nullptr, sets, 0, total);
       }
       __syncwarp();
     }
-    if (lane == 0) lb_done(a.lb, count);
   }
-  // near_pairs returns the same value on every lane: count it once per warp
+  if (lane == 0 && a.lb.test_stall) lb_stall(a.lb);
+  total = warp_sum_u64(total);
   if (lane == 0) {
-    atomicAdd(&a.lb.ctr->count, cnt);
-    atomicAdd(&a.lb.ctr->tasks, ntasks);
+    if (total) atomicAdd(&ctr->count, total);
+    atomicAdd(&ctr->tasks, ntasks);
   }
 }
 
 template <int C>
-static int launch_near(const NearArgs& a0, LaunchCtx& ctx, int* grid_out) {
+static int launch_near(const NearArgs& a, LaunchCtx& ctx, int* grid_out) {
   const int block = 32 * NEAR_WARPS;
   auto kern = near_clique_kernel<C>;
   static LaunchCache cache;
   int occ = 0;
   DM_CUDA(cached_occupancy(cache, kern, ctx.device, block, 0, &occ));
   if (occ < 1) return fail(DM_EINVAL, "near-clique kernel does not fit on an SM");
-  int grid = ctx.num_sms * occ;
+  int grid = std::min(ctx.num_sms * occ, (a.n_items + NEAR_WARPS - 1) / NEAR_WARPS);
   if (ctx.threads > 0) grid = std::max(1, std::min(grid, (ctx.threads + block - 1) / block));
-  if (grid * NEAR_WARPS > ctx.arena_warps) grid = std::max(1, ctx.arena_warps / NEAR_WARPS);
-  NearArgs a = a0;
-  a.lb.hungry_trigger = 0;  // no donation in this kernel
+  if (a.arena && grid * NEAR_WARPS > ctx.arena_warps) grid = std::max(1, ctx.arena_warps / NEAR_WARPS);
   kern<<<grid, block, 0, ctx.stream>>>(a);
   ctx.launches++;
   *grid_out = grid;
@@ -190,17 +213,20 @@ static int launch_near(const NearArgs& a0, LaunchCtx& ctx, int* grid_out) {
 int near_clique_launch(const NearLaunch& L, LaunchCtx& ctx, int* grid) {
   NearArgs a;
   a.dag = L.dag;
-  a.und = L.und;
-  a.orig = L.orig;
+  a.in_end = L.in_end;
+  a.in_deg = L.in_deg;
+  a.in = reinterpret_cast<const int2*>(L.in);
   a.roots = L.roots;
-  a.n_roots = L.n_roots;
-  a.lb = LBArgs{L.ctr, reinterpret_cast<QHeader*>(L.queue),
-                reinterpret_cast<QSlot*>(reinterpret_cast<char*>(L.queue) + sizeof(QHeader) * L.nq), L.qcap, 0, 0,
-                (long long)ctx.donate_after_us * 1000ll, (long long)ctx.timeout_ms * 1000000ll, ctx.test_stall, 32,
-                L.nq};
+  a.steps = reinterpret_cast<const int4*>(L.steps);
+  a.n_steps = L.n_steps;
+  a.n_items = L.n_items;
+  a.lb = LBArgs{};
+  a.lb.ctr = L.ctr;
+  a.lb.timeout_ns = (long long)ctx.timeout_ms * 1000000ll;
+  a.lb.test_stall = ctx.test_stall;
   a.arena = L.arena;
-  a.dag_cap = L.dag_cap;
-  a.und_cap = L.und_cap;
+  a.arena_ints = L.arena_ints;
+  a.list_cap = L.list_cap;
   switch (L.c) {
     case 2: return launch_near<2>(a, ctx, grid);
     case 3: return launch_near<3>(a, ctx, grid);
@@ -216,6 +242,11 @@ int near_clique_launch(const NearLaunch& L, LaunchCtx& ctx, int* grid) {
   }
 }
 
-size_t near_clique_warp_ints(int c, int dag_cap, int und_cap) { return (size_t)c * dag_cap + 2 * (size_t)und_cap; }
+// Ints of a warp's arena for edges of roots of out-degree d and degree `deg` (0: shared memory
+// holds every edge's universe, rows and sets).
+size_t near_clique_rows(int d, int deg) {
+  const size_t W = ((size_t)deg + 31) / 32, rows = (size_t)std::max(d - 1, 0) * W;
+  return deg <= NEAR_LIST && rows <= NEAR_ROWS ? 0 : rows + NEAR_SETS * W;
+}
 
 }  // namespace dmb
