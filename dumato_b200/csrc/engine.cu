@@ -365,7 +365,7 @@ static std::map<int, std::multimap<size_t, void*>> g_buf_pool;
 static size_t g_buf_pooled = 0;
 constexpr size_t BUF_POOL_MAX = (size_t)4 << 30;
 
-static cudaError_t gbuf_alloc(void** p, size_t bytes) {
+cudaError_t gbuf_alloc(void** p, size_t bytes) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -384,7 +384,7 @@ static cudaError_t gbuf_alloc(void** p, size_t bytes) {
   return e;
 }
 
-static void gbuf_free(void* p, int dev) {
+void gbuf_free(void* p, int dev) {
   if (!p) return;
   std::lock_guard<std::mutex> lk(g_buf_mu);
   auto it = g_buf_size.find(p);

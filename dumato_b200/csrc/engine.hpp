@@ -265,6 +265,10 @@ inline cudaError_t cached_occupancy(LaunchCache& c, Kern kern, int device, int b
 // Host helpers shared by the entry points (engine.cu).
 int select_device(const dm_opts* o, LaunchCtx& ctx);   // device, stream and options -> ctx
 int check_opts(const dm_opts* o);
+// Device buffers from the library's per-device pool (current device; safe from any thread). A
+// buffer is given back only once nothing on the device uses it any more.
+cudaError_t gbuf_alloc(void** p, size_t bytes);
+void gbuf_free(void* p, int dev);
 int queue_init_launch(void* queue, int nq, int cap, cudaStream_t st);  // empty donation queue
 constexpr int QUEUE_SHARDS = 64;        // donation-queue shards of a workspace
 constexpr int QUEUE_SHARD_SLOTS = 2048; // slots per shard

@@ -151,3 +151,41 @@ def test_learned_schedule_on_device_every_path(dm, orc, gpu):
     a, _ = dm.count_motifs(g, 3, d)
     shards = [dm.count_motifs(g, 3, d, dm.Options(**L, rank=r, world_size=2))[0] for r in range(2)]
     assert np.array_equal(a, shards[0] + shards[1])
+
+
+@pytest.mark.parametrize("n,batch", [(1, 1), (7, 3), (500, 256), (1000, 9), (700, 300), (5000, 4096), (9000, 4097)])
+def test_training_matches_float64_adam(dm, gpu, n, batch):
+    """Epoch kernel (batches up to 4,096) and per-step launches (above) against Adam in float64 over
+    the same minibatches: a block's share of a batch is empty, part of a tile, or several tiles.
+    Each step moves a parameter by at most about lr, with an FP32 relative error of a few ulps per
+    summed gradient: 1e-3 of a step per step bounds the drift."""
+    rng = np.random.default_rng(n)
+    X = rng.normal(size=(n, F)).astype(np.float32)
+    T = (X[:, 0] - 0.5 * X[:, 3] + 0.1 * rng.normal(size=n)).astype(np.float32)
+    epochs, lr, seed = 2, 3e-3, 11
+    pr = dm.Predictor(seed=seed)
+    p = pr.get_params().astype(np.float64)
+    loss = pr.train(X, T, epochs=epochs, batch=batch, lr=lr)
+    M = (1 << 64) - 1
+    s, order, steps = seed ^ 0x5DEECE66D, list(range(n)), 0
+    m, v = np.zeros_like(p), np.zeros_like(p)
+    b1, b2 = float(np.float32(0.9)), float(np.float32(0.999))
+    for _ in range(epochs):
+        for i in range(n - 1, 0, -1):  # Fisher-Yates from a splitmix64 chain
+            s = (s + 0x9E3779B97F4A7C15) & M
+            s = ((s ^ (s >> 30)) * 0xBF58476D1CE4E5B9) & M
+            s = ((s ^ (s >> 27)) * 0x94D049BB133111EB) & M
+            s ^= s >> 31
+            j = s % (i + 1)
+            order[i], order[j] = order[j], order[i]
+        total = 0.0
+        for off in range(0, n, batch):
+            q = order[off:off + batch]
+            _, mse, g = cpu_forward_backward(p, X[q], T[q])
+            total += mse * len(q)
+            steps += 1
+            m = b1 * m + (1 - b1) * g
+            v = b2 * v + (1 - b2) * g * g
+            p = p - lr * (m / (1 - b1 ** steps)) / (np.sqrt(v / (1 - b2 ** steps)) + 1e-8)
+    assert np.abs(pr.get_params() - p).max() <= 1e-3 * lr * steps + 1e-6
+    assert abs(loss - total / n) <= 1e-4 * max(1.0, total / n)
