@@ -215,7 +215,7 @@ class Graph:
         returns the graph and the device time in ms."""
         h = _P()
         ms = ctypes.c_double()
-        o = (opts or Options()).to_c()
+        o = (opts or _DEFAULT).to_c()
         _check(lib().dm_graph_load_edgelist_device(str(path).encode(), ctypes.byref(o), ctypes.byref(h),
                                                    ctypes.byref(ms)))
         return cls(h), ms.value
@@ -495,6 +495,10 @@ class Options:
         return fn
 
 
+# the options of a call that passes none: built once (the library only reads them)
+_DEFAULT = Options()
+
+
 @dataclass
 class Stats:
     kernel_ms: float = 0.0
@@ -544,7 +548,7 @@ TEST_EAGER_DONATION = 2
 
 def plan_roots(g: Graph, k: int, clique: bool = True, opts: Optional[Options] = None) -> tuple[np.ndarray, np.ndarray]:
     """The ordered root tasks (original ids, part words) this shard would run (host only)."""
-    o = (opts or Options()).to_c()
+    o = (opts or _DEFAULT).to_c()
     n = ctypes.c_int64()
     _check(lib().dm_plan_roots(g.handle, int(k), 1 if clique else 0, ctypes.byref(o), None, None, 0, ctypes.byref(n)))
     roots = np.empty(n.value, np.int32)
@@ -556,7 +560,7 @@ def plan_roots(g: Graph, k: int, clique: bool = True, opts: Optional[Options] = 
 
 def count_cliques(g: Graph, k: int, opts: Optional[Options] = None) -> tuple[int, Stats]:
     """Number of k-cliques of g (exact uint64), computed on the GPU."""
-    o = (opts or Options()).to_c()
+    o = (opts or _DEFAULT).to_c()
     out = ctypes.c_uint64()
     st = _Stats()
     _check(lib().dm_count_cliques(g.handle, int(k), ctypes.byref(o), ctypes.byref(out), ctypes.byref(st)))
@@ -565,7 +569,7 @@ def count_cliques(g: Graph, k: int, opts: Optional[Options] = None) -> tuple[int
 
 def count_cliques_upto(g: Graph, kmax: int, opts: Optional[Options] = None) -> tuple[dict, Stats]:
     """Clique counts of every size 3..kmax from one traversal: ({k: count}, stats)."""
-    o = (opts or Options()).to_c()
+    o = (opts or _DEFAULT).to_c()
     out = np.zeros(kmax - 2, np.uint64)
     st = _Stats()
     _check(lib().dm_count_cliques_upto(g.handle, int(kmax), ctypes.byref(o), _ptr(out), ctypes.byref(st)))
@@ -575,7 +579,7 @@ def count_cliques_upto(g: Graph, kmax: int, opts: Optional[Options] = None) -> t
 def count_near_cliques(g: Graph, n: int, opts: Optional[Options] = None) -> tuple[int, Stats]:
     """The reference's pattern-aware query q_n (n = 4..13): non-induced copies of K_n minus
     one edge (src/main/q4_PA.cu .. q13_PA.cu)."""
-    o = (opts or Options()).to_c()
+    o = (opts or _DEFAULT).to_c()
     out = ctypes.c_uint64()
     st = _Stats()
     _check(lib().dm_count_near_cliques(g.handle, int(n), ctypes.byref(o), ctypes.byref(out), ctypes.byref(st)))
@@ -588,7 +592,7 @@ def count_motifs(g: Graph, k: int, dictionary: Optional[Dictionary] = None,
     d = dictionary or Dictionary.generate(k)
     if d.k != k:
         raise ValueError(f"dictionary is for k={d.k}, asked for k={k}")
-    o = (opts or Options()).to_c()
+    o = (opts or _DEFAULT).to_c()
     out = np.zeros(d.n_classes, np.uint64)
     st = _Stats()
     _check(lib().dm_count_motifs(g.handle, int(k), d.handle, ctypes.byref(o), _ptr(out), ctypes.byref(st)))
@@ -635,7 +639,7 @@ class Batch:
             arr[i] = _Query(kind=q.kind, k=q.k, graph=q.graph.handle,
                             dict=q.dictionary.handle if q.dictionary is not None else None,
                             vwarp=q.vwarp, threshold=q.threshold, mode=q.mode)
-        o = (opts or Options()).to_c()
+        o = (opts or _DEFAULT).to_c()
         h = _P()
         _check(lib().dm_batch_create(arr, len(self._queries), ctypes.byref(o), int(autotune), ctypes.byref(h)))
         self._h = h

@@ -46,6 +46,9 @@ static CachedArgs cached_args(const CliqueLaunch& L, LaunchCtx& ctx) {
   a.desc = L.desc;
   a.blocks = reinterpret_cast<const uint4*>(L.blocks);
   a.boff = L.boff;
+  a.out = L.out;
+  a.c.lb.cursor0 = L.n_static;
+  a.c.lb.pending0 = L.n_roots;
   a.static_chunk = L.static_chunk;
   a.n_static = L.n_static;
   return a;

@@ -29,7 +29,7 @@ const char* cuda_err_str(cudaError_t e) { return cudaGetErrorString(e); }
 
 // Per-(graph, device) workspace, reused across calls.
 struct Workspace {
-  DevCounters* d_ctr = nullptr;
+  DevCounters* d_ctr = nullptr;     // [0] initialised by every call, [1] self-clearing (index kernel)
   int32_t* d_tasks = nullptr;
   size_t tasks_cap = 0;
   void* d_scratch = nullptr;
@@ -235,7 +235,7 @@ static std::map<int, cudaStream_t> g_report_streams;
 
 class Reporter {
  public:
-  int start(const dm_opts* o, int dev, const DevCounters* ctr, int warps, int64_t roots) {
+  int start(const dm_opts* o, int dev, const DevCounters* ctr, int warps, int64_t roots, int cursor0 = 0, int pending0 = 0) {
     if (!o || !o->report || o->report_ms <= 0) return DM_OK;
     {
       std::lock_guard<std::mutex> lk(g_dev_mu);
@@ -254,6 +254,8 @@ class Reporter {
     ctr_ = ctr;
     warps_ = warps;
     roots_ = roots;
+    cursor0_ = cursor0;
+    pending0_ = pending0;
     t0_ = std::chrono::steady_clock::now();
     th_ = std::thread([this] { run(); });
     return DM_OK;
@@ -283,9 +285,9 @@ class Reporter {
       r.elapsed_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0_).count();
       r.warps = warps_;
       r.hungry_warps = std::max(0, std::min(warps_, snap_->hungry));
-      r.roots_claimed = std::min<int64_t>(roots_, snap_->cursor);
+      r.roots_claimed = std::min<int64_t>(roots_, (int64_t)snap_->cursor + cursor0_);
       r.roots_total = roots_;
-      r.pending = snap_->pending;
+      r.pending = (int64_t)snap_->pending + pending0_;
       r.donations = snap_->donations;
       r.progress = snap_->progress;
       fn_(&r, user_);
@@ -300,6 +302,7 @@ class Reporter {
   void* user_ = nullptr;
   int ms_ = 0, dev_ = 0, warps_ = 0;
   int64_t roots_ = 0;
+  int cursor0_ = 0, pending0_ = 0;  // where a self-clearing launch counts from
   std::chrono::steady_clock::time_point t0_;
 };
 
@@ -487,7 +490,10 @@ static int ensure_ws_bytes(void** p, size_t* cap, size_t want) {
 }
 
 static int prepare_ws(Workspace& ws, cudaStream_t st) {
-  if (!ws.d_ctr) DM_CUDA(cudaMalloc(&ws.d_ctr, sizeof(DevCounters)));
+  if (!ws.d_ctr) {
+    DM_CUDA(cudaMalloc(&ws.d_ctr, 2 * sizeof(DevCounters)));
+    DM_CUDA(cudaMemsetAsync(ws.d_ctr, 0, 2 * sizeof(DevCounters), st));
+  }
   if (!ws.h_init) DM_CUDA(cudaMallocHost(&ws.h_init, sizeof(DevCounters)));
   if (!ws.h_out) DM_CUDA(cudaMallocHost(&ws.h_out, sizeof(DevCounters)));
   if (!ws.ev0) {
@@ -506,23 +512,22 @@ static int prepare_ws(Workspace& ws, cudaStream_t st) {
   return DM_OK;
 }
 
-// Initial counters: every root task is pending until a warp finishes it; the root cursor
-// starts after the entries dealt statically.
+// Initial counters: every root task is pending until a warp finishes it.
 // (pinned source: the copy is asynchronous; the previous call's copies have completed, since
 // every call ends by synchronising its stream)
-static int init_counters(Workspace& ws, int n_roots, cudaStream_t st, int cursor = 0) {
+static int init_counters(Workspace& ws, int n_roots, cudaStream_t st) {
   DevCounters* h = ws.h_init;
   std::memset(h, 0, sizeof(DevCounters));
   h->pending = n_roots;
-  h->cursor = cursor;
   DM_CUDA(cudaMemcpyAsync(ws.d_ctr, h, sizeof(DevCounters), cudaMemcpyHostToDevice, st));
   return DM_OK;
 }
 
 // A call that ended in an error may leave tasks in the queue: start the next one clean.
 static int reset_queue(Workspace& ws, const DevCounters& h, cudaStream_t st) {
-  if (h.err) return init_queue(ws, st);
-  return DM_OK;
+  if (!h.err) return DM_OK;
+  DM_CUDA(cudaMemsetAsync(ws.d_ctr, 0, 2 * sizeof(DevCounters), st));
+  return init_queue(ws, st);
 }
 
 void release_device_graphs(dm_graph* g) {
@@ -935,7 +940,10 @@ static int count_cliques_impl(dm_graph* g, int32_t k, const dm_opts* o, uint64_t
   DeviceSlot* s = slot_for(g, ctx.device);
   Workspace& ws = s->ws;
   if ((rc = prepare_ws(ws, ctx.stream))) return rc;
-  DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
+  // (a plain call on a resident graph prepares nothing: no event, prep_ms 0)
+  const bool prepares = !s->dg.has_oriented || s->index_state == 0 ||
+                        (o && (o->scheduler != DM_SCHED_PLAIN || o->world_size > 1 || o->mode != DM_MODE_AUTO));
+  if (prepares) DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
   if (!s->dg.has_oriented && (rc = upload_clique_image(g, s, ctx.stream))) return rc;
   // tasks: roots (rank space) with at least k-1 out-neighbours
   const int need = upto ? 2 : k - 1;  // a fused count starts from every root with a local edge
@@ -1052,8 +1060,12 @@ static int count_cliques_impl(dm_graph* g, int32_t k, const dm_opts* o, uint64_t
   L.qcap = ws.qcap;
   L.nq = QUEUE_SHARDS;
   L.max_donations = ctx.donations_per_warp;
-  int grid = 0, cursor = 0;
+  int grid = 0;
+  DevCounters* ctr = ws.d_ctr;
   if (use_index) {
+    ctr = ws.d_ctr + 1;
+    L.ctr = ctr;
+    L.out = ws.h_out;
     // a root's block is staged in one round trip, so tasks are short: a task may donate
     // after 2 us instead of 20
     ctx.donate_after_us = std::min(ctx.donate_after_us, 2);
@@ -1069,10 +1081,12 @@ static int count_cliques_impl(dm_graph* g, int32_t k, const dm_opts* o, uint64_t
       const int warps = grid * 8;
       L.static_chunk = std::max(1, std::min(16, (n_roots + warps - 1) / std::max(warps, 1)));
       L.n_static = (int)std::min<int64_t>(n_roots, (int64_t)warps * L.static_chunk);
-      cursor = L.n_static;
+    } else {
+      std::memset(ws.h_out, 0, sizeof(DevCounters));  // no launch
     }
+  } else if ((rc = init_counters(ws, n_roots, ctx.stream))) {
+    return rc;
   }
-  if ((rc = init_counters(ws, n_roots, ctx.stream, cursor))) return rc;
   L2Window l2;
   if (o && (o->flags & DM_FLAG_L2_PERSIST)) {
     if (use_index) rc = l2.begin(ctx.device, ctx.stream, s->d_blocks, s->index_bytes);
@@ -1084,10 +1098,13 @@ static int count_cliques_impl(dm_graph* g, int32_t k, const dm_opts* o, uint64_t
   if (n_roots > 0) {
     rc = use_index ? clique_cached_launch(L, ctx, grid) : clique_launch(L, ctx, &grid);
     if (rc) return rc;
-    if ((rc = reporter.start(o, ctx.device, ws.d_ctr, grid * 8, n_roots))) return rc;
+    if ((rc = reporter.start(o, ctx.device, ctr, grid * 8, n_roots, use_index ? L.n_static : 0,
+                             use_index ? n_roots : 0)))
+      return rc;
   }
   DM_CUDA(cudaEventRecord(ws.k1, ctx.stream));
-  DM_CUDA(cudaMemcpyAsync(ws.h_out, ws.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, ctx.stream));
+  if (!use_index)
+    DM_CUDA(cudaMemcpyAsync(ws.h_out, ws.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, ctx.stream));
   std::vector<unsigned long long> per_rank;
   if (want_log) {
     per_rank.resize(g->n);
@@ -1100,7 +1117,7 @@ static int count_cliques_impl(dm_graph* g, int32_t k, const dm_opts* o, uint64_t
   if ((rc = reset_queue(ws, h, ctx.stream))) return rc;
   float kms = 0, pms = 0;
   cudaEventElapsedTime(&kms, ws.k0, ws.k1);
-  cudaEventElapsedTime(&pms, ws.ev0, ws.k0);
+  if (prepares) cudaEventElapsedTime(&pms, ws.ev0, ws.k0);
   if (h.err)
     return fail(kernel_status(h.err),
                 "clique kernel reported error " + std::to_string(h.err));

@@ -36,7 +36,7 @@ struct alignas(128) DevCounters {
   int max_task_root;             // its root (best effort under races)
   int test_gate;                 // never written by the library (failure-path tests)
   int err;                       // first error code raised by a kernel (0 = none)
-  int err_info;
+  int blocks_done;               // self-clearing launches: blocks that have added their sums
 };
 
 constexpr int ERR_ARENA_OVERFLOW = 1;
@@ -142,6 +142,7 @@ struct CliqueLaunch {
   const RootDesc* desc = nullptr;   // task list (n_roots entries)
   const void* blocks = nullptr;     // the index (16-byte units)
   const uint32_t* boff = nullptr;   // block offset per root
+  DevCounters* out = nullptr;       // page-locked host copy of the counters, written by the kernel
   int static_chunk = 1;             // warp w starts with entries [w * static_chunk, +static_chunk)
   int n_static = 0;                 // entries dealt statically; the root cursor starts here
   bool tma = true;                  // stage blocks by bulk asynchronous copies (else 16-byte loads)

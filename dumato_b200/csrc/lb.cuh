@@ -67,6 +67,9 @@ struct LBArgs {
   int test_stall;             // test hook: wait at exit on a word nothing sets
   int min_split;              // a task keeps ranges shorter than this
   int nq;                     // shards
+  // a kernel on self-clearing counters (zero at launch) counts from these instead
+  int cursor0 = 0;            // the root cursor's start
+  int pending0 = 0;           // tasks pending at the start
 };
 
 __device__ __forceinline__ long long global_ns() {
@@ -191,12 +194,12 @@ static __device__ __noinline__ bool lb_next(const LBArgs& lb, int n_roots, int t
                                             int& b, int& e, bool& donated, int& level, int* path,
                                             int* unflushed = nullptr, unsigned long long* idle = nullptr) {
   DevCounters* c = lb.ctr;
-  int cur = vload(&c->cursor);
+  int cur = vload(&c->cursor) + lb.cursor0;
   if (cur < n_roots) {
     // light tail roots are claimed several at a time to keep the cursor line cool
     int chunk = (n_roots - cur) / (8 * total_warps);
     chunk = chunk < 1 ? 1 : (chunk > 16 ? 16 : chunk);
-    const int r = atomicAdd(&c->cursor, chunk);
+    const int r = atomicAdd(&c->cursor, chunk) + lb.cursor0;
     if (r < n_roots) {
       first = r;
       count = min(chunk, n_roots - r);
@@ -216,7 +219,7 @@ static __device__ __noinline__ bool lb_next(const LBArgs& lb, int n_roots, int t
   const long long t_hungry = global_ns();
   long long t0 = t_hungry;
   unsigned long long last = vload64(&c->progress);
-  int last_pending = vload(&c->pending);
+  int last_pending = vload(&c->pending) + lb.pending0;
   unsigned backoff = 128;
   unsigned long long polls = 0;
   bool got = false;
@@ -230,7 +233,7 @@ static __device__ __noinline__ bool lb_next(const LBArgs& lb, int n_roots, int t
       got = true;
       break;
     }
-    const int pend = vload(&c->pending);
+    const int pend = vload(&c->pending) + lb.pending0;
     if (pend <= 0 && lb.test_stall) {
       lb_stall(lb);
       break;
