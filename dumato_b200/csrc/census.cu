@@ -28,7 +28,7 @@
 // taken by one warp each with a hash table of its own (SMALL_PATHS); the others by a block each
 // with direct 16-bit counters over the ranks below u, cleared in a few 16-byte stores per thread.
 // Measured per call, enumeration before: k = 3 on an R-MAT graph of 98,552 vertices and 1.08M edges
-// 2,981 -> 53 us; k = 4 on a Chung-Lu graph of 18,700 vertices and 198,000 edges 12,994 -> 467 us.
+// 2,981 -> 29 us; k = 4 on a Chung-Lu graph of 18,700 vertices and 198,000 edges 12,994 -> 169 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,8 +40,9 @@
 
 namespace dmb {
 
-// sums[]: rows kernel, then the two-path kernels
-enum { CENSUS_WEDGE, CENSUS_STAR, CENSUS_TRI, CENSUS_EDGE, CENSUS_PAW, CENSUS_K4, CENSUS_C4, CENSUS_DIA, CENSUS_PAW_TOP };
+// sums[]: k = 4: rows kernel, then the two-path kernels; k = 3: triangles, wedges
+enum { CENSUS_STAR, CENSUS_TRI, CENSUS_EDGE, CENSUS_PAW, CENSUS_K4, CENSUS_C4, CENSUS_DIA, CENSUS_PAW_TOP };
+enum { FLAT_TRI, FLAT_WEDGE, FLAT_SUMS };
 static_assert(CENSUS_PAW_TOP + 1 == CENSUS_SUMS, "engine.hpp sizes the buffer");
 
 // A vertex's in-list entry: v -> u, and the place of u in v's padded out-row (the edge's id).
@@ -58,7 +59,8 @@ struct CensusArgs {
   uint32_t* up;              // by edge id: triangles on the edge whose third vertex is above both
   unsigned long long* sums;  // CENSUS_SUMS
   int* list;                 // vertices left to the block kernel
-  int* ctl;                  // [0] length of list, [1] warp cursor, [2] block cursor
+  int* ctl;                  // [0] length of list, [1] warp cursor, [2] block cursor, [3] blocks done
+  unsigned long long* out;   // page-locked host memory: the sums at the end of the launches
   const int32_t* order;      // ranks by descending out-degree
   int n_wide;                // of them, those with 32 or more out-neighbours
   int base;                  // first rank with degree >= 2 (lower ranks lie on no cycle)
@@ -145,21 +147,17 @@ __device__ __forceinline__ unsigned long long choose3(unsigned long long d) {
   return a * b * c;
 }
 
-// One root's share of the sums by G lanes (l of G): wedges and stars from the degree; for every
-// edge the popcount t of its index row (the triangles on it whose third vertex is above both);
-// FOUR: also the 4-cliques above it, the paths' edge sum, the paws at the two lower vertices of
-// those triangles, and t itself in `up`.
-template <bool FOUR, int G>
-__device__ __forceinline__ void census_root(const CensusArgs& a, int r, int l, unsigned long long (&s)[6]) {
+// One root's share of the k = 4 sums by G lanes (l of G): stars from the degree; for every edge the popcount t of its index row (the triangles on it whose third vertex is above both);
+// the 4-cliques above it, the paths' edge sum, the paws at the two lower vertices of those
+// triangles, and t itself in `up`.
+template <int G>
+__device__ __forceinline__ void census_root(const CensusArgs& a, int r, int l, unsigned long long (&s)[5]) {
   const int d = __ldg(a.g.deg + r);
   const unsigned long long du = (unsigned long long)__ldg(a.ud + r);
-  if (l == 0) {
-    s[CENSUS_WEDGE] += choose2(du);
-    if (FOUR) s[CENSUS_STAR] += choose3(du);
-  }
+  if (l == 0) s[CENSUS_STAR] += choose3(du);
   const int nw = (d + 63) >> 6;
   const uint64_t* rows = d >= 2 ? reinterpret_cast<const uint64_t*>(a.blocks + __ldg(a.boff + r)) : nullptr;
-  const int b = FOUR ? __ldg(a.g.row + r) : 0;
+  const int b = __ldg(a.g.row + r);
   for (int i = l; i < d; i += G) {
     unsigned t = 0, q = 0;
     if (rows) {
@@ -167,36 +165,75 @@ __device__ __forceinline__ void census_root(const CensusArgs& a, int r, int l, u
       for (int w = 0; w < nw; ++w) {
         uint64_t m = __ldg(ri + w);
         t += __popcll(m);
-        if (FOUR) {
-          // (members are numbered in rank order, so row j holds no bit at or below j)
-          while (m) {
-            const uint64_t* rj = rows + (size_t)(w * 64 + __ffsll((long long)m) - 1) * nw;
-            m &= m - 1;
-            for (int x = w; x < nw; ++x) q += __popcll(__ldg(ri + x) & __ldg(rj + x));
-          }
+        // (members are numbered in rank order, so row j holds no bit at or below j)
+        while (m) {
+          const uint64_t* rj = rows + (size_t)(w * 64 + __ffsll((long long)m) - 1) * nw;
+          m &= m - 1;
+          for (int x = w; x < nw; ++x) q += __popcll(__ldg(ri + x) & __ldg(rj + x));
         }
       }
     }
+    const unsigned long long dv = (unsigned long long)__ldg(a.ud + __ldg(a.g.adj + b + i));
+    a.up[b + i] = t;
     s[CENSUS_TRI] += t;
-    if (FOUR) {
-      const unsigned long long dv = (unsigned long long)__ldg(a.ud + __ldg(a.g.adj + b + i));
-      a.up[b + i] = t;
-      s[CENSUS_EDGE] += (du - 1) * (dv - 1);
-      s[CENSUS_PAW] += (unsigned long long)t * (du + dv - 4);
-      s[CENSUS_K4] += q;
-    }
+    s[CENSUS_EDGE] += (du - 1) * (dv - 1);
+    s[CENSUS_PAW] += (unsigned long long)t * (du + dv - 4);
+    s[CENSUS_K4] += q;
   }
 }
 
 // All ranks in descending out-degree order: a warp per root for the wide ones (at least 32 rows),
 // eight lanes per root for the others.
-template <bool FOUR>
 __global__ void __launch_bounds__(256) census_rows_kernel(const __grid_constant__ CensusArgs a) {
-  unsigned long long s[6] = {0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
+  unsigned long long s[5] = {0ull, 0ull, 0ull, 0ull, 0ull};
   const int t = blockIdx.x * 256 + threadIdx.x, T = gridDim.x * 256;
-  for (int i = t >> 5; i < a.n_wide; i += T >> 5) census_root<FOUR, 32>(a, __ldg(a.order + i), t & 31, s);
-  for (int i = a.n_wide + (t >> 3); i < a.g.n; i += T >> 3) census_root<FOUR, 8>(a, __ldg(a.order + i), t & 7, s);
+  for (int i = t >> 5; i < a.n_wide; i += T >> 5) census_root<32>(a, __ldg(a.order + i), t & 31, s);
+  for (int i = a.n_wide + (t >> 3); i < a.g.n; i += T >> 3) census_root<8>(a, __ldg(a.order + i), t & 7, s);
   add_sums(s, a.sums);
+}
+
+// End of a call's last kernel: its last block hands the n sums to the host and zeroes them and the
+// cursors for the next call, which then needs no copy before or after its launches.
+__device__ __forceinline__ void census_finish(unsigned long long* sums, int* ctl, int n, unsigned long long* out) {
+  __shared__ int last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ctl + 3, 1) == (int)gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if ((int)threadIdx.x < n) {
+    volatile unsigned long long* v = sums + threadIdx.x;
+    out[threadIdx.x] = *v;
+    *v = 0ull;
+  }
+  if (threadIdx.x < 4) ctl[threadIdx.x] = 0;
+}
+
+// k = 3: triangles as the popcount of the whole index (every row bit is one triangle; the blocks
+// lie end to end and their padding is zero), and with ud the wedges from the degrees. A stream of
+// 16-byte loads, four in flight per thread, where staging the blocks root by root pays for the
+// task list, the cursor and the wait for the last warp: triangles of a graph of 2,000 vertices took
+// 35.5 us per call, now 23.7; the census of 98,552 vertices (a 20 MB index) 53 us, now 29 (9 us of
+// them this kernel, 2.2 TB/s out of L2).
+__global__ void __launch_bounds__(256) census_flat_kernel(const uint4* __restrict__ blocks, uint64_t units,
+                                                          const int32_t* __restrict__ ud, int n,
+                                                          unsigned long long* sums, int* ctl, unsigned long long* out) {
+  unsigned long long s[FLAT_SUMS] = {0ull, 0ull};
+  const uint64_t T = gridDim.x * 256ull, t = blockIdx.x * 256ull + threadIdx.x;
+  for (uint64_t i = t; i < units; i += 4 * T) {
+    uint4 v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = i + q * T < units ? __ldg(blocks + i + q * T) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s[FLAT_TRI] += (unsigned)(__popc(v[q].x) + __popc(v[q].y) + __popc(v[q].z) + __popc(v[q].w));
+  }
+  if (ud)
+    for (uint64_t i = t; i < (uint64_t)n; i += T) s[FLAT_WEDGE] += choose2((unsigned long long)__ldg(ud + i));
+  add_sums(s, sums);
+  census_finish(sums, ctl, FLAT_SUMS, out);
 }
 
 // ---------------- two-paths below u ----------------
@@ -264,14 +301,16 @@ __global__ void __launch_bounds__(32 * SMALL_WARPS) census_small_kernel(const __
   int* key = sm + warp_in_block() * 2 * SMALL_SLOTS;
   unsigned* cnt = reinterpret_cast<unsigned*>(key + SMALL_SLOTS);
   unsigned long long s[3] = {0ull, 0ull, 0ull};  // cycles, diamonds, paws at the highest vertex
+  // (runs of 32 on every graph left a graph of 18,700 vertices on 584 warps: 321 us)
+  const int run = max(1, min(32, (a.g.n - a.base) / (4 * (int)gridDim.x * SMALL_WARPS)));
   while (true) {
-    // vertices in descending rank, 32 at a time: the list of large ones starts with the hubs
+    // vertices in descending rank, `run` at a time: the list of large ones starts with the hubs
     int c = 0;
-    if (lane == 0) c = atomicAdd(a.ctl + 1, 32);
+    if (lane == 0) c = atomicAdd(a.ctl + 1, run);
     c = __shfl_sync(FULL_MASK, c, 0);
     if (c >= a.g.n - a.base) break;
     const int mine = a.g.n - 1 - c - lane;
-    const int nd = mine >= a.base ? __ldg(a.in_deg + mine) : 0;
+    const int nd = lane < run && mine >= a.base ? __ldg(a.in_deg + mine) : 0;
     const int e0 = nd ? __ldg(a.in_end + mine) - nd : 0;
     // a vertex with one lower neighbour closes nothing: its edge keeps the triangles above it
     if (nd == 1) s[1] += choose2(a.up[__ldg(&a.in[e0].y)]);
@@ -345,6 +384,7 @@ __global__ void census_large_kernel(const __grid_constant__ CensusArgs a, int sp
   __shared__ unsigned long long s_two;
   const int lane = lane_id();
   const int n_list = *reinterpret_cast<volatile int*>(a.ctl);
+  const int warps = blockDim.x >> 5;
   unsigned long long s[3] = {0ull, 0ull, 0ull};
   while (true) {
     if (threadIdx.x == 0) s_item = atomicAdd(a.ctl + 2, 1);
@@ -362,12 +402,15 @@ __global__ void census_large_kernel(const __grid_constant__ CensusArgs a, int sp
       for (int i = threadIdx.x; i < words; i += blockDim.x) reinterpret_cast<uint4*>(cw)[i] = make_uint4(0u, 0u, 0u, 0u);
       if (threadIdx.x == 0) s_batch = 0;
       __syncthreads();
+      // a warp takes `take` in-neighbours at a time, so that a vertex with few of them still
+      // occupies every warp of the block
+      const int take = max(1, min(32, I / warps));
       while (true) {
         int i0 = 0;
-        if (lane == 0) i0 = atomicAdd(&s_batch, 32);
+        if (lane == 0) i0 = atomicAdd(&s_batch, take);
         i0 = __shfl_sync(FULL_MASK, i0, 0);
         if (i0 >= I) break;
-        const PathBatch p = path_batch(a, L, i0, I);
+        const PathBatch p = path_batch(a, L, i0, min(I, i0 + take));
         for (int f0 = 0; f0 < p.total; f0 += 128) {
           int x[4];
 #pragma unroll
@@ -404,6 +447,7 @@ __global__ void census_large_kernel(const __grid_constant__ CensusArgs a, int sp
     if (threadIdx.x == 0) s[2] += (s_two >> 1) * (unsigned long long)(__ldg(a.ud + u) - 2);
   }
   add_sums(s, a.sums + CENSUS_C4);
+  census_finish(a.sums, a.ctl, CENSUS_SUMS, a.out);
 }
 
 // ---------------- launcher ----------------
@@ -434,6 +478,18 @@ static int launch_large(const CensusArgs& a, LaunchCtx& ctx) {
   return DM_OK;
 }
 
+int census_flat(const void* blocks, uint64_t units, const int32_t* ud, int n, unsigned long long* sums,
+                unsigned long long* out, LaunchCtx& ctx) {
+  // about four 16-byte units or degrees per thread, at most two full waves of threads
+  const int64_t want = std::max<int64_t>(((int64_t)units + 1023) / 1024, ud ? (n + 1023) / 1024 : 1);
+  const int grid = census_grid(std::min<int64_t>(ctx.num_sms * 8, want), 256, ctx);
+  census_flat_kernel<<<grid, 256, 0, ctx.stream>>>(reinterpret_cast<const uint4*>(blocks), units, ud, n, sums,
+                                                   reinterpret_cast<int*>(sums + CENSUS_SUMS), out);
+  ctx.launches++;
+  DM_CUDA(cudaGetLastError());
+  return DM_OK;
+}
+
 int census_launch(const CensusLaunch& L, LaunchCtx& ctx) {
   CensusArgs a;
   a.g = L.g;
@@ -446,19 +502,17 @@ int census_launch(const CensusLaunch& L, LaunchCtx& ctx) {
   a.up = L.up;
   a.sums = L.sums;
   a.ctl = reinterpret_cast<int*>(L.sums + CENSUS_SUMS);
+  a.out = L.out;
   a.list = L.list;
   a.order = L.order;
   a.n_wide = L.n_wide;
   a.base = L.base;
-  DM_CUDA(cudaMemsetAsync(L.sums, 0, CENSUS_BYTES, ctx.stream));
   const int grid = census_grid(std::min<int64_t>(ctx.num_sms * 8, ((int64_t)a.g.n * 8 + 255) / 256), 256, ctx);
-  if (L.k == 3) census_rows_kernel<false><<<grid, 256, 0, ctx.stream>>>(a);
-  else census_rows_kernel<true><<<grid, 256, 0, ctx.stream>>>(a);
+  census_rows_kernel<<<grid, 256, 0, ctx.stream>>>(a);
   ctx.launches++;
   DM_CUDA(cudaGetLastError());
-  if (L.k == 3) return DM_OK;
   DM_CUDA(cudaFuncSetAttribute(census_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_SMEM));
-  const int small = census_grid(std::min(ctx.num_sms * 3, (a.g.n - a.base + 32 * SMALL_WARPS - 1) / (32 * SMALL_WARPS)),
+  const int small = census_grid(std::min(ctx.num_sms * 3, (a.g.n - a.base + SMALL_WARPS - 1) / SMALL_WARPS),
                                 32 * SMALL_WARPS, ctx);
   census_small_kernel<<<small, 32 * SMALL_WARPS, SMALL_SMEM, ctx.stream>>>(a);
   ctx.launches++;
@@ -468,12 +522,12 @@ int census_launch(const CensusLaunch& L, LaunchCtx& ctx) {
 
 // Class counts of the census (indices of census_class).
 void census_classes(int k, const uint64_t* s, uint64_t* c) {
-  const uint64_t T = s[CENSUS_TRI];
   if (k == 3) {
-    c[0] = s[CENSUS_WEDGE] - 3 * T;
-    c[1] = T;
+    c[0] = s[FLAT_WEDGE] - 3 * s[FLAT_TRI];
+    c[1] = s[FLAT_TRI];
     return;
   }
+  const uint64_t T = s[CENSUS_TRI];
   const uint64_t k4 = s[CENSUS_K4];
   const uint64_t dia = s[CENSUS_DIA] - 6 * k4;
   const uint64_t cyc = s[CENSUS_C4] - dia - 3 * k4;

@@ -30,6 +30,7 @@ const char* cuda_err_str(cudaError_t e) { return cudaGetErrorString(e); }
 // Per-(graph, device) workspace, reused across calls.
 struct Workspace {
   DevCounters* d_ctr = nullptr;     // [0] initialised by every call, [1] self-clearing (index kernel)
+  unsigned long long* d_sums = nullptr;  // census sums (CENSUS_BYTES behind d_ctr), self-clearing
   int32_t* d_tasks = nullptr;
   size_t tasks_cap = 0;
   void* d_scratch = nullptr;
@@ -45,9 +46,8 @@ struct Workspace {
   size_t per_root_cap = 0;
   int32_t* d_parts = nullptr;       // scheduler part words, parallel to the task list
   size_t parts_cap = 0;
-  unsigned char* d_census = nullptr;  // census: sums, vertex list, edge array
+  unsigned char* d_census = nullptr;  // census: vertex list, edge array
   size_t census_cap = 0;
-  unsigned long long* h_census = nullptr;  // pinned: the sums read back
   uint32_t* d_bits = nullptr;       // motif membership bitmaps, all zero between calls
   size_t bits_cap = 0;
   RootDesc* d_desc = nullptr;       // task list of a call on the clique index
@@ -68,7 +68,9 @@ struct Workspace {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, k0 = nullptr, k1 = nullptr;
   DevCounters* h_init = nullptr;    // pinned: a call's initial counters (asynchronous upload)
   DevCounters* h_out = nullptr;     // pinned: the counters read back after the kernel
+  unsigned long long* h_sums = nullptr;  // pinned (behind h_out): the census sums of a call
 };
+constexpr size_t CTR_BYTES = 2 * sizeof(DevCounters) + CENSUS_BYTES;
 
 
 // Empty state: every shard's positions at 0, slot j of a shard carrying sequence j.
@@ -337,7 +339,6 @@ static void free_workspace(Workspace& w) {
   if (w.h_init) cudaFreeHost(w.h_init);
   if (w.h_hdr) cudaFreeHost(w.h_hdr);
   if (w.h_out) cudaFreeHost(w.h_out);
-  if (w.h_census) cudaFreeHost(w.h_census);
   w = Workspace();
 }
 
@@ -491,11 +492,15 @@ static int ensure_ws_bytes(void** p, size_t* cap, size_t want) {
 
 static int prepare_ws(Workspace& ws, cudaStream_t st) {
   if (!ws.d_ctr) {
-    DM_CUDA(cudaMalloc(&ws.d_ctr, 2 * sizeof(DevCounters)));
-    DM_CUDA(cudaMemsetAsync(ws.d_ctr, 0, 2 * sizeof(DevCounters), st));
+    DM_CUDA(cudaMalloc(&ws.d_ctr, CTR_BYTES));
+    DM_CUDA(cudaMemsetAsync(ws.d_ctr, 0, CTR_BYTES, st));
+    ws.d_sums = reinterpret_cast<unsigned long long*>(ws.d_ctr + 2);
   }
   if (!ws.h_init) DM_CUDA(cudaMallocHost(&ws.h_init, sizeof(DevCounters)));
-  if (!ws.h_out) DM_CUDA(cudaMallocHost(&ws.h_out, sizeof(DevCounters)));
+  if (!ws.h_out) {
+    DM_CUDA(cudaMallocHost(&ws.h_out, sizeof(DevCounters) + CENSUS_BYTES));
+    ws.h_sums = reinterpret_cast<unsigned long long*>(ws.h_out + 1);
+  }
   if (!ws.ev0) {
     DM_CUDA(cudaEventCreate(&ws.ev0));
     DM_CUDA(cudaEventCreate(&ws.ev1));
@@ -526,7 +531,7 @@ static int init_counters(Workspace& ws, int n_roots, cudaStream_t st) {
 // A call that ended in an error may leave tasks in the queue: start the next one clean.
 static int reset_queue(Workspace& ws, const DevCounters& h, cudaStream_t st) {
   if (!h.err) return DM_OK;
-  DM_CUDA(cudaMemsetAsync(ws.d_ctr, 0, 2 * sizeof(DevCounters), st));
+  DM_CUDA(cudaMemsetAsync(ws.d_ctr, 0, CTR_BYTES, st));
   return init_queue(ws, st);
 }
 
@@ -1014,6 +1019,10 @@ static int count_cliques_impl(dm_graph* g, int32_t k, const dm_opts* o, uint64_t
   // the plain task list on the index holds the parts of the split roots too (they lead it)
   if (use_index && d_desc == s->d_desc_deg && n_roots > 0) n_roots += g->idx_extra;
   if (upto && (!use_index || max_d > INDEX_MAX_DEGREE || (o && o->subtree_counts))) return 1;
+  // triangles of the whole graph: the popcount of the index (an explicit staging, a report or a test
+  // hook asks for the task kernel)
+  const bool flat = k == 3 && !upto && use_index && d_desc == s->d_desc_deg && max_d <= INDEX_MAX_DEGREE &&
+                    !(o && (o->subtree_counts || o->staging != DM_STAGE_AUTO || o->report || o->test_flags));
   CliqueLaunch L;
   L.k = k;
   if (mode == DM_MODE_LIST) {
@@ -1074,7 +1083,9 @@ static int count_cliques_impl(dm_graph* g, int32_t k, const dm_opts* o, uint64_t
     L.blocks = s->d_blocks;
     L.boff = s->d_boff;
     L.tma = !(o && o->staging == DM_STAGE_LOADS);
-    if (n_roots > 0) {
+    if (flat) {
+      std::memset(ws.h_out, 0, sizeof(DevCounters));  // (the sums come back behind it)
+    } else if (n_roots > 0) {
       if ((rc = clique_cached_grid(L, ctx, &grid))) return rc;
       // every warp starts on static entries of the list (w, w + T, ...): no cursor atomics
       // while the first CHUNK_MAX x T entries are counted
@@ -1095,7 +1106,9 @@ static int count_cliques_impl(dm_graph* g, int32_t k, const dm_opts* o, uint64_t
   }
   DM_CUDA(cudaEventRecord(ws.k0, ctx.stream));
   Reporter reporter;
-  if (n_roots > 0) {
+  if (flat) {
+    if ((rc = census_flat(s->d_blocks, g->idx_units, nullptr, 0, ws.d_sums, ws.h_sums, ctx))) return rc;
+  } else if (n_roots > 0) {
     rc = use_index ? clique_cached_launch(L, ctx, grid) : clique_launch(L, ctx, &grid);
     if (rc) return rc;
     if ((rc = reporter.start(o, ctx.device, ctr, grid * 8, n_roots, use_index ? L.n_static : 0,
@@ -1113,7 +1126,11 @@ static int count_cliques_impl(dm_graph* g, int32_t k, const dm_opts* o, uint64_t
                               ctx.stream));
   }
   DM_CUDA(cudaStreamSynchronize(ctx.stream));
-  const DevCounters h = *ws.h_out;
+  DevCounters h = *ws.h_out;
+  if (flat) {
+    h.count = ws.h_sums[0];
+    h.tasks = (unsigned long long)n_roots;
+  }
   if ((rc = reset_queue(ws, h, ctx.stream))) return rc;
   float kms = 0, pms = 0;
   cudaEventElapsedTime(&kms, ws.k0, ws.k1);
@@ -1359,49 +1376,56 @@ static int motif_census(dm_graph* g, int k, const dm_dictionary* dict, const int
   Workspace& ws = s->ws;
   int rc;
   if ((rc = prepare_ws(ws, ctx.stream))) return rc;
-  DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
+  const bool prepares = !s->dg.has_oriented || s->index_state == 0 || !s->d_udeg || (k == 4 && !s->d_in);
+  if (prepares) DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
   if (!s->dg.has_oriented && (rc = upload_clique_image(g, s, ctx.stream))) return rc;
   if ((rc = ensure_index(g, s, ctx))) return rc;
   if (s->index_state != 1) return 1;
   if ((rc = ensure_census(g, s, k, ctx))) return rc;
-  const size_t list_off = (CENSUS_BYTES + 255) / 256 * 256;
-  const size_t up_off = list_off + (k == 4 ? (sizeof(int) * (size_t)g->n + 255) / 256 * 256 : 0);
-  const size_t bytes = up_off + (k == 4 ? sizeof(uint32_t) * g->img_adj_ints : 0);
-  if ((rc = ensure_ws_bytes(reinterpret_cast<void**>(&ws.d_census), &ws.census_cap, bytes))) return rc;
-  if (!ws.h_census) DM_CUDA(cudaMallocHost(&ws.h_census, CENSUS_BYTES));
   CensusLaunch L;
-  L.g = GraphView{s->dg.d_orow, s->dg.d_odeg, s->dg.d_oadj, g->n};
-  L.k = k;
-  L.blocks = s->d_blocks;
-  L.boff = s->d_boff;
-  L.ud = s->d_udeg;
-  L.order = s->d_deg_order;
-  L.n_wide = 32 < (int)g->cnt_ge.size() ? (int)g->cnt_ge[32] : 0;
-  L.base = g->n_deg01;
-  L.wide_counters = g->max_degree >= 65536;
-  L.in_end = s->d_in_end;
-  L.in_deg = s->d_in_deg;
-  L.in = s->d_in;
-  L.sums = reinterpret_cast<unsigned long long*>(ws.d_census);
-  L.list = reinterpret_cast<int*>(ws.d_census + list_off);
-  L.up = reinterpret_cast<uint32_t*>(ws.d_census + up_off);
+  if (k == 4) {
+    const size_t up_off = (sizeof(int) * (size_t)g->n + 255) / 256 * 256;
+    if ((rc = ensure_ws_bytes(reinterpret_cast<void**>(&ws.d_census), &ws.census_cap,
+                              up_off + sizeof(uint32_t) * g->img_adj_ints)))
+      return rc;
+    L.g = GraphView{s->dg.d_orow, s->dg.d_odeg, s->dg.d_oadj, g->n};
+    L.blocks = s->d_blocks;
+    L.boff = s->d_boff;
+    L.ud = s->d_udeg;
+    L.order = s->d_deg_order;
+    L.n_wide = 32 < (int)g->cnt_ge.size() ? (int)g->cnt_ge[32] : 0;
+    L.base = g->n_deg01;
+    L.wide_counters = g->max_degree >= 65536;
+    L.in_end = s->d_in_end;
+    L.in_deg = s->d_in_deg;
+    L.in = s->d_in;
+    L.sums = ws.d_sums;
+    L.out = ws.h_sums;
+    L.list = reinterpret_cast<int*>(ws.d_census);
+    L.up = reinterpret_cast<uint32_t*>(ws.d_census + up_off);
+  }
   L2Window l2;
   if (o && (o->flags & DM_FLAG_L2_PERSIST) && (rc = l2.begin(ctx.device, ctx.stream, s->d_blocks, s->index_bytes)))
     return rc;
   DM_CUDA(cudaEventRecord(ws.k0, ctx.stream));
-  if ((rc = census_launch(L, ctx))) return rc;
+  rc = k == 3 ? census_flat(s->d_blocks, g->idx_units, s->d_udeg, g->n, ws.d_sums, ws.h_sums, ctx)
+              : census_launch(L, ctx);
+  if (rc) {
+    // a launch may have been refused after an earlier one ran: leave the sums zero
+    cudaMemsetAsync(ws.d_sums, 0, CENSUS_BYTES, ctx.stream);
+    return rc;
+  }
   DM_CUDA(cudaEventRecord(ws.k1, ctx.stream));
-  DM_CUDA(cudaMemcpyAsync(ws.h_census, ws.d_census, CENSUS_BYTES, cudaMemcpyDeviceToHost, ctx.stream));
   DM_CUDA(cudaStreamSynchronize(ctx.stream));
   uint64_t sums[CENSUS_SUMS], types[6];
-  for (int i = 0; i < CENSUS_SUMS; ++i) sums[i] = ws.h_census[i];
+  for (int i = 0; i < CENSUS_SUMS; ++i) sums[i] = ws.h_sums[i];
   census_classes(k, sums, types);
   std::memset(class_counts, 0, sizeof(uint64_t) * dict->n_classes);
   for (int t = 0; t < (k == 3 ? 2 : 6); ++t) class_counts[cls[t]] += types[t];
   if (st) {
     float kms = 0, pms = 0;
     cudaEventElapsedTime(&kms, ws.k0, ws.k1);
-    cudaEventElapsedTime(&pms, ws.ev0, ws.k0);
+    if (prepares) cudaEventElapsedTime(&pms, ws.ev0, ws.k0);
     std::memset(st, 0, sizeof(*st));
     st->kernel_ms = kms;
     st->prep_ms = pms;

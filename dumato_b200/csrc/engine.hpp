@@ -182,11 +182,15 @@ int near_clique_launch(const NearLaunch& L, LaunchCtx& ctx, int* grid);
 size_t near_clique_rows(int d, int deg);  // arena ints (beyond the list) for a root's edges
 
 // Whole-graph census of the connected 3- and 4-vertex classes (census.cu).
-constexpr int CENSUS_SUMS = 9;
-constexpr size_t CENSUS_BYTES = (CENSUS_SUMS + 2) * sizeof(unsigned long long);  // sums and cursors
-struct CensusLaunch {
+constexpr int CENSUS_SUMS = 8;
+// sums and cursors of a call: zero at launch, and zeroed again by the call's last block
+constexpr size_t CENSUS_BYTES = (CENSUS_SUMS + 2) * sizeof(unsigned long long);
+// k = 3, and triangles alone (ud null): sums 0 (triangles) and 1 (wedges) into out, page-locked
+// host memory, from the clique index of `units` 16-byte units and the degrees.
+int census_flat(const void* blocks, uint64_t units, const int32_t* ud, int n, unsigned long long* sums,
+                unsigned long long* out, LaunchCtx& ctx);
+struct CensusLaunch {              // k = 4
   GraphView g;                     // degree-ordered DAG in rank space
-  int k = 3;
   const void* blocks = nullptr;    // clique index: a block for every root with 2 or more out-neighbours
   const uint32_t* boff = nullptr;
   const int32_t* ud = nullptr;     // undirected degree by rank
@@ -194,13 +198,14 @@ struct CensusLaunch {
   int n_wide = 0;
   int base = 0;                    // ranks below it have degree 0 or 1
   bool wide_counters = false;      // a degree of 65,536 or more: 32-bit path counters
-  // k = 4: in-lists (census_in_lists), edge array (one word per padded DAG entry) and vertex list
+  // in-lists (census_in_lists), edge array (one word per padded DAG entry) and vertex list
   const int32_t* in_end = nullptr;
   const int32_t* in_deg = nullptr;
   const void* in = nullptr;
   uint32_t* up = nullptr;
   int* list = nullptr;
-  unsigned long long* sums = nullptr;  // CENSUS_BYTES, zeroed by the launch
+  unsigned long long* sums = nullptr;  // CENSUS_BYTES
+  unsigned long long* out = nullptr;   // page-locked host memory: CENSUS_SUMS
 };
 int census_launch(const CensusLaunch& L, LaunchCtx& ctx);
 // In-lists of the DAG: n end offsets, n lengths, 8 bytes per edge, and one scratch int.
