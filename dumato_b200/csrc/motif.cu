@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(32 * MOTIF_WARPS, 4) motif_kernel(const __grid
       if (!donated && a.parts) part_bounds(__ldg(a.parts + first + ti), bb, ee);
       ++ntasks;
       // block-level class counters, added to the global ones at exit
-      motif_run_task<K, W>(c, bhist, ws, warp_arena, warp_bits, v0, bb, ee, level, path, nodes);
+      motif_run_task<K, W>(c, ClassHist{reinterpret_cast<unsigned*>(bhist), nullptr}, ws, warp_arena, warp_bits, v0, bb, ee, level, path, nodes);
     }
     if (lane == 0) lb_done(c.lb, count);
   }

@@ -75,6 +75,26 @@ struct alignas(16) MotifSweep {
   unsigned mh[8];              // k = 3: leaf-mask histogram
 };
 
+// 64-bit class counters: in shared memory (w, as pairs of 32-bit words, low word first: a 64-bit
+// add to shared memory is a compare-and-swap loop, and many lanes add to the same few classes;
+// two 32-bit adds with the carry taken from the first one's old value are native), else in
+// global memory (g).
+struct ClassHist {
+  unsigned* w;
+  unsigned long long* g;
+  __device__ __forceinline__ void add(int c, unsigned long long v) const {
+    if (w) {
+      const unsigned lo = (unsigned)v;
+      unsigned hi = (unsigned)(v >> 32);
+      const unsigned old = atomicAdd(w + 2 * c, lo);
+      hi += old + lo < old ? 1u : 0u;
+      if (hi) atomicAdd(w + 2 * c + 1, hi);
+    } else {
+      atomicAdd(g + c, v);
+    }
+  }
+};
+
 // Task state shared by the groups of one warp.
 struct alignas(16) MotifShared {
   unsigned long long range;    // second vertices not taken yet (pack_range)
@@ -179,7 +199,7 @@ __device__ __forceinline__ void mask_hist(const int2* list, int lo, int hi, unsi
 // Bound by instruction issue: a step of about 45 instructions takes W row entries (an owner
 // search by shuffles, one load of the entry, one 8-byte load of both bitmaps, one ballot).
 template <int K, int W, class Between>
-__device__ __forceinline__ unsigned long long leaf_sweep(const MotifCtx& c, unsigned long long* hist, MotifSweep<K>* sw,
+__device__ __forceinline__ unsigned long long leaf_sweep(const MotifCtx& c, const ClassHist& hist, MotifSweep<K>* sw,
                                                          const int2* E, int n, int lo, const int* lim, int v0,
                                                          unsigned quick_t, const uint32_t* Ub, const int32_t* E0,
                                                          int n0, const int2* runs1, size_t rstride, const int* runn,
@@ -269,7 +289,7 @@ __device__ __forceinline__ unsigned long long leaf_sweep(const MotifCtx& c, unsi
         for (int b = gl; b < MASKS; b += W) {
           const unsigned t = sw->rest[b];
           if (t) {
-            atomicAdd(hist + __ldg(c.q2c + code(m, b)), (unsigned long long)t);
+            hist.add(__ldg(c.q2c + code(m, b)), (unsigned long long)t);
             counted += t;
           }
         }
@@ -281,34 +301,34 @@ __device__ __forceinline__ unsigned long long leaf_sweep(const MotifCtx& c, unsi
   }
   if (c.sym && i0 < n) mask_hist<W>(E, i0, n, sw->rest, gl, gmask);
   __syncwarp(gmask);
-  for (int a = 1; a < MASKS; ++a) {
+  // every (a, b) to a lane
+  for (int ab = gl; ab < MASKS * MASKS; ab += W) {
+    const int a = ab / MASKS, b = ab % MASKS;
     const unsigned ra = sw->swept[a];
     if (ra == 0) continue;
-    for (int b = gl; b < MASKS; b += W) {
-      unsigned long long pairs = 0;
-      if (c.sym) {
-        const unsigned long long rb = sw->swept[b];
-        if (b == a) pairs = (rb & 1) ? rb * ((rb - 1) >> 1) : (rb >> 1) * (rb - 1);
-        else if (b > a) pairs = (unsigned long long)ra * rb;
-        pairs += (unsigned long long)ra * sw->rest[b];
-      }
-      const unsigned join = sw->joined[a * MASKS + b];
-      if (join) {
-        sw->joined[a * MASKS + b] = 0u;
-        atomicAdd(hist + __ldg(c.q2c + code(a, b | (1 << P))), (unsigned long long)join);
-      }
-      // (a pair joined in the order (a, b) was taken in that order or, with equal classes, in the
-      // other: the difference may be negative here, the class total is not)
-      if (pairs != join) atomicAdd(hist + __ldg(c.q2c + code(a, b)), pairs - join);
-      counted += pairs;
+    unsigned long long pairs = 0;
+    if (c.sym) {
+      const unsigned long long rb = sw->swept[b];
+      if (b == a) pairs = (rb & 1) ? rb * ((rb - 1) >> 1) : (rb >> 1) * (rb - 1);
+      else if (b > a) pairs = (unsigned long long)ra * rb;
+      pairs += (unsigned long long)ra * sw->rest[b];
     }
-    if (gl == 0) {
-      const unsigned fr = sw->fresh[a];
-      if (fr) {
-        sw->fresh[a] = 0u;
-        atomicAdd(hist + __ldg(c.q2c + code(a, 1 << P)), (unsigned long long)fr);
-        counted += fr;
-      }
+    const unsigned join = sw->joined[ab];
+    if (join) {
+      sw->joined[ab] = 0u;
+      hist.add(__ldg(c.q2c + code(a, b | (1 << P))), (unsigned long long)join);
+    }
+    // (a pair joined in the order (a, b) was taken in that order or, with equal classes, in the
+    // other: the difference may be negative here, the class total is not)
+    if (pairs != join) hist.add(__ldg(c.q2c + code(a, b)), pairs - join);
+    counted += pairs;
+  }
+  for (int a = gl; a < MASKS; a += W) {
+    const unsigned fr = sw->fresh[a];
+    if (fr) {
+      sw->fresh[a] = 0u;
+      hist.add(__ldg(c.q2c + code(a, 1 << P)), (unsigned long long)fr);
+      counted += fr;
     }
   }
   __syncwarp(gmask);
@@ -319,13 +339,13 @@ __device__ __forceinline__ unsigned long long leaf_sweep(const MotifCtx& c, unsi
 
 // k = 3: flushes the group's leaf-mask histogram (masks below 4) into the class counters.
 template <int W>
-__device__ __forceinline__ void flush_masks(unsigned* mh, const int32_t* q2c, unsigned long long* hist,
+__device__ __forceinline__ void flush_masks(unsigned* mh, const int32_t* q2c, const ClassHist& hist,
                                             unsigned long long& task_cnt, int gl, unsigned gmask) {
   for (int m = gl; m < 4; m += W) {
     const unsigned c = mh[m];
     if (c) {
       mh[m] = 0;
-      atomicAdd(hist + __ldg(q2c + m), (unsigned long long)c);
+      hist.add(__ldg(q2c + m), (unsigned long long)c);
       task_cnt += c;
     }
   }
@@ -399,7 +419,7 @@ __device__ __forceinline__ void motif_donate(const LBArgs& lb, MotifShared* ws, 
 // k = 3: the subgraphs (v0, w, x) with w the member of E_0 = N(v0) above v0 at index it.
 template <int W>
 __device__ __forceinline__ void leaf_pairs(const MotifCtx& c, unsigned* mh, const int32_t* E0, int n0, int it, int v0,
-                                           unsigned long long* hist, unsigned long long& task_cnt, int gl,
+                                           const ClassHist& hist, unsigned long long& task_cnt, int gl,
                                            unsigned gmask) {
   const int w = __ldg(E0 + it);
   const int32_t* Nw = c.g.adj + __ldg(c.g.row + w);
@@ -439,11 +459,10 @@ __device__ __forceinline__ void leaf_pairs(const MotifCtx& c, unsigned* mh, cons
 
 // Runs one task on the calling warp (all 32 lanes). level 0: second vertices [bb, ee) of v0
 // (task_range encoding); level L >= 1: replay path[0..L-1], then expand positions [bb, ee) of
-// E_L (group 0 only). Adds the task's subgraphs to hist (class counters in shared or global
-// memory); nodes counts expansions (every
+// E_L (group 0 only). Adds the task's subgraphs to hist; nodes counts expansions (every
 // lane of a group counts the same nodes; the caller keeps group leaders' counts only).
 template <int K, int W>
-__device__ __forceinline__ void motif_run_task(const MotifCtx& c, unsigned long long* hist, MotifShared* ws,
+__device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHist& hist, MotifShared* ws,
                                                int2* warp_arena, uint32_t* warp_bits, int v0, int bb, int ee,
                                                int level, const int* path, unsigned long long& nodes) {
   static_assert(W == 8 || W == 16 || W == 32, "virtual warp width must be 8, 16 or 32");
