@@ -562,7 +562,12 @@ int dm_batch_create(const dm_query* queries, int32_t n, const dm_opts* opts, int
     arena_bytes = std::max(arena_bytes, (need + 255) / 256 * 256);
   }
   const size_t budget = (size_t)8 << 30;
-  const size_t warps_fit = std::max<size_t>(BATCH_WARPS, budget / arena_bytes);
+  size_t bits_words = 0;  // vertex bitmaps of the largest motif query
+  for (int32_t i = 0; i < n; ++i)
+    if (desc[i].kind == DM_QUERY_MOTIF)
+      bits_words = std::max(bits_words, motif_warp_bit_words(desc[i].k, desc[i].bit_words, desc[i].vwarp));
+  const size_t warps_fit =
+      std::max<size_t>(BATCH_WARPS, budget / std::max(arena_bytes, bits_words * sizeof(uint32_t)));
   b->grid = std::max(1, std::min(b->grid, (int)(warps_fit / BATCH_WARPS)));
   const int warps = b->grid * BATCH_WARPS;
   // a threshold is a percentage of the warps (>= 100: this query never donates)
@@ -573,13 +578,8 @@ int dm_batch_create(const dm_query* queries, int32_t n, const dm_opts* opts, int
   ce = cudaMalloc(&b->d_arena, arena_bytes * (size_t)warps);
   if (ce != cudaSuccess)
     return fail_release(b, fail(DM_ECUDA, std::string("dm_batch_create: arena: ") + cudaGetErrorString(ce)));
-  // membership bitmaps of the motif queries: per warp, 32/W groups x 2 bitmaps over the
-  // largest motif graph (zeroed here; every task leaves them zero)
-  size_t bits_words = 0;
-  for (int32_t i = 0; i < n; ++i)
-    if (desc[i].kind == DM_QUERY_MOTIF)
-      bits_words = std::max(bits_words, (size_t)desc[i].bit_words * 2 * (32 / desc[i].vwarp));
-  if (bits_words && bits_words * sizeof(uint32_t) * (size_t)warps <= ((size_t)2 << 30)) {
+  // vertex bitmaps of the motif queries, per warp (zeroed here; every task leaves them zero)
+  if (bits_words) {
     b->bits_bytes = bits_words * sizeof(uint32_t) * (size_t)warps;
     ce = cudaMalloc(&b->d_bits, b->bits_bytes);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(b->d_bits, 0, b->bits_bytes, b->stream);
@@ -623,7 +623,7 @@ int dm_batch_create(const dm_query* queries, int32_t n, const dm_opts* opts, int
       d.mctx.maxdeg = d.maxdeg;
       d.mctx.arena_stride = d.arena_stride;
       d.mctx.bit_base = d.vbase;
-      d.mctx.bit_words = b->d_bits ? d.bit_words : 0;
+      d.mctx.bit_words = d.bit_words;
     }
   }
   if ((rc = upload(reinterpret_cast<void**>(&b->d_desc), desc.data(), sizeof(BatchQuery) * desc.size())))

@@ -1550,22 +1550,27 @@ int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_
   const int vwarp = (ctx.vwarp == 8 || ctx.vwarp == 16) ? ctx.vwarp : 32;
   const size_t per_warp = motif_arena_stride(k, maxdeg, vwarp) * sizeof(int2);
   const size_t budget = (size_t)8 << 30;
-  ctx.arena_warps = (int)std::min<size_t>((size_t)ctx.num_sms * 64, std::max<size_t>(8, budget / per_warp));
-  if ((rc = ensure_ws_bytes(&ws.d_scratch, &ws.scratch_cap, per_warp * ctx.arena_warps))) return rc;
-  // membership bitmaps (2 per group, zero between calls; skipped past 2 GB)
+  // (the kernel keeps 32 warps per SM)
+  ctx.arena_warps = (int)std::min<size_t>((size_t)ctx.num_sms * 32, std::max<size_t>(8, budget / per_warp));
+  // vertex bitmaps, zero between calls; past 2 GB they get up to a quarter of the free memory (at
+  // most 8 GB), and the launch as many warps as that holds
   const int bit_words = motif_bit_words(g->n);
-  const size_t bits_bytes = (size_t)bit_words * 2 * (32 / vwarp) * sizeof(uint32_t) * ctx.arena_warps;
-  uint32_t* d_bits = nullptr;
-  if (bits_bytes <= ((size_t)2 << 30)) {
-    if (ws.bits_cap < bits_bytes) {
-      cudaFree(ws.d_bits);
-      ws.d_bits = nullptr;
-      ws.bits_cap = 0;
-      DM_CUDA(cudaMalloc(&ws.d_bits, bits_bytes));
-      DM_CUDA(cudaMemsetAsync(ws.d_bits, 0, bits_bytes, ctx.stream));
-      ws.bits_cap = bits_bytes;
-    }
-    d_bits = ws.d_bits;
+  const size_t warp_bits = sizeof(uint32_t) * motif_warp_bit_words(k, bit_words, vwarp);
+  if (warp_bits * ctx.arena_warps > ((size_t)2 << 30)) {
+    size_t free_b = 0, tot_b = 0;
+    DM_CUDA(cudaMemGetInfo(&free_b, &tot_b));
+    const size_t room = std::max<size_t>(ws.bits_cap, std::min<size_t>((size_t)8 << 30, free_b / 4));
+    ctx.arena_warps = (int)std::min<size_t>(ctx.arena_warps, std::max<size_t>(8, room / warp_bits));
+  }
+  if ((rc = ensure_ws_bytes(&ws.d_scratch, &ws.scratch_cap, per_warp * ctx.arena_warps))) return rc;
+  const size_t bits_bytes = warp_bits * ctx.arena_warps;
+  if (ws.bits_cap < bits_bytes) {
+    cudaFree(ws.d_bits);
+    ws.d_bits = nullptr;
+    ws.bits_cap = 0;
+    DM_CUDA(cudaMalloc(&ws.d_bits, bits_bytes));
+    ws.bits_cap = bits_bytes;
+    DM_CUDA(cudaMemsetAsync(ws.d_bits, 0, bits_bytes, ctx.stream));
   }
   const bool want_log = o && o->subtree_counts;
   if (want_log) {
@@ -1596,7 +1601,7 @@ int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_
   L.maxdeg = maxdeg;
   L.per_root = want_log ? ws.d_per_root : nullptr;
   L.vwarp = vwarp;
-  L.bits = d_bits;
+  L.bits = ws.d_bits;
   L.bit_words = bit_words;
   L2Window l2;
   if (o && (o->flags & DM_FLAG_L2_PERSIST) &&
@@ -1619,7 +1624,7 @@ int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_
                             cudaMemcpyDeviceToHost, ctx.stream));
   DM_CUDA(cudaStreamSynchronize(ctx.stream));
   const DevCounters h = *ws.h_out;
-  if (h.err && d_bits) {
+  if (h.err && ws.d_bits) {
     // a failed launch can leave bits set: clear them for the next call
     DM_CUDA(cudaMemsetAsync(ws.d_bits, 0, ws.bits_cap, ctx.stream));
     DM_CUDA(cudaStreamSynchronize(ctx.stream));

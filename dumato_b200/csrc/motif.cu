@@ -19,14 +19,14 @@ struct MotifArgs {
   int n_classes;
   unsigned long long* hist;    // n_classes
   int2* arena;                 // per warp: 32/W group arenas of c.arena_stride int2
-  uint32_t* bits;              // per warp: 32/W groups x 2 membership bitmaps of c.bit_words (or null)
+  uint32_t* bits;              // per warp: 32/W groups x motif_bit_stride(k) bitmaps of c.bit_words (k >= 4)
   const int32_t* parts;        // optional per-root-entry part word (p | P << 16)
   int bits_smem;               // the bitmaps live in shared memory (zeroed at launch), not in `bits`
 };
 
-// Shared-memory budget of one block's membership bitmaps; larger graphs keep them in global
-// memory.
-constexpr size_t MOTIF_SMEM_BITS_MAX = 64 * 1024;
+// Shared-memory budget of one block's vertex bitmaps (three blocks per SM then still fit; up to
+// 13,800 vertices for k <= 5, 9,200 above); larger graphs keep them in global memory.
+constexpr size_t MOTIF_SMEM_BITS_MAX = 54 * 1024;
 
 template <int K, int W>
 __global__ void __launch_bounds__(32 * MOTIF_WARPS, 4) motif_kernel(const __grid_constant__ MotifArgs a) {
@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(32 * MOTIF_WARPS, 4) motif_kernel(const __grid
   const int wib = warp_in_block();
   MotifShared* ws = reinterpret_cast<MotifShared*>(wbase + motif_warp_smem<K, W>() * wib);
   const MotifCtx& c = a.c;
-  const size_t warp_bit_words = (size_t)c.bit_words * 2 * (32 / W);
+  const size_t warp_bit_words = (size_t)c.bit_words * motif_bit_stride(K) * (32 / W);
   uint32_t* sbits = reinterpret_cast<uint32_t*>(wbase + motif_warp_smem<K, W>() * MOTIF_WARPS);
   for (int cl = threadIdx.x; cl < a.n_classes; cl += blockDim.x) bhist[cl] = 0;
   if (a.bits_smem)
@@ -93,6 +93,11 @@ __global__ void __launch_bounds__(32 * MOTIF_WARPS, 4) motif_kernel(const __grid
     if (bhist[cl]) atomicAdd(a.hist + cl, bhist[cl]);
 }
 
+size_t motif_warp_bit_words(int k, int bit_words, int vwarp) {
+  const int w = (vwarp == 8 || vwarp == 16) ? vwarp : 32;
+  return k < 4 ? 0 : (size_t)bit_words * motif_bit_stride(k) * (size_t)(32 / w);
+}
+
 size_t motif_arena_stride(int k, int maxdeg, int vwarp) {
   const int w = (vwarp == 8 || vwarp == 16) ? vwarp : 32;
   return motif_group_stride(k, maxdeg) * (size_t)(32 / w);
@@ -101,8 +106,8 @@ size_t motif_arena_stride(int k, int maxdeg, int vwarp) {
 template <int K, int W>
 static int launch_motif(MotifArgs a, LaunchCtx& ctx, int* grid_out) {
   const int block = 32 * MOTIF_WARPS;
-  const size_t bits_bytes = (size_t)a.c.bit_words * 2 * (32 / W) * sizeof(uint32_t) * MOTIF_WARPS;
-  a.bits_smem = a.bits && a.c.bit_words > 0 && bits_bytes <= MOTIF_SMEM_BITS_MAX ? 1 : 0;
+  const size_t bits_bytes = (size_t)a.c.bit_words * motif_bit_stride(K) * (32 / W) * sizeof(uint32_t) * MOTIF_WARPS;
+  a.bits_smem = K >= 4 && bits_bytes <= MOTIF_SMEM_BITS_MAX ? 1 : 0;
   const size_t smem = sizeof(unsigned long long) * ((a.n_classes + 1) & ~1) +
                       motif_warp_smem<K, W>() * MOTIF_WARPS + (a.bits_smem ? bits_bytes : 0);
   auto kern = motif_kernel<K, W>;
@@ -144,7 +149,7 @@ int motif_launch(const MotifLaunch& L, LaunchCtx& ctx, int* grid) {
   a.c.arena_stride = (int)motif_group_stride(L.k, L.maxdeg);
   a.c.per_root = L.per_root;
   a.c.bit_base = 0;
-  a.c.bit_words = L.bits ? L.bit_words : 0;
+  a.c.bit_words = L.bit_words;
   a.bits = L.bits;
   a.roots = L.roots;
   a.n_roots = L.n_roots;

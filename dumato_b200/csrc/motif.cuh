@@ -15,21 +15,22 @@
 // (the inherited members keep their source, and the only new constraint is "> w"; the new
 // members have w as their source). Every member carries its adjacency mask to the prefix
 // (bit i = edge to v_i), so quick codes come from masks, not from the reference's per-leaf
-// adjacency scans. The excluded set U_t = N(v_0..v_t) cap (v0, inf) is kept as disjoint
-// sorted runs (run 0 = N(v0) above v0, run i = excl(v_i)). E_t is kept sorted by vertex id, so
-// the inherited members are the suffix of E_t after w.
+// adjacency scans. The excluded set U_t = N(v_0..v_t) cap (v0, inf) is kept as disjoint runs
+// (run 0 = N(v0) above v0, run i = excl(v_i)); E_t lists the inherited members in E_{t-1}'s order,
+// then excl(v_t) ascending, so it is a deterministic function of the path.
 //
 // The last two vertices are counted in bulk (leaf_sweep): once E_{k-3} of a (k-2)-prefix is
 // materialised, no member is expanded. With R_a the number of members of mask a, the pairs
 // (w, x) of members contribute R_a R_b (C(R_a,2) for a = b) subgraphs of masks a, b, of which
 // those joined by an edge are moved to the joined class; and a member w adds its neighbours above
-// v0 that lie outside U_{k-3}. So the sweep only walks the members' rows above v0 once, testing
-// each neighbour against the two bitmaps, and adds to the class counters once per prefix and
-// mask pair. The rows of W members are laid end to end, one entry per lane, so rows shorter than
+// v0 that lie outside U_{k-3}. So the sweep only walks the members' rows above v0 once, looking
+// each neighbour up in the bitmaps, and adds to the class counters once per prefix and mask pair. The rows of W members are laid end to end, one entry per lane, so rows shorter than
 // the group waste no lanes. Expanding every member w on its own (its row scanned, its leaf
 // masks looked up and flushed) took 12.6 ms for k = 5 on a Chung-Lu graph of 3,000 vertices and
 // 18,000 edges, 10.4 ms for k = 6 on a random graph of 2,000 / 10,000, 387 ms for a batch of 24
-// graphs; the sweep takes 7.0, 5.2 and 86 ms.
+// graphs; the sweep took 6.5, 5.3 and 86 ms while the sets were sorted lists in global memory that
+// masks and adjacency were searched in, and takes 3.8, 4.2 and 51 ms with one bitmap per mask bit
+// and the sets of level k-3 in shared memory.
 //
 // Virtual warps (the reference's DM_WCV variant, src/DM_WCV/DuMatoGPU.cu:12-37): with W < 32
 // the groups of a warp take second vertices of the same task from its shared item range and
@@ -83,15 +84,15 @@ struct ClassHist {
   unsigned* w;
   unsigned long long* g;
   __device__ __forceinline__ void add(int c, unsigned long long v) const {
-    if (w) {
-      const unsigned lo = (unsigned)v;
-      unsigned hi = (unsigned)(v >> 32);
-      const unsigned old = atomicAdd(w + 2 * c, lo);
-      hi += old + lo < old ? 1u : 0u;
-      if (hi) atomicAdd(w + 2 * c + 1, hi);
-    } else {
+    if (!w) {
       atomicAdd(g + c, v);
+      return;
     }
+    const unsigned lo = (unsigned)v;
+    unsigned hi = (unsigned)(v >> 32);
+    const unsigned old = atomicAdd(w + 2 * c, lo);
+    hi += old + lo < old ? 1u : 0u;
+    if (hi) atomicAdd(w + 2 * c + 1, hi);
   }
 };
 
@@ -102,9 +103,19 @@ struct alignas(16) MotifShared {
   int busy;                    // serialises level-0 splits
 };
 
+// The lists of level k-3 of one group, in shared memory while they fit (arena otherwise): they are
+// written and read back at once, and a global store read back by the same warp costs a trip to L2.
+template <int W>
+struct alignas(16) MotifLists {
+  static constexpr int CAP = 4 * W;
+  int2 ext[CAP];
+  int run[CAP];
+};
+
+// A warp's shared memory: MotifShared | a MotifGroup, a MotifSweep and a MotifLists per group.
 template <int K, int W>
 __host__ __device__ constexpr size_t motif_warp_smem() {
-  return sizeof(MotifShared) + (sizeof(MotifGroup) + sizeof(MotifSweep<K>)) * (32 / W);
+  return sizeof(MotifShared) + (sizeof(MotifGroup) + sizeof(MotifSweep<K>) + sizeof(MotifLists<W>)) * (32 / W);
 }
 
 // Everything a motif task needs besides its own (v0, range) or prefix.
@@ -117,33 +128,42 @@ struct MotifCtx {
   int arena_stride;            // int2 slots per group
   unsigned long long* per_root;  // optional: subgraphs found under each v0 (subtree logger)
   int bit_base;                // membership bitmaps index vertex x at bit x - bit_base
-  int bit_words;               // 32-bit words per bitmap (0 = no bitmaps: binary searches only)
+  int bit_words;               // 32-bit words per bitmap
 };
 
-// Membership bitmaps of one group (bit_words pairs of words, all zero between tasks; word 2i of
-// U and word 2i + 1 of E, so that one 8-byte load answers both questions): U holds
-// U_t = N(v_0..v_t) above v0 for the levels materialised on the current path, E holds E_{k-3}.
-// They turn the sweep and the exclusion test into one probe per neighbour instead of binary
-// searches over the runs (k >= 4).
-__device__ __forceinline__ bool bit_test(const uint32_t* b, int x) { return (b[2 * (x >> 5)] >> (x & 31)) & 1u; }
+// Vertex bitmaps of one group (k >= 4), all zero between tasks: the words of 32 vertices lie
+// together, so one or three vector loads answer everything about a vertex. Word 0: U_t above v0
+// for the levels materialised on the current path; word 1 + i: the members of E_{k-3} adjacent to
+// v_i (a member's mask, bit by bit). Word k - 2 (i = k - 3) also marks N(w) while a set is built.
+__host__ __device__ constexpr int motif_bit_stride(int k) { return k <= 5 ? 4 : 6; }
 
-template <int W>
-__device__ __forceinline__ void bits_flip_ids(uint32_t* b, int base, const int32_t* ids, int n, bool set, int gl) {
-  for (int i = gl; i < n; i += W) {
-    const int x = __ldg(ids + i) - base;
-    if (set) atomicOr(b + 2 * (x >> 5), 1u << (x & 31));
-    else atomicAnd(b + 2 * (x >> 5), ~(1u << (x & 31)));
+template <int K>
+struct MotifBits {
+  static constexpr int STRIDE = motif_bit_stride(K);
+  static constexpr int MARK = K - 2;
+  uint32_t* b;
+  int base;
+  __device__ __forceinline__ uint32_t* at(int x) const { return b + STRIDE * ((x - base) >> 5); }
+  __device__ __forceinline__ uint32_t bit(int x) const { return 1u << ((x - base) & 31); }
+  // (x in U, mask of x in E_{k-3})
+  __device__ __forceinline__ void look(int x, bool& in_u, unsigned& mask) const {
+    const int s = (x - base) & 31;
+    if constexpr (STRIDE == 4) {
+      const uint4 v = *reinterpret_cast<const uint4*>(at(x));
+      in_u = (v.x >> s) & 1u;
+      mask = ((v.y >> s) & 1u) | (((v.z >> s) & 1u) << 1);
+      if constexpr (K >= 5) mask |= ((v.w >> s) & 1u) << 2;
+    } else {
+      const uint2* q = reinterpret_cast<const uint2*>(at(x));
+      const uint2 v0 = q[0], v1 = q[1], v2 = q[2];
+      in_u = (v0.x >> s) & 1u;
+      mask = ((v0.y >> s) & 1u) | (((v1.x >> s) & 1u) << 1) | (((v1.y >> s) & 1u) << 2) | (((v2.x >> s) & 1u) << 3);
+      if constexpr (K >= 7) mask |= ((v2.y >> s) & 1u) << 4;
+    }
   }
-}
-
-template <int W>
-__device__ __forceinline__ void bits_flip_list(uint32_t* b, int base, const int2* list, int n, bool set, int gl) {
-  for (int i = gl; i < n; i += W) {
-    const int x = list[i].x - base;
-    if (set) atomicOr(b + 2 * (x >> 5), 1u << (x & 31));
-    else atomicAnd(b + 2 * (x >> 5), ~(1u << (x & 31)));
-  }
-}
+  __device__ __forceinline__ void set(int x, int word) const { atomicOr(at(x) + word, bit(x)); }
+  __device__ __forceinline__ void clear(int x, int word) const { atomicAnd(at(x) + word, ~bit(x)); }
+};
 
 // int2 slots of one group's arena: extension levels 1..k-3 (level t holds at most
 // (t+1) * maxdeg members) then runs 1..k-3 (at most maxdeg each).
@@ -154,30 +174,7 @@ __host__ __device__ inline size_t motif_group_stride(int k, int maxdeg) {
   return s < 1 ? 1 : s;
 }
 
-// First index in [lo, hi) of an id-sorted (vertex, mask) list whose vertex is >= x.
-__device__ __forceinline__ int lower_bound2(const int2* a, int lo, int hi, int32_t x) {
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (a[mid].x < x) lo = mid + 1; else hi = mid;
-  }
-  return lo;
-}
-
 __device__ __forceinline__ int ilog2p1(int x) { return 32 - __clz(x | 1); }
-
-// Membership of x in the disjoint sorted runs 0..t (run 0 is the CSR suffix of v0; run i >= 1
-// starts at runs1 + (i - 1) * rstride).
-__device__ __forceinline__ bool in_runs(int32_t x, const int32_t* run0, int n0, const int2* runs1, size_t rstride,
-                                        const int* runn, int t) {
-  if (contains(run0, n0, x)) return true;
-  for (int i = 1; i <= t; ++i) {
-    const int2* r = runs1 + (size_t)(i - 1) * rstride;
-    const int nr = runn[i];
-    const int j = lower_bound2(r, 0, nr, x);
-    if (j < nr && r[j].x == x) return true;
-  }
-  return false;
-}
 
 // Adds the masks of list[lo, hi) to the group's 32-entry histogram h (aggregated per mask).
 template <int W>
@@ -190,30 +187,53 @@ __device__ __forceinline__ void mask_hist(const int2* list, int lo, int hi, unsi
   __syncwarp(gmask);
 }
 
-// Sweeps members [lo, *lim) of the materialised set E = E_{K-3} (n members, sorted by id) of the
-// prefix whose quick code is quick_t: every subgraph with at least one of its last two vertices
-// in the range, the other one after it in E or new, is added to hist. `between` runs after every
-// batch of W members with the next position (group-uniform; it may lower *lim). Returns this
-// lane's share of the subgraphs counted.
+// Tables whose classes depend on the order of the last two vertices: the pairs of member i of
+// E (n members) with every member of a larger id, in that order (a member list per mask first).
+template <int K, int W>
+__device__ __noinline__ unsigned long long leaf_ordered(const MotifCtx& c, const ClassHist& hist, MotifSweep<K>* sw,
+                                                        const int2* E, int n, int i, unsigned quick_t, int gl,
+                                                        unsigned gmask) {
+  unsigned long long counted = 0;
+  const int2 w = E[i];
+  for (int j0 = 0; j0 < n; j0 += W) {
+    const int j = j0 + gl;
+    const int2 x = j < n ? E[j] : make_int2(-1, 0);
+    dm_gpm::aggregate_pattern<W>(sw->rest, x.y, x.x > w.x);
+  }
+  __syncwarp(gmask);
+  for (int b = gl; b < MotifSweep<K>::MASKS; b += W) {
+    const unsigned t = sw->rest[b];
+    sw->rest[b] = 0u;
+    if (t) {
+      const unsigned q = quick_t + ((unsigned)w.y << quick_off(K - 2)) + ((unsigned)b << quick_off(K - 1));
+      hist.add(__ldg(c.q2c + q), (unsigned long long)t);
+      counted += t;
+    }
+  }
+  __syncwarp(gmask);
+  return counted;
+}
+
+// Sweeps members [lo, *lim) of the materialised set E = E_{K-3} (n members) of the prefix whose
+// quick code is quick_t: every pair of a swept member with a member after it in E, and of a swept
+// member with a new vertex, is added to hist (an edge between two members is credited to the
+// one of smaller id, wherever that one is swept). `between` runs after every batch of W
+// members with the next position (group-uniform; it may lower *lim). Returns this lane's share of
+// the subgraphs counted.
 //
-// Bound by instruction issue: a step of about 45 instructions takes W row entries (an owner
-// search by shuffles, one load of the entry, one 8-byte load of both bitmaps, one ballot).
+// Bound by instruction issue: a step of about 40 instructions takes W row entries (an owner
+// search by shuffles, one load of the entry, one lookup in the bitmaps, one ballot).
 template <int K, int W, class Between>
 __device__ __forceinline__ unsigned long long leaf_sweep(const MotifCtx& c, const ClassHist& hist, MotifSweep<K>* sw,
                                                          const int2* E, int n, int lo, const int* lim, int v0,
-                                                         unsigned quick_t, const uint32_t* Ub, const int32_t* E0,
-                                                         int n0, const int2* runs1, size_t rstride, const int* runn,
-                                                         int gl, int gsrc, unsigned gmask, Between&& between) {
+                                                         unsigned quick_t, const MotifBits<K>& bits, int gl, int gsrc,
+                                                         unsigned gmask, Between&& between) {
   constexpr int P = K - 2;  // position of the first of the two vertices; the second is at K - 1
   constexpr int MASKS = MotifSweep<K>::MASKS;
   unsigned long long counted = 0;
   auto code = [&](unsigned a, unsigned b) -> unsigned {
-    return quick_t + (P >= 2 ? a << quick_off(P) : 0u) + (b << quick_off(K - 1));
+    return quick_t + (a << quick_off(P)) + (b << quick_off(K - 1));
   };
-  if (!c.sym) {
-    // pairs in id order, one member at a time: the masks of the members after it
-    mask_hist<W>(E, lo, n, sw->rest, gl, gmask);
-  }
   int i0 = lo;
   while (i0 < *reinterpret_cast<const volatile int*>(lim)) {
     const int end = min(*reinterpret_cast<const volatile int*>(lim), i0 + W);
@@ -246,56 +266,29 @@ __device__ __forceinline__ unsigned long long leaf_sweep(const MotifCtx& c, cons
         const int o = __shfl_sync(gmask, off, j + h, W);
         j = o <= f ? j + h : j;
       }
-      const int ob = __shfl_sync(gmask, base, j, W) + (f - __shfl_sync(gmask, off, j, W));
+      const int ob = __shfl_sync(gmask, base - off, j, W) + f;
       const int ow = __shfl_sync(gmask, wm.x, j, W);
       const int om = __shfl_sync(gmask, wm.y, j, W);
-      bool in_u = false, in_e = false;
-      int x = 0;
+      bool in_u = false;
+      unsigned xm = 0;
       if (f < total) {
-        x = __ldg(c.g.adj + ob);
-        if (Ub) {
-          const int xb = x - c.bit_base;
-          const uint2 ue = *reinterpret_cast<const uint2*>(Ub + 2 * (xb >> 5));
-          in_u = (ue.x >> (xb & 31)) & 1u;
-          in_e = x > ow && ((ue.y >> (xb & 31)) & 1u);
-        } else {
-          in_u = in_runs(x, E0, n0, runs1, rstride, runn, K - 3);
-          in_e = in_u && x > ow;
-        }
+        const int x = __ldg(c.g.adj + ob);
+        bits.look(x, in_u, xm);
+        if (xm && x > ow) atomicAdd(&sw->joined[om * MASKS + xm], 1u);
       }
       const unsigned bal = __ballot_sync(gmask, in_u) >> gsrc;
       const int a0 = min(max(off - f0, 0), W), a1 = min(max(off + len - f0, 0), W);
       const unsigned upto1 = a1 >= 32 ? 0xffffffffu : (1u << a1) - 1u;
       const unsigned upto0 = a0 >= 32 ? 0xffffffffu : (1u << a0) - 1u;
       inside += __popc(bal & upto1 & ~upto0);
-      if (in_e) {
-        const int q = lower_bound2(E, i0 + j + 1, n, x);
-        if (q < n) {
-          const int2 y = E[q];
-          if (y.x == x) atomicAdd(&sw->joined[om * MASKS + y.y], 1u);
-        }
-      }
     }
     if (valid) {
       if (len > (int)inside) atomicAdd(&sw->fresh[wm.y], (unsigned)len - inside);
       atomicAdd(&sw->swept[wm.y], 1u);
     }
     __syncwarp(gmask);
-    if (!c.sym) {
-      for (int i = i0; i < end; ++i) {
-        const int m = E[i].y;
-        if (gl == 0) sw->rest[m] -= 1u;
-        __syncwarp(gmask);
-        for (int b = gl; b < MASKS; b += W) {
-          const unsigned t = sw->rest[b];
-          if (t) {
-            hist.add(__ldg(c.q2c + code(m, b)), (unsigned long long)t);
-            counted += t;
-          }
-        }
-        __syncwarp(gmask);
-      }
-    }
+    if (!c.sym)
+      for (int i = i0; i < end; ++i) counted += leaf_ordered<K, W>(c, hist, sw, E, n, i, quick_t, gl, gmask);
     i0 = end;
     between(end);
   }
@@ -314,13 +307,13 @@ __device__ __forceinline__ unsigned long long leaf_sweep(const MotifCtx& c, cons
       pairs += (unsigned long long)ra * sw->rest[b];
     }
     const unsigned join = sw->joined[ab];
+    // (a pair joined in the order (a, b) may have been counted in the other order, or in another
+    // range of E: the difference may be negative here, the class total is not)
+    if (pairs != join) hist.add(__ldg(c.q2c + code(a, b)), pairs - join);
     if (join) {
       sw->joined[ab] = 0u;
       hist.add(__ldg(c.q2c + code(a, b | (1 << P))), (unsigned long long)join);
     }
-    // (a pair joined in the order (a, b) was taken in that order or, with equal classes, in the
-    // other: the difference may be negative here, the class total is not)
-    if (pairs != join) hist.add(__ldg(c.q2c + code(a, b)), pairs - join);
     counted += pairs;
   }
   for (int a = gl; a < MASKS; a += W) {
@@ -402,8 +395,7 @@ __device__ __forceinline__ void motif_donate(const LBArgs& lb, MotifShared* ws, 
   for (int s = floor; s <= t; ++s) {
     const int ps = sg->pos[s], lim = sg->lim[s];
     if (lim - ps >= 2) {
-      // E_s is sorted by id: member i inherits the n - i - 1 members above it
-      const int mid = split_mid(ps, lim, sg->n[s]);
+      const int mid = split_mid(ps, lim, 0);
       int path[QPATH];
       path[0] = it;
       for (int j = 1; j < s && j < QPATH; ++j) path[j] = sg->pos[j] - 1;
@@ -471,23 +463,26 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHis
   const int gi = lane / W;
   const unsigned gmask = (W == 32) ? FULL_MASK : (((1u << W) - 1u) << (gi * W));
   const int gsrc = gi * W;  // the group leader's lane
-  // the warp's words: MotifShared | a MotifGroup per group | a MotifSweep per group
-  MotifGroup* sg = reinterpret_cast<MotifGroup*>(ws + 1) + gi;
-  MotifSweep<K>* sw = reinterpret_cast<MotifSweep<K>*>(reinterpret_cast<MotifGroup*>(ws + 1) + 32 / W) + gi;
+  // the warp's words (motif_warp_smem)
+  MotifGroup* const groups = reinterpret_cast<MotifGroup*>(ws + 1);
+  MotifSweep<K>* const sweeps = reinterpret_cast<MotifSweep<K>*>(groups + 32 / W);
+  MotifGroup* sg = groups + gi;
+  MotifSweep<K>* sw = sweeps + gi;
+  MotifLists<W>* const sl = reinterpret_cast<MotifLists<W>*>(sweeps + 32 / W) + gi;
   // level t (1..K-3): extension list E_t at ext_at(t); run t at run_at(t) (no pointer
   // tables, so nothing indexed dynamically lives in local memory)
   int2* const arena = warp_arena + (size_t)gi * c.arena_stride;
   const size_t md = (size_t)c.maxdeg;
   auto ext_at = [&](int t) -> int2* { return arena + md * (size_t)(t * (t + 1) / 2 - 1) + 32 * (size_t)(t - 1); };
   int2* const runs1 = ext_at(K - 2);
-  const size_t rstride = md + 32;
-  auto run_at = [&](int t) -> int2* { return runs1 + (size_t)(t - 1) * rstride; };
-  // (k = 3 has a single level: setting and clearing E_0's bits per task costs more than the
-  // binary searches it saves)
-  const bool use_bits = K >= 4 && warp_bits != nullptr && c.bit_words > 0;
-  uint32_t* const Ub = use_bits ? warp_bits + (size_t)gi * 2 * c.bit_words : nullptr;
-  uint32_t* const Eb = use_bits ? Ub + 1 : nullptr;
-  int bdepth = 0;  // levels 1..bdepth have their run (and, at level k-3, E) bits set
+  auto run_at = [&](int t) -> int* { return reinterpret_cast<int*>(runs1 + (size_t)(t - 1) * (md + 32)); };
+  // (k = 3 has a single level and uses binary searches only)
+  constexpr bool use_bits = K >= 4;
+  const MotifBits<K> bits{use_bits ? warp_bits + (size_t)gi * MotifBits<K>::STRIDE * c.bit_words : nullptr, c.bit_base};
+  int bdepth = 0;         // levels 1..bdepth have their bits set
+  bool top_small = true;  // the lists of level K-3 are in shared memory
+  auto ext_of = [&](int t) -> int2* { return t == K - 3 && top_small ? sl->ext : ext_at(t); };
+  auto run_of = [&](int t) -> int* { return t == K - 3 && top_small ? sl->run : run_at(t); };
   unsigned long long task_cnt = 0;
   const long long t_start = global_ns();
   // E_0 = run 0 = N(v0) above v0: a suffix of the sorted CSR row
@@ -510,7 +505,8 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHis
     sg->spill_lo = sg->spill_hi = 0;
   }
   for (int m = gl; m < (int)(sizeof(MotifSweep<K>) / sizeof(unsigned)); m += W) reinterpret_cast<unsigned*>(sw)[m] = 0u;
-  if (use_bits) bits_flip_ids<W>(Ub, c.bit_base, E0, n0, true, gl);
+  if constexpr (use_bits)
+    for (int i = gl; i < n0; i += W) bits.set(__ldg(E0 + i), 0);
   MotifDemand dm;  // group leader
   if (gl == 0) motif_sample(c.lb, dm);
   unsigned long long checked = nodes;
@@ -518,8 +514,17 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHis
   // drops the bits of levels from..bdepth (the group's lanes, then a group barrier)
   auto drop_levels = [&](int from) {
     for (int L = bdepth; L >= from; --L) {
-      bits_flip_list<W>(Ub, c.bit_base, run_at(L), sg->runn[L], false, gl);
-      if (L == K - 3) bits_flip_list<W>(Eb, c.bit_base, ext_at(L), sg->n[L], false, gl);
+      const int* Rl = run_of(L);
+      for (int i = gl; i < sg->runn[L]; i += W) bits.clear(Rl[i], 0);
+      if (L == K - 3) {
+        const int2* El = ext_of(L);
+        for (int i = gl; i < sg->n[L]; i += W) {
+          const int2 e = El[i];
+#pragma unroll
+          for (int q = 0; q <= K - 3; ++q)
+            if ((e.y >> q) & 1) bits.clear(e.x, 1 + q);
+        }
+      }
     }
     if (bdepth >= from) bdepth = from - 1;
     __syncwarp(gmask);
@@ -583,63 +588,79 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHis
         if (p >= 2) quick_p += ((unsigned)wmask & ((1u << p) - 1u)) << quick_off(p);
         const int32_t* Nw = c.g.adj + __ldg(c.g.row + w);
         const int dw = __ldg(c.g.deg + w);
-        // inherited members: e in E_t with e > w. E_t is sorted by vertex id and w is its
-        // member at position pos[t] - 1 (E_0: index it), so they are the suffix from there.
+        // inherited members: e in E_t with e > w (E_0 is sorted: those after index it)
         const int2* Et = t == 0 ? nullptr : ext_at(t);
-        const int nE = (t == 0) ? n0 : sg->n[t];
-        const int startE = (t == 0) ? it + 1 : sg->pos[t];
-        // materialise E_{p} = inherited + excl(w), merged by vertex id; excl(w) is also run
-        // p. Both parts are sorted and disjoint, so each member's place is its index in its
-        // own part plus the number of smaller members of the other part.
-        int2* Ep = ext_at(p);
-        int2* Rp = run_at(p);
-        if (use_bits) drop_levels(p);  // the previous member's sets at levels >= p
+        const int nE = t == 0 ? n0 : sg->n[t];
+        drop_levels(p);  // the previous member's sets at levels >= p
         const int sw0 = dw <= 2 * W ? 0 : lower_bound(Nw, 0, dw, v0 + 1);
+        if (p == K - 3) top_small = (t == 0 ? n0 - it - 1 : nE) + (dw - sw0) <= MotifLists<W>::CAP;
+        int2* const Ep = ext_of(p);
+        int* const Rp = run_of(p);
+        // N(w) above v0: marked, and listed as run p where outside U_t
         int rn = 0;
         for (int i0 = sw0; i0 < dw; i0 += W) {
           const int i = i0 + gl;
-          int32_t x = 0;
+          const int x = i < dw ? __ldg(Nw + i) : 0;
+          const bool above = i < dw && x > v0;
           bool nw = false;
-          if (i < dw && Nw[i] > v0) {
-            x = Nw[i];
-            nw = use_bits ? !bit_test(Ub, x - c.bit_base) : !in_runs(x, E0, n0, runs1, rstride, sg->runn, t);
+          if (above) {
+            nw = !(bits.at(x)[0] & bits.bit(x));
+            bits.set(x, MotifBits<K>::MARK);
           }
           const unsigned bal = __ballot_sync(gmask, nw) >> gsrc;
-          if (nw) Rp[rn + __popc(bal & ((1u << gl) - 1u))] = make_int2(x, 0);
+          if (nw) Rp[rn + __popc(bal & ((1u << gl) - 1u))] = x;
           rn += __popc(bal);
         }
         __syncwarp(gmask);
-        for (int i = startE + gl; i < nE; i += W) {
-          int ev, em;
-          if (t == 0) {
-            ev = __ldg(E0 + i);
-            em = 1;
-          } else {
-            const int2 x = Et[i];
-            ev = x.x;
-            em = x.y;
+        // the inherited members, with their bit for w
+        int m = 0;
+        for (int i0 = t == 0 ? it + 1 : 0; i0 < nE; i0 += W) {
+          const int i = i0 + gl;
+          int2 e = make_int2(-1, 0);
+          if (i < nE) e = t == 0 ? make_int2(__ldg(E0 + i), 1) : Et[i];
+          const bool keep = e.x > w;
+          const unsigned bal = __ballot_sync(gmask, keep) >> gsrc;
+          if (keep) {
+            if (p == K - 3) {
+#pragma unroll
+              for (int q = 0; q < K - 3; ++q)
+                if ((e.y >> q) & 1) bits.set(e.x, 1 + q);
+            }
+            if (bits.at(e.x)[MotifBits<K>::MARK] & bits.bit(e.x)) e.y |= 1 << p;
+            Ep[m + __popc(bal & ((1u << gl) - 1u))] = e;
           }
-          if (contains(Nw, dw, ev)) em |= 1 << p;
-          Ep[(i - startE) + lower_bound2(Rp, 0, rn, ev)] = make_int2(ev, em);
+          m += __popc(bal);
         }
-        for (int j = gl; j < rn; j += W) {
-          const int32_t x = Rp[j].x;
-          const int cnt_lt = (t == 0) ? lower_bound(E0, 0, n0, x) : lower_bound2(Et, 0, nE, x);
-          Ep[j + max(0, cnt_lt - startE)] = make_int2(x, 1 << p);
-        }
-        const int m = (nE - startE) + rn;
         __syncwarp(gmask);
-        if (use_bits) {
-          bits_flip_list<W>(Ub, c.bit_base, Rp, rn, true, gl);
-          if (p == K - 3) bits_flip_list<W>(Eb, c.bit_base, Ep, m, true, gl);
-          bdepth = p;
-          __syncwarp(gmask);
+        // the marks: dropped, but at level K - 3 they stay as the members' bit for w (new vertices and
+        // inherited members; a vertex of U_t that is no member has no other bit)
+        for (int i = sw0 + gl; i < dw; i += W) {
+          const int x = __ldg(Nw + i);
+          if (x <= v0) continue;
+          bool stays = false;
+          if (p == K - 3) {
+            bool in_u;
+            unsigned mask;
+            bits.look(x, in_u, mask);
+            stays = !in_u || (mask & ((1u << (K - 3)) - 1u)) != 0u;
+          }
+          if (!stays) bits.clear(x, MotifBits<K>::MARK);
         }
+        __syncwarp(gmask);
+        for (int j = gl; j < rn; j += W) {
+          const int x = Rp[j];
+          Ep[m + j] = make_int2(x, 1 << p);
+          bits.set(x, 0);
+        }
+        m += rn;
+        bdepth = p;
+        __syncwarp(gmask);
         if (p < level) {
           // replaying a donated prefix: the path fixes the member expanded at level p
           const int idx = (p < QPATH) ? path[p] : -1;
           if (idx < 0 || idx >= m) {
             if (gl == 0) set_err(c.lb.ctr, ERR_BAD_TASK);
+            bdepth = p - 1;  // (its lists are not recorded; the host clears the bits of a failed call)
             bad = true;
             break;
           }
@@ -670,8 +691,8 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHis
         if (p == K - 3) {
           // the last two vertices in bulk
           int last = first_pos;
-          task_cnt += leaf_sweep<K, W>(c, hist, sw, Ep, m, first_pos, &sg->lim[p], v0, quick_p, Ub, E0, n0, runs1, rstride,
-                                       sg->runn, gl, gsrc, gmask, [&](int next) {
+          task_cnt += leaf_sweep<K, W>(c, hist, sw, Ep, m, first_pos, &sg->lim[p], v0, quick_p, bits, gl, gsrc, gmask,
+                                       [&](int next) {
                                          const unsigned long long before = nodes;
                                          nodes += (unsigned long long)(next - last);
                                          last = next;
@@ -702,11 +723,12 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHis
         }
         if (!found) break;
       }
-      if (use_bits) drop_levels(1);
+      drop_levels(1);
       if (bad) break;
     }
   }
-  if (use_bits) bits_flip_ids<W>(Ub, c.bit_base, E0, n0, false, gl);
+  if constexpr (use_bits)
+    for (int i = gl; i < n0; i += W) bits.clear(__ldg(E0 + i), 0);
   __syncwarp();
   if (c.per_root) {
     const unsigned long long tsum = warp_sum_u64(task_cnt);
