@@ -28,7 +28,7 @@
 // taken by one warp each with a hash table of its own (SMALL_PATHS); the others by a block each
 // with direct 16-bit counters over the ranks below u, cleared in a few 16-byte stores per thread.
 // Measured per call, enumeration before: k = 3 on an R-MAT graph of 98,552 vertices and 1.08M edges
-// 2,981 -> 29 us; k = 4 on a Chung-Lu graph of 18,700 vertices and 198,000 edges 12,994 -> 169 us.
+// 2,981 -> 29 us; k = 4 on a Chung-Lu graph of 18,700 vertices and 198,000 edges 12,994 -> 157 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -402,9 +402,9 @@ __global__ void census_large_kernel(const __grid_constant__ CensusArgs a, int sp
       for (int i = threadIdx.x; i < words; i += blockDim.x) reinterpret_cast<uint4*>(cw)[i] = make_uint4(0u, 0u, 0u, 0u);
       if (threadIdx.x == 0) s_batch = 0;
       __syncthreads();
-      // a warp takes `take` in-neighbours at a time, so that a vertex with few of them still
-      // occupies every warp of the block
-      const int take = max(1, min(32, I / warps));
+      // a warp takes `take` in-neighbours at a time: a vertex with few of them still occupies every
+      // warp of the block, and with many the warps that met long rows take fewer
+      const int take = max(1, min(32, I / (4 * warps)));
       while (true) {
         int i0 = 0;
         if (lane == 0) i0 = atomicAdd(&s_batch, take);
