@@ -405,7 +405,7 @@ int dm_batch_create(const dm_query* queries, int32_t n, const dm_opts* opts, int
     const bool clique = q.kind == DM_QUERY_CLIQUE;
     if (clique) ensure_oriented(g);
     const std::vector<int64_t>& row = clique ? g->orow : g->row;
-    const std::vector<int32_t>& adj = clique ? g->oadj : g->adj;
+    const raw_vector<int32_t>& adj = clique ? g->oadj : g->adj;
     int maxd = 0;
     for (int32_t v = 0; v < g->n; ++v) {
       const int64_t d = row[v + 1] - row[v];

@@ -2,6 +2,8 @@
 #pragma once
 
 #include <cstdint>
+#include <memory>
+#include <new>
 #include <string>
 #include <vector>
 #include <mutex>
@@ -22,6 +24,26 @@ struct Rng {
   double uniform();                  // [0, 1) with 53 random bits
   uint64_t below(uint64_t bound);    // unbiased in [0, bound)
 };
+
+// Vectors whose resize() leaves new elements uninitialised, for arrays that are then written
+// whole: zeroing them first touches every page of a large graph twice.
+template <typename T>
+struct NoInit : std::allocator<T> {
+  template <typename U>
+  struct rebind {
+    using other = NoInit<U>;
+  };
+  template <typename U>
+  void construct(U* p) {
+    ::new (static_cast<void*>(p)) U;
+  }
+  template <typename U, typename... A>
+  void construct(U* p, A&&... a) {
+    ::new (static_cast<void*>(p)) U(static_cast<A&&>(a)...);
+  }
+};
+template <typename T>
+using raw_vector = std::vector<T, NoInit<T>>;
 
 // Device-resident copy of one graph (owned by the graph, one per device). Rows start on
 // 16-byte boundaries (offsets are multiples of 4 ints) and are padded with INT32_MAX so a
@@ -52,27 +74,27 @@ struct dm_graph {
   int32_t max_degree = 0;
   // undirected CSR, rows sorted ascending, no self-loops, no duplicates
   std::vector<int64_t> row;      // n+1
-  std::vector<int32_t> adj;      // 2m
+  dmb::raw_vector<int32_t> adj;  // 2m
   // degree-ordered orientation: rank[v] = position of v in (degree, id) order;
   // out-neighbours of rank r are ranks > r, sorted ascending
   bool oriented_built = false;
   std::vector<int32_t> rank;     // n
   std::vector<int64_t> orow;     // n+1 (rank space)
-  std::vector<int32_t> oadj;     // m
+  dmb::raw_vector<int32_t> oadj; // m
   int32_t max_out_degree = 0;
   // k-independent predictor features per vertex (6 per vertex), for cliques and motifs
   std::vector<float> feat[2];
-  // padded device layout of the CSRs (0: undirected, 1: degree-ordered DAG), built on the
-  // first upload and kept, so uploading the graph again is a plain copy
-  std::vector<int32_t> pad_row[2], pad_deg[2], pad_adj[2];
+  // padded device layout of the undirected CSR, built on the first upload and kept, so uploading
+  // the graph again is a plain copy (the DAG's is part of img)
+  std::vector<int32_t> pad_row, pad_deg;
+  dmb::raw_vector<int32_t> pad_adj;
   // device-independent task orders and clique-index layout, computed once and kept with the
   // graph for the same reason
   std::vector<int32_t> deg_order;     // ranks by descending DAG out-degree (stable in rank)
   std::vector<int64_t> cnt_ge;        // cnt_ge[d] = ranks with out-degree >= d
   std::vector<uint32_t> idx_boff;     // clique-index block offset per rank (16-byte units)
-  std::vector<int32_t> idx_desc;      // task list of deg_order on the index, 4 ints per entry
-                                      // (kept until the clique image holds it)
-  std::vector<uint8_t> img;           // clique image: padded oriented CSR, order, index tables
+  dmb::raw_vector<uint8_t> img;       // clique image: padded oriented CSR, order, index tables
+  bool img_used = false;              // uploaded before (page-locked from the second time on)
   size_t img_off[6] = {0, 0, 0, 0, 0, 0};
   size_t img_adj_ints = 0;            // ints of the padded oriented adjacency
   int32_t idx_extra = 0;              // entries beyond one per root (roots split into parts)

@@ -12,7 +12,9 @@
 #include <atomic>
 #include <chrono>
 #include <climits>
+#include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <numeric>
@@ -401,6 +403,121 @@ void gbuf_free(void* p, int dev) {
   cudaFree(p);
 }
 
+// Page-locked staging for one-off transfers of pageable host memory (a graph's first upload, a
+// file being read, results going into fresh vectors): pieces of STAGE_BYTES go through two
+// buffers, so the host copies one piece while the other one is on the bus. Registering the
+// caller's memory instead costs more than one transfer gains. The buffers are pooled per device
+// (at most STAGE_POOL pairs are kept).
+constexpr size_t STAGE_BYTES = (size_t)4 << 20;
+constexpr size_t STAGE_POOL = 4;
+static std::mutex g_stage_mu;
+static std::map<int, std::vector<Staging>> g_stage_pool;
+
+Stager::Stager(int device, cudaStream_t st) : dev_(device), st_(st) {
+  {
+    std::lock_guard<std::mutex> lk(g_stage_mu);
+    auto& pool = g_stage_pool[dev_];
+    if (!pool.empty()) {
+      s_ = pool.back();
+      pool.pop_back();
+      return;
+    }
+  }
+  for (int i = 0; i < 2; ++i) {
+    // without page-locked memory the pieces are plain pageable copies
+    if (s_.pinned && cudaMallocHost(&s_.buf[i], STAGE_BYTES) != cudaSuccess) {
+      cudaGetLastError();
+      if (i == 1) cudaFreeHost(s_.buf[0]);
+      s_.pinned = false;
+      i = 0;
+    }
+    if (!s_.pinned && !(s_.buf[i] = std::malloc(STAGE_BYTES))) err_ = cudaErrorMemoryAllocation;
+  }
+  for (int i = 0; i < 2 && err_ == cudaSuccess; ++i) err_ = cudaEventCreateWithFlags(&s_.ev[i], cudaEventDisableTiming);
+}
+
+Stager::~Stager() {
+  if (err_ == cudaSuccess && s_.pinned) {
+    // (copies still on the bus are waited for by whoever fills that buffer next)
+    std::lock_guard<std::mutex> lk(g_stage_mu);
+    auto& pool = g_stage_pool[dev_];
+    if (pool.size() < STAGE_POOL) {
+      pool.push_back(s_);
+      return;
+    }
+  }
+  for (int i = 0; i < 2; ++i) {
+    if (s_.busy[i]) cudaEventSynchronize(s_.ev[i]);
+    if (s_.ev[i]) cudaEventDestroy(s_.ev[i]);
+    if (s_.pinned) cudaFreeHost(s_.buf[i]);
+    else std::free(s_.buf[i]);
+  }
+  cudaGetLastError();
+}
+
+cudaError_t Stager::wait(int i) {
+  if (err_ == cudaSuccess && s_.busy[i]) err_ = cudaEventSynchronize(s_.ev[i]);
+  s_.busy[i] = false;
+  return err_;
+}
+
+cudaError_t Stager::sent(int i) {
+  if (err_ == cudaSuccess) err_ = cudaEventRecord(s_.ev[i], st_);
+  s_.busy[i] = err_ == cudaSuccess;
+  return err_;
+}
+
+cudaError_t Stager::upload(void* dst, size_t bytes, const std::function<size_t(void*, size_t)>& fill, size_t* got) {
+  size_t off = 0;
+  while (off < bytes && err_ == cudaSuccess) {
+    const int i = next_;
+    next_ ^= 1;
+    if (wait(i) != cudaSuccess) break;
+    const size_t want = std::min(STAGE_BYTES, bytes - off);
+    const size_t n = fill(s_.buf[i], want);
+    if (n) {
+      err_ = cudaMemcpyAsync(static_cast<char*>(dst) + off, s_.buf[i], n, cudaMemcpyHostToDevice, st_);
+      sent(i);
+      off += n;
+    }
+    if (n < want) break;
+  }
+  if (got) *got = off;
+  return err_;
+}
+
+cudaError_t Stager::upload(void* dst, const void* src, size_t bytes) {
+  const char* p = static_cast<const char*>(src);
+  return upload(dst, bytes, [&](void* buf, size_t n) {
+    std::memcpy(buf, p, n);
+    p += n;
+    return n;
+  }, nullptr);
+}
+
+cudaError_t Stager::download(void* dst, const void* src, size_t bytes) {
+  size_t off = 0, held[2] = {0, 0}, at[2] = {0, 0};
+  auto drain = [&](int i) {
+    if (held[i] && wait(i) == cudaSuccess) std::memcpy(static_cast<char*>(dst) + at[i], s_.buf[i], held[i]);
+    held[i] = 0;
+  };
+  while (off < bytes && err_ == cudaSuccess) {
+    const int i = next_;
+    next_ ^= 1;
+    drain(i);
+    if (wait(i) != cudaSuccess) break;
+    const size_t n = std::min(STAGE_BYTES, bytes - off);
+    err_ = cudaMemcpyAsync(s_.buf[i], static_cast<const char*>(src) + off, n, cudaMemcpyDeviceToHost, st_);
+    sent(i);
+    held[i] = n;
+    at[i] = off;
+    off += n;
+  }
+  drain(next_);
+  drain(next_ ^ 1);
+  return err_;
+}
+
 // Registers a host array of the graph with the driver once (page-locked), so uploads from it
 // are asynchronous DMA; the arrays are never resized afterwards and are unregistered when the
 // graph is freed.
@@ -419,37 +536,46 @@ void unpin_host_arrays(dm_graph* g) {
   cudaGetLastError();
 }
 
-// Pads rows to multiples of 4 ints (16 bytes) filled with INT32_MAX; the padded layout is
-// built on the first upload of a graph and kept (page-locked) with it.
-static int host_pad_csr(const std::vector<int64_t>& row, const std::vector<int32_t>& adj, int32_t n,
-                        std::vector<int32_t>& prow, std::vector<int32_t>& pdeg, std::vector<int32_t>& padj) {
+// Rows padded to multiples of 4 ints (16 bytes): starts and degrees into prow / pdeg (n entries),
+// the padded total returned (-1: beyond 32-bit offsets).
+static int64_t padded_rows(const std::vector<int64_t>& row, int32_t n, int32_t* prow, int32_t* pdeg) {
+  int64_t total = 0;
+  for (int32_t v = 0; v < n; ++v) {
+    const int64_t d = row[v + 1] - row[v];
+    prow[v] = (int32_t)total;
+    pdeg[v] = (int32_t)d;
+    total += (d + 3) & ~3ll;
+    if (total >= INT32_MAX) return -1;
+  }
+  return std::max<int64_t>(total, 4);
+}
+
+// The padded rows themselves, filled up with INT32_MAX.
+static void padded_adj(const std::vector<int64_t>& row, const raw_vector<int32_t>& adj, int32_t n, int64_t total,
+                       int32_t* padj) {
+  int64_t at = 0;
+  for (int32_t v = 0; v < n; ++v) {
+    const int64_t d = row[v + 1] - row[v];
+    std::copy(adj.data() + row[v], adj.data() + row[v + 1], padj + at);
+    at += d;
+    while (at & 3) padj[at++] = INT32_MAX;
+  }
+  while (at < total) padj[at++] = INT32_MAX;
+}
+
+// Device copy of the undirected CSR in the padded layout, built on the first upload of a graph and
+// kept (page-locked) with it.
+static int upload_csr(dm_graph* g, int32_t** d_row, int32_t** d_deg, int32_t** d_adj, cudaStream_t st) {
+  const int32_t n = g->n;
+  auto &prow = g->pad_row, &pdeg = g->pad_deg;
+  auto& padj = g->pad_adj;
   if (padj.empty()) {
     prow.assign(n, 0);
     pdeg.assign(n, 0);
-    int64_t total = 0;
-    for (int32_t v = 0; v < n; ++v) {
-      int64_t d = row[v + 1] - row[v];
-      prow[v] = (int32_t)total;
-      pdeg[v] = (int32_t)d;
-      total += (d + 3) & ~3ll;
-      if (total >= INT32_MAX) {
-        prow.clear();
-        pdeg.clear();
-        return fail(DM_EOVERFLOW, "padded adjacency exceeds 32-bit offsets");
-      }
-    }
-    padj.assign((size_t)std::max<int64_t>(total, 4), INT32_MAX);
-    for (int32_t v = 0; v < n; ++v) std::memcpy(padj.data() + prow[v], adj.data() + row[v], sizeof(int32_t) * pdeg[v]);
-  }
-  return DM_OK;
-}
-
-static int upload_csr(dm_graph* g, const std::vector<int64_t>& row, const std::vector<int32_t>& adj, int32_t n,
-                      std::vector<int32_t>& prow, std::vector<int32_t>& pdeg, std::vector<int32_t>& padj,
-                      int32_t** d_row, int32_t** d_deg, int32_t** d_adj, cudaStream_t st) {
-  if (padj.empty()) {
-    int rc = host_pad_csr(row, adj, n, prow, pdeg, padj);
-    if (rc) return rc;
+    const int64_t total = padded_rows(g->row, n, prow.data(), pdeg.data());
+    if (total < 0) return fail(DM_EOVERFLOW, "padded adjacency exceeds 32-bit offsets");
+    padj.resize((size_t)total);
+    padded_adj(g->row, g->adj, n, total, padj.data());
     pin_host(g, prow.data(), sizeof(int32_t) * prow.size());
     pin_host(g, pdeg.data(), sizeof(int32_t) * pdeg.size());
     pin_host(g, padj.data(), sizeof(int32_t) * padj.size());
@@ -666,60 +792,54 @@ static void host_index_tables(dm_graph* g) {
     g->idx_boff.swap(boff);
     g->idx_units = total;
     g->idx_maxd = max_d;
-    // roots of 32 or more out-neighbours enter the list as split_parts(d) entries, each for
-    // an even share of the root's items: the warps dealt those entries start on the heaviest
-    // roots together instead of one warp walking each of them alone
-    g->idx_desc.clear();
-    g->idx_desc.reserve((size_t)4 * n);
-    for (int32_t i = 0; i < n; ++i) {
-      const int32_t r = g->deg_order[i];
-      const int P = split_parts((int)(g->orow[r + 1] - g->orow[r]));
-      for (int q = 0; q < P; ++q) {
-        const RootDesc rd = root_desc(g, nullptr, r, P > 1 ? (q | (P << 16)) : 0);
-        const int32_t* w = reinterpret_cast<const int32_t*>(&rd);
-        g->idx_desc.insert(g->idx_desc.end(), w, w + 4);
-      }
-    }
-    g->idx_extra = (int32_t)(g->idx_desc.size() / 4 - (size_t)n);
+    // (roots of 20 to 64 out-neighbours enter the task list as split_parts(d) entries)
+    int64_t extra = 0;
+    for (int32_t r = 0; r < n; ++r) extra += split_parts((int)(g->orow[r + 1] - g->orow[r])) - 1;
+    g->idx_extra = (int32_t)extra;
   }
 }
 
-// The clique path's host arrays in one page-locked image, so that a device copy of the graph
-// is one host-to-device copy: the padded oriented CSR (row starts, degrees, rows), the
-// descending-degree order, the index block offsets and the plain task list, each starting
-// on 256 bytes. Built once per graph; the separate padded CSR and task list are dropped.
+// The clique path's host arrays in one image, so that a device copy of the graph is one
+// host-to-device copy: the padded oriented CSR (row starts, degrees, rows), the descending-degree
+// order, the index block offsets and the plain task list, each starting on 256 bytes and written
+// in place, once per graph.
 // (One copy of the 1.57 MB of chunglu18k took 38 µs, seven copies of its parts 67 µs.)
 static int host_clique_image(dm_graph* g) {
   if (!g->img.empty()) return DM_OK;
-  int rc = host_pad_csr(g->orow, g->oadj, g->n, g->pad_row[1], g->pad_deg[1], g->pad_adj[1]);
-  if (rc) return rc;
   host_deg_order(g);
   host_index_tables(g);
-  const size_t n = (size_t)std::max(g->n, 1);
-  const size_t sizes[6] = {4 * n, 4 * n, 4 * g->pad_adj[1].size(), 4 * n, 4 * n,
-                           std::max<size_t>(4 * g->idx_desc.size(), 16)};
+  const int32_t nn = g->n;
+  const size_t n = (size_t)std::max(nn, 1);
+  int64_t total = 0;
+  for (int32_t v = 0; v < nn; ++v) total += (g->orow[v + 1] - g->orow[v] + 3) & ~3ll;
+  if (total >= INT32_MAX) return fail(DM_EOVERFLOW, "padded adjacency exceeds 32-bit offsets");
+  total = std::max<int64_t>(total, 4);
+  const size_t entries = (size_t)nn + (size_t)g->idx_extra;
+  const size_t sizes[6] = {4 * n, 4 * n, 4 * (size_t)total, 4 * n, 4 * n, std::max<size_t>(sizeof(RootDesc) * entries, 16)};
   size_t off = 0;
   for (int i = 0; i < 6; ++i) {
     g->img_off[i] = off;
     off += (sizes[i] + 255) / 256 * 256;
   }
-  std::vector<uint8_t> img(off, 0);
-  const int32_t nn = g->n;
+  raw_vector<uint8_t> img(off);
+  auto part = [&](int i) { return reinterpret_cast<int32_t*>(img.data() + g->img_off[i]); };
+  padded_rows(g->orow, nn, part(0), part(1));
+  padded_adj(g->orow, g->oadj, nn, total, part(2));
   if (nn) {
-    std::memcpy(img.data() + g->img_off[0], g->pad_row[1].data(), 4 * (size_t)nn);
-    std::memcpy(img.data() + g->img_off[1], g->pad_deg[1].data(), 4 * (size_t)nn);
-    std::memcpy(img.data() + g->img_off[3], g->deg_order.data(), 4 * (size_t)nn);
-    std::memcpy(img.data() + g->img_off[4], g->idx_boff.data(), 4 * (size_t)nn);
+    std::memcpy(part(3), g->deg_order.data(), 4 * (size_t)nn);
+    std::memcpy(part(4), g->idx_boff.data(), 4 * (size_t)nn);
   }
-  std::memcpy(img.data() + g->img_off[2], g->pad_adj[1].data(), 4 * g->pad_adj[1].size());
-  if (!g->idx_desc.empty()) std::memcpy(img.data() + g->img_off[5], g->idx_desc.data(), 4 * g->idx_desc.size());
-  g->img_adj_ints = g->pad_adj[1].size();
+  // roots of 20 to 64 out-neighbours enter the list as split_parts(d) entries, each for an even
+  // share of the root's items: the warps dealt those entries start on the heaviest roots
+  // together instead of one warp walking each of them alone
+  RootDesc* desc = reinterpret_cast<RootDesc*>(part(5));
+  for (int32_t i = 0; i < nn; ++i) {
+    const int32_t r = g->deg_order[i];
+    const int P = split_parts((int)(g->orow[r + 1] - g->orow[r]));
+    for (int q = 0; q < P; ++q) *desc++ = root_desc(g, nullptr, r, P > 1 ? (q | (P << 16)) : 0);
+  }
+  g->img_adj_ints = (size_t)total;
   g->img.swap(img);
-  pin_host(g, g->img.data(), g->img.size());
-  std::vector<int32_t>().swap(g->pad_row[1]);
-  std::vector<int32_t>().swap(g->pad_deg[1]);
-  std::vector<int32_t>().swap(g->pad_adj[1]);
-  std::vector<int32_t>().swap(g->idx_desc);
   return DM_OK;
 }
 
@@ -730,7 +850,15 @@ static int upload_clique_image(dm_graph* g, DeviceSlot* s, cudaStream_t st) {
   if (rc) return rc;
   void* base = nullptr;
   cudaError_t e = gbuf_alloc(&base, g->img.size());
-  if (e == cudaSuccess) e = cudaMemcpyAsync(base, g->img.data(), g->img.size(), cudaMemcpyHostToDevice, st);
+  // the first copy goes through the staging buffers; a graph uploaded again is page-locked (once)
+  if (e == cudaSuccess && !g->img_used) {
+    Stager stager(s->dg.device, st);
+    e = stager.upload(base, g->img.data(), g->img.size());
+    g->img_used = true;
+  } else if (e == cudaSuccess) {
+    pin_host(g, g->img.data(), g->img.size());
+    e = cudaMemcpyAsync(base, g->img.data(), g->img.size(), cudaMemcpyHostToDevice, st);
+  }
   if (e != cudaSuccess) {
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1464,8 +1592,7 @@ int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_
   if ((rc = prepare_ws(ws, ctx.stream))) return rc;
   DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
   if (!s->dg.has_undirected) {
-    rc = upload_csr(g, g->row, g->adj, g->n, g->pad_row[0], g->pad_deg[0], g->pad_adj[0], &s->dg.d_row,
-                    &s->dg.d_deg, &s->dg.d_adj, ctx.stream);
+    rc = upload_csr(g, &s->dg.d_row, &s->dg.d_deg, &s->dg.d_adj, ctx.stream);
     if (rc) return rc;
     s->dg.has_undirected = true;
   }
@@ -1605,7 +1732,7 @@ int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_
   L.bit_words = bit_words;
   L2Window l2;
   if (o && (o->flags & DM_FLAG_L2_PERSIST) &&
-      (rc = l2.begin(ctx.device, ctx.stream, s->dg.d_adj, sizeof(int32_t) * g->pad_adj[0].size())))
+      (rc = l2.begin(ctx.device, ctx.stream, s->dg.d_adj, sizeof(int32_t) * g->pad_adj.size())))
     return rc;
   DM_CUDA(cudaEventRecord(ws.k0, ctx.stream));
   int grid = 0;

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <functional>
 #include <vector>
 
 #include "dm_internal.hpp"
@@ -276,6 +277,35 @@ int check_opts(const dm_opts* o);
 // buffer is given back only once nothing on the device uses it any more.
 cudaError_t gbuf_alloc(void** p, size_t bytes);
 void gbuf_free(void* p, int dev);
+// Transfers of pageable host memory through pooled page-locked buffers (engine.cu), on `st`.
+struct Staging {
+  void* buf[2] = {nullptr, nullptr};
+  cudaEvent_t ev[2] = {nullptr, nullptr};  // the last copy from or into the buffer
+  bool busy[2] = {false, false};
+  bool pinned = true;
+};
+class Stager {
+ public:
+  Stager(int device, cudaStream_t st);
+  ~Stager();
+  Stager(const Stager&) = delete;
+  Stager& operator=(const Stager&) = delete;
+  // The source may change as soon as the call returns; the destination is written in stream order.
+  cudaError_t upload(void* dst, const void* src, size_t bytes);
+  // fill(buf, n) writes up to n bytes and returns how many (fewer end the upload); *got: the total
+  cudaError_t upload(void* dst, size_t bytes, const std::function<size_t(void*, size_t)>& fill, size_t* got);
+  // The destination is complete when the call returns.
+  cudaError_t download(void* dst, const void* src, size_t bytes);
+
+ private:
+  cudaError_t wait(int i);
+  cudaError_t sent(int i);
+  int dev_;
+  cudaStream_t st_;
+  Staging s_;
+  int next_ = 0;
+  cudaError_t err_ = cudaSuccess;
+};
 int queue_init_launch(void* queue, int nq, int cap, cudaStream_t st);  // empty donation queue
 constexpr int QUEUE_SHARDS = 64;        // donation-queue shards of a workspace
 constexpr int QUEUE_SHARD_SLOTS = 2048; // slots per shard

@@ -159,24 +159,29 @@ void ensure_oriented(dm_graph* g) {
   }
   g->rank.assign(n, 0);
   for (int32_t r = 0; r < n; ++r) g->rank[order[r]] = r;
+  // one pass over the neighbours for the out-degrees, and one over the targets in ascending rank:
+  // every out-list is filled in order, so nothing is sorted
   g->orow.assign((size_t)n + 1, 0);
+  const int32_t* rank = g->rank.data();
   for (int32_t v = 0; v < n; ++v) {
-    int32_t rv = g->rank[v];
-    for (int64_t e = g->row[v]; e < g->row[v + 1]; ++e)
-      if (g->rank[g->adj[e]] > rv) g->orow[rv + 1]++;
+    const int32_t rv = rank[v];
+    int64_t d = 0;
+    for (int64_t e = g->row[v]; e < g->row[v + 1]; ++e) d += rank[g->adj[e]] > rv;
+    g->orow[rv + 1] = d;
   }
-  for (int32_t r = 0; r < n; ++r) g->orow[r + 1] += g->orow[r];
-  g->oadj.resize((size_t)g->m);
   int32_t mo = 0;
   for (int32_t r = 0; r < n; ++r) {
-    int32_t v = order[r];
-    int64_t pos = g->orow[r];
+    mo = std::max<int32_t>(mo, (int32_t)g->orow[r + 1]);
+    g->orow[r + 1] += g->orow[r];
+  }
+  g->oadj.resize((size_t)g->m);
+  std::vector<int64_t> pos(g->orow.begin(), g->orow.end() - 1);
+  for (int32_t r = 0; r < n; ++r) {
+    const int32_t v = order[r];
     for (int64_t e = g->row[v]; e < g->row[v + 1]; ++e) {
-      int32_t ru = g->rank[g->adj[e]];
-      if (ru > r) g->oadj[pos++] = ru;
+      const int32_t ru = rank[g->adj[e]];
+      if (ru < r) g->oadj[pos[ru]++] = r;
     }
-    std::sort(g->oadj.begin() + g->orow[r], g->oadj.begin() + g->orow[r + 1]);
-    mo = std::max<int32_t>(mo, (int32_t)(g->orow[r + 1] - g->orow[r]));
   }
   g->max_out_degree = mo;
   g->oriented_built = true;

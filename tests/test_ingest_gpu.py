@@ -72,3 +72,23 @@ def test_device_ingest_empty_file(dm, gpu, tmp_path):
     path.write_text("")
     g, _ = dm.Graph.load_edgelist_device(path)
     assert g.info().n_vertices == 0 and g.info().n_edges == 0
+
+
+@pytest.mark.parametrize("size", [(4 << 20) - 1, 4 << 20, (4 << 20) + 1, (8 << 20) + 3])
+def test_device_ingest_staging_edges(dm, gpu, tmp_path, size):
+    """Files that end just before, at and after a 4 MiB staging piece, with a token across it."""
+    rng = np.random.default_rng(size)
+    head = "\n".join(f"{a} {b}" for a, b in rng.integers(0, 70_000, (30_000, 2))) + "\n"
+    cut = min(size - 40, (4 << 20) - 3)
+    text = head + " " * (cut - len(head)) + "123456 654321\n"  # straddles the first piece's end
+    text += "9 10\n" * max(0, (size - len(text)) // 5)
+    text += "\n" * (size - len(text))
+    assert len(text) == size
+    path = tmp_path / "edge.edgelist"
+    path.write_text(text)
+    g, _ = dm.Graph.load_edgelist_device(path)
+    h = dm.Graph.load_edgelist(path)
+    _same_graph(dm, g, h)
+    for _ in range(2):  # staged first upload, then the page-locked one
+        assert dm.count_cliques(g, 3)[0] == dm.count_cliques(h, 3)[0]
+        g.release_device()
