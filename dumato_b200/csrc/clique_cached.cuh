@@ -278,6 +278,130 @@ __device__ __forceinline__ unsigned long long heavy_run(const CachedArgs& a, con
   return heavy_walk<K, NW, MULTI>(a, tw, rows, S, root, it, lo, hi, eager, acc, cs);
 }
 
+// Sum over the members y of T of |T & row[y]| (rows hold only members above their own): the edges
+// inside T. The words of T are taken as a queue, so the loop body is the same for every member.
+template <int NW>
+__device__ __forceinline__ unsigned edges_inside(const Bits<NW>& T, const uint64_t* rows) {
+  unsigned sum = 0;
+  Bits<NW> left = T;
+  int base = 0;
+  while (true) {
+#pragma unroll
+    for (int h = 0; h + 1 < NW; ++h) {
+      if (left.w[0] == 0ull && base + 64 < 64 * NW) {
+#pragma unroll
+        for (int w = 0; w + 1 < NW; ++w) left.w[w] = left.w[w + 1];
+        left.w[NW - 1] = 0ull;
+        base += 64;
+      }
+    }
+    if (left.w[0] == 0ull) break;
+    const int y = base + __ffsll((long long)left.w[0]) - 1;
+    left.w[0] &= left.w[0] - 1ull;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) sum += (unsigned)__popcll(T.w[w] & rows[y * NW + w]);
+  }
+  return sum;
+}
+
+// 5- and 6-cliques of a wide root (rows of two or more words), items [tw.range) of its local
+// edges (c1, c2). With S = row[c1] & row[c2], a 5-clique is an edge inside S, a 6-clique an edge
+// inside T = S & row[c3] for a member c3 of S. Lanes take 32 items together; for k = 6 the (item,
+// c3) pairs of the 32 sets are laid end to end over the lanes through the prefix of their sizes,
+// and each lane counts the edges inside its T in a loop of its own.
+//
+// The lockstep walk pays about 100 instructions of stack, counters and selects for every node,
+// and at these sizes (out-degrees to 171, 4.5e8 of 5.2e8 nodes of the k = 6 walk at its last level
+// on an R-MAT graph of 98,552 vertices) nearly all nodes are last ones, whose whole work is one AND
+// and popcount per word: 6-cliques of that graph took 6.8 ms per call, now 3.6. Rows of one word stay with the walk: their sets are too
+// small to fill a loop.
+template <int K, int NW>
+__device__ __forceinline__ unsigned long long wide_run(const CachedArgs& a, const TaskWords& tw, const uint64_t* rows,
+                                                       const int32_t* sE, int root, int d, bool eager, CheckState& cs) {
+  const int lane = lane_id();
+  const LBArgs& lb = a.c.lb;
+  const long long t_start = lane == 0 ? clock64() : 0;
+  const int need = lb.min_split > 2 ? lb.min_split : 2;
+  int xb = 0, xe = 0;  // lane 0: split-off items that no queue slot took
+  unsigned long long cnt = 0;
+  uint64_t* sets = tw.stk;  // k = 6: the 32 items' sets, [word][lane]
+  while (true) {
+    unsigned long long old = 0ull;
+    if (lane == 0) old = atomicAdd(tw.range, 32ull);
+    old = __shfl_sync(FULL_MASK, old, 0);
+    const int next = (int)(unsigned)old, end = (int)(unsigned)(old >> 32);
+    if (next >= end) {
+      const int b0 = __shfl_sync(FULL_MASK, xb, 0), e0 = __shfl_sync(FULL_MASK, xe, 0);
+      if (e0 <= b0) break;
+      if (lane == 0) {
+        *tw.range = pack_range(b0, e0);
+        xb = xe = 0;
+      }
+      __syncwarp();
+      continue;
+    }
+    const int it = next + lane;
+    Bits<NW> S;
+    int p = 0;
+    if (it < end) {
+      const int c1 = lower_bound_bl<(NW == 2 ? 128 : 256)>(sE, d + 1, it + 1) - 1;
+      const int c2 = select_row<NW>(rows + c1 * NW, it - sE[c1]);
+#pragma unroll
+      for (int w = 0; w < NW; ++w) S.w[w] = rows[c1 * NW + w] & rows[c2 * NW + w];
+      p = popc(S);
+    }
+    if constexpr (K == 5) {
+      if (p >= 2) cnt += edges_inside<NW>(S, rows);
+    } else {
+      if (p < 3) p = 0;  // (three more vertices are needed)
+#pragma unroll
+      for (int w = 0; w < NW; ++w) sets[w * 32 + lane] = S.w[w];
+      int off = p;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(FULL_MASK, off, o);
+        if (lane >= o) off += y;
+      }
+      const int total = __shfl_sync(FULL_MASK, off, 31);
+      off -= p;
+      __syncwarp();
+      for (int f0 = 0; f0 < total; f0 += 32) {
+        const int f = f0 + lane;
+        int j = 0;  // owner: the last item whose pairs start at or before f
+#pragma unroll
+        for (int h = 16; h >= 1; h >>= 1) {
+          const int o = __shfl_sync(FULL_MASK, off, j + h);
+          j = o <= f ? j + h : j;
+        }
+        const int pos = f - __shfl_sync(FULL_MASK, off, j);
+        if (f < total) {
+          uint64_t own[NW];
+#pragma unroll
+          for (int w = 0; w < NW; ++w) own[w] = sets[w * 32 + j];
+          const int c3 = select_row<NW>(own, pos);
+          Bits<NW> T;
+#pragma unroll
+          for (int w = 0; w < NW; ++w) T.w[w] = own[w] & rows[c3 * NW + w];
+          cnt += edges_inside<NW>(T, rows);
+        }
+      }
+      __syncwarp();
+    }
+    if (lane == 0) {
+      atomicAdd(&lb.ctr->progress, 32ull);
+      if (lb.hungry_trigger > 0) {
+        if (next + 32 < end)
+          lockstep_donate(lb, tw, cs, end - next - 32, need, root, t_start, 0, 0, 0, nullptr, eager, xb, xe);
+        cs.hungry = vload(&lb.ctr->hungry);  // read after the next items: never waited for
+        cs.queued = vload(&lb.ctr->queued);
+      }
+    }
+    __syncwarp();
+  }
+  __syncwarp();
+  return cnt;
+}
+
 // Counts one root's task from its staged rows: level 0 runs items [b, e) (task_range
 // encoding; items are the local edges, or the rows when k == 3), level 1 runs positions
 // [b, e) of item `it`'s candidate set. Returns this lane's share.
@@ -349,6 +473,8 @@ __device__ __forceinline__ unsigned long long staged_run(const CachedArgs& a, co
     }
     __syncwarp();
     return cnt;
+  } else if constexpr (!MULTI && NW >= 2 && (K == 5 || K == 6)) {
+    return wide_run<K, NW>(a, tw, rows, sE, root, d, eager, cs);
   } else {
     WalkR<K, NW, MULTI, 4> wk;
     wk.stk = tw.stk;
