@@ -306,14 +306,15 @@ __device__ __forceinline__ unsigned edges_inside(const Bits<NW>& T, const uint64
 
 // 5- and 6-cliques of a wide root (rows of two or more words), items [tw.range) of its local
 // edges (c1, c2). With S = row[c1] & row[c2], a 5-clique is an edge inside S, a 6-clique an edge
-// inside T = S & row[c3] for a member c3 of S. Lanes take 32 items together; for k = 6 the (item,
-// c3) pairs of the 32 sets are laid end to end over the lanes through the prefix of their sizes,
+// inside T = S & row[c3] for a member c3 of S. A warp takes TAKE items together; for k = 6 the (item,
+// c3) pairs of their sets are laid end to end over the lanes through the prefix of their sizes,
 // and each lane counts the edges inside its T in a loop of its own.
 //
 // The lockstep walk pays about 100 instructions of stack, counters and selects for every node,
 // and at these sizes (out-degrees to 171, 4.5e8 of 5.2e8 nodes of the k = 6 walk at its last level
 // on an R-MAT graph of 98,552 vertices) nearly all nodes are last ones, whose whole work is one AND
-// and popcount per word: 6-cliques of that graph took 6.8 ms per call, now 3.6. Rows of one word stay with the walk: their sets are too
+// and popcount per word: 6-cliques of that graph took 6.8 ms per call, now 3.3 (3.6 with 32 items
+// at a time, 0.32 instead of 0.14 of the warp time idle). Rows of one word stay with the walk: their sets are too
 // small to fill a loop.
 template <int K, int NW>
 __device__ __forceinline__ unsigned long long wide_run(const CachedArgs& a, const TaskWords& tw, const uint64_t* rows,
@@ -321,13 +322,16 @@ __device__ __forceinline__ unsigned long long wide_run(const CachedArgs& a, cons
   const int lane = lane_id();
   const LBArgs& lb = a.c.lb;
   const long long t_start = lane == 0 ? clock64() : 0;
-  const int need = lb.min_split > 2 ? lb.min_split : 2;
+  // items taken together: a 6-clique item holds some hundred pairs at these sizes, so few of them
+  // fill the lanes, and ranges stay divisible for idle warps almost to their end
+  constexpr int TAKE = K == 6 ? 8 : 32;
+  constexpr int need = TAKE;
   int xb = 0, xe = 0;  // lane 0: split-off items that no queue slot took
   unsigned long long cnt = 0;
-  uint64_t* sets = tw.stk;  // k = 6: the 32 items' sets, [word][lane]
+  uint64_t* sets = tw.stk;  // k = 6: the items' sets, [word][lane]
   while (true) {
     unsigned long long old = 0ull;
-    if (lane == 0) old = atomicAdd(tw.range, 32ull);
+    if (lane == 0) old = atomicAdd(tw.range, (unsigned long long)TAKE);
     old = __shfl_sync(FULL_MASK, old, 0);
     const int next = (int)(unsigned)old, end = (int)(unsigned)(old >> 32);
     if (next >= end) {
@@ -343,7 +347,7 @@ __device__ __forceinline__ unsigned long long wide_run(const CachedArgs& a, cons
     const int it = next + lane;
     Bits<NW> S;
     int p = 0;
-    if (it < end) {
+    if (lane < TAKE && it < end) {
       const int c1 = lower_bound_bl<(NW == 2 ? 128 : 256)>(sE, d + 1, it + 1) - 1;
       const int c2 = select_row<NW>(rows + c1 * NW, it - sE[c1]);
 #pragma unroll
@@ -388,10 +392,10 @@ __device__ __forceinline__ unsigned long long wide_run(const CachedArgs& a, cons
       __syncwarp();
     }
     if (lane == 0) {
-      atomicAdd(&lb.ctr->progress, 32ull);
+      atomicAdd(&lb.ctr->progress, (unsigned long long)TAKE);
       if (lb.hungry_trigger > 0) {
-        if (next + 32 < end)
-          lockstep_donate(lb, tw, cs, end - next - 32, need, root, t_start, 0, 0, 0, nullptr, eager, xb, xe);
+        if (next + TAKE < end)
+          lockstep_donate(lb, tw, cs, end - next - TAKE, need, root, t_start, 0, need, 0, nullptr, eager, xb, xe);
         cs.hungry = vload(&lb.ctr->hungry);  // read after the next items: never waited for
         cs.queued = vload(&lb.ctr->queued);
       }
