@@ -207,13 +207,12 @@ __global__ void adam_kernel(float* __restrict__ P, const float* __restrict__ g, 
 // A step is a chain of small dependent pieces, bound by latency: with three launches per step
 // (clear, backward, Adam) the launches and one thread per sample took about 29 us per step of 256
 // samples; four epochs over the subtree log of a graph of 18,700 vertices and a count scheduled
-// with the result took 9.29 ms, now 1.88 ms. Batches above EP_BATCH_MAX (16 tiles per step) keep
-// those launches, which use every SM.
-constexpr int EP_CTAS = 8, EP_THREADS = 256, EP_TILE = 32;  // samples per block and tile
-constexpr int EP_SLICE = (MLP_NP + EP_CTAS - 1) / EP_CTAS;
+// with the result took 9.29 ms, with a cluster of 8 blocks 1.88 ms and of 16 about 1.6 ms (a step is
+// then 4.5 us). Batches above EP_BATCH_MAX keep those launches, which use every SM.
+constexpr int EP_THREADS = 256, EP_TILE = 32;  // samples per block and tile
 constexpr int EP_LD = MLP_H + 4;                            // padded row of 32 floats (16-byte rows)
 constexpr int EP_BATCH_MAX = 4096;
-static_assert(EP_SLICE <= EP_THREADS && EP_TILE * MLP_F == EP_THREADS, "thread maps of the epoch kernel");
+static_assert((MLP_NP + 7) / 8 <= EP_THREADS && EP_TILE * MLP_F == EP_THREADS, "thread maps of the epoch kernel");
 
 struct EpochArgs {
   float* P;
@@ -229,6 +228,7 @@ struct EpochArgs {
 };
 
 // Tile t0 of the minibatch starting at `off`.
+template <int EP_CTAS>
 struct EpochTile {
   int off, t0;
   __device__ __forceinline__ int size(const EpochArgs& a) const { return min(a.batch, a.n - off); }
@@ -248,8 +248,10 @@ struct EpochTile {
   }
 };
 
+template <int EP_CTAS>
 __global__ void __cluster_dims__(EP_CTAS, 1, 1) __launch_bounds__(EP_THREADS) mlp_epoch_kernel(const __grid_constant__ EpochArgs a) {
   namespace cg = cooperative_groups;
+  constexpr int EP_SLICE = (MLP_NP + EP_CTAS - 1) / EP_CTAS;
   cg::cluster_group cl = cg::this_cluster();
   const int cta = (int)cl.block_rank(), t = threadIdx.x;
   __shared__ __align__(16) float W1[MLP_H * MLP_F], W2[MLP_H * EP_LD];
@@ -280,7 +282,7 @@ __global__ void __cluster_dims__(EP_CTAS, 1, 1) __launch_bounds__(EP_THREADS) ml
   const int hi = t >> 4, lo = t & 15;    // 2 x 2 tiles: rows hi, hi + 16, columns lo, lo + 16
   float gw2[4], gw1, gb;                 // the batch's gradients this thread holds
   float loss = 0.f;
-  EpochTile cur{0, 0}, nxt{0, 0};
+  EpochTile<EP_CTAS> cur{0, 0}, nxt{0, 0};
   // samples of the first tile, and the indices of the second
   int at = cur.place(a, cta, s8);
   int sidx = at >= 0 ? a.idx[at] : -1;
@@ -449,6 +451,32 @@ __global__ void __cluster_dims__(EP_CTAS, 1, 1) __launch_bounds__(EP_THREADS) ml
   }
   for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
   if ((t & 31) == 0 && loss != 0.f) atomicAdd(a.loss_sum, loss);
+}
+
+// Blocks of the epoch kernel's cluster: 16 (beyond the portable eight, half a tile each at 256
+// samples) where the device can place them, else 8.
+static int epoch_ctas(int dev) {
+  static std::atomic<int> known[LAUNCH_CACHE_DEVICES];
+  int c = dev >= 0 && dev < LAUNCH_CACHE_DEVICES ? known[dev].load() : 0;
+  if (c) return c;
+  c = 8;
+  auto kern = mlp_epoch_kernel<16>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    cfg.gridDim = 16;
+    cfg.blockDim = EP_THREADS;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 16;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n >= 1) c = 16;
+  }
+  cudaGetLastError();
+  if (dev >= 0 && dev < LAUNCH_CACHE_DEVICES) known[dev].store(c);
+  return c;
 }
 
 static int pred_device(int* dev) {
@@ -934,6 +962,7 @@ int dm_predictor_train(dm_predictor* p, const float* X, const float* T, int64_t 
   if (rc) return rc;
   // one buffer from the library's pool: P, M, V, gradient, loss | X | T | two index buffers | bias
   const bool fused = batch <= EP_BATCH_MAX;
+  const int ctas = fused ? epoch_ctas(dev) : 0;
   const int64_t steps = (n + batch - 1) / batch;
   const size_t pad = 64;  // floats: every part starts on 256 bytes
   auto room = [&](size_t floats) { return (floats + pad - 1) / pad * pad; };
@@ -972,7 +1001,8 @@ int dm_predictor_train(dm_predictor* p, const float* X, const float* T, int64_t 
       float* db = dBias[ep & 1];
       cudaMemcpyAsync(db, bias.data(), sizeof(float) * bias.size(), cudaMemcpyHostToDevice);
       const EpochArgs a{dP, dM, dV, dX, dT, di, reinterpret_cast<const float2*>(db), dL, (int)n, batch, lr, b1, b2, 1e-8f};
-      mlp_epoch_kernel<<<EP_CTAS, EP_THREADS>>>(a);
+      if (ctas == 16) mlp_epoch_kernel<16><<<16, EP_THREADS>>>(a);
+      else mlp_epoch_kernel<8><<<8, EP_THREADS>>>(a);
     } else {
       for (int64_t q = 0; q < steps; ++q) {
         const int64_t off = q * batch;
