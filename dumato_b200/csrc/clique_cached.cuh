@@ -736,7 +736,7 @@ __global__ void __launch_bounds__(256, cached_min_blocks<M>()) clique_cached_ker
   // finished, subtracted from `pending` by the last of its warps to finish its static chunk
   __shared__ unsigned long long blk_sum[4];
   __shared__ unsigned long long blk_k[16];  // fused counts by clique size
-  __shared__ int blk_static_done, blk_warps_done, blk_last;
+  __shared__ int blk_static_done, blk_warps_done;
   if (threadIdx.x < 4) blk_sum[threadIdx.x] = 0ull;
   if (MULTI && threadIdx.x < 16) blk_k[threadIdx.x] = 0ull;
   if (threadIdx.x == 0) {
@@ -910,22 +910,8 @@ __global__ void __launch_bounds__(256, cached_min_blocks<M>()) clique_cached_ker
       for (int j = 3; j <= K; ++j)
         if (blk_k[j]) atomicAdd(&a.c.lb.ctr->count_k[j], blk_k[j]);
     }
-    __threadfence();
-    blk_last = atomicAdd(&a.c.lb.ctr->blocks_done, 1) == (int)gridDim.x - 1 ? 1 : 0;
   }
-  __syncthreads();
-  // The launch clears up after itself: its last block hands the counters to the host and zeroes
-  // them for the next launch, so a call needs no copy before and none after the kernel (each
-  // took 3 to 5 us of a call of 45 us whose kernel runs for 13)
-  if (blk_last) {
-    __threadfence();
-    volatile unsigned* c = reinterpret_cast<volatile unsigned*>(a.c.lb.ctr);
-    unsigned* out = reinterpret_cast<unsigned*>(a.out);
-    for (int i = threadIdx.x; i < (int)(sizeof(DevCounters) / sizeof(unsigned)); i += blockDim.x) {
-      out[i] = c[i];
-      c[i] = 0u;
-    }
-  }
+  counters_to_host(a.c.lb.ctr, a.out);
 }
 
 }  // namespace dmb

@@ -103,6 +103,7 @@ struct dm_graph {
   std::vector<int32_t> up_order;      // motif roots by descending upper degree
   std::vector<int32_t> udeg;          // undirected degree by rank (census)
   int32_t n_deg01 = 0;                // vertices of degree 0 or 1: the lowest ranks
+  std::vector<int32_t> near_steps;    // runs of equal out-degree of deg_order (engine.hpp NearStep)
   int32_t near_list = 0;              // near-clique arena bounds: largest universe, and rows of an
   int64_t near_rows = -1;             // edge (-1: not computed)
   std::vector<void*> pinned;          // host arrays registered with the CUDA driver

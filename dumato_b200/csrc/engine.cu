@@ -131,6 +131,7 @@ struct DeviceSlot {
   int32_t* d_udeg = nullptr;
   int32_t *d_in_end = nullptr, *d_in_deg = nullptr;
   void* d_in = nullptr;
+  void* d_near = nullptr;           // near-clique item runs of deg_order
 };
 
 static std::mutex g_dev_mu;
@@ -680,7 +681,7 @@ void release_device_graphs(dm_graph* g) {
       for (void* p : {(void*)s->dg.d_row, (void*)s->dg.d_deg, (void*)s->dg.d_adj, (void*)s->dg.d_orow,
                       (void*)s->dg.d_odeg, (void*)s->dg.d_oadj, (void*)s->d_deg_order, (void*)s->d_up_order,
                       s->d_blocks, (void*)s->d_boff, (void*)s->d_desc_deg, (void*)s->d_feat[0], (void*)s->d_feat[1],
-                      (void*)s->d_orig, (void*)s->d_udeg, (void*)s->d_in_end, (void*)s->d_in_deg, s->d_in})
+                      (void*)s->d_orig, (void*)s->d_udeg, (void*)s->d_in_end, (void*)s->d_in_deg, s->d_in, s->d_near})
         gbuf_free(p, dv);
       {
         std::lock_guard<std::mutex> lk(g_dev_mu);
@@ -1385,16 +1386,17 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
   DeviceSlot* s = slot_for(g, ctx.device);
   Workspace& ws = s->ws;
   if ((rc = prepare_ws(ws, ctx.stream))) return rc;
-  DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
+  const int world = (o && o->world_size > 1) ? o->world_size : 1;
+  const bool prepares = !s->dg.has_oriented || !s->d_deg_order || !s->d_in || !s->d_near || world > 1;
+  if (prepares) DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
   if (!s->dg.has_oriented && (rc = upload_clique_image(g, s, ctx.stream))) return rc;
   if ((rc = ensure_deg_order(g, s, ctx.stream))) return rc;
   if ((rc = ensure_census(g, s, 4, ctx))) return rc < 0 ? rc : fail(DM_ENOMEM, "no device memory for the in-lists");
   const int c = n - 2;
   const int need = c - 1;  // out-neighbours a root needs to start a c-clique
-  const int world = (o && o->world_size > 1) ? o->world_size : 1;
   int n_roots = need <= g->max_out_degree ? (int)g->cnt_ge[need] : 0;
   const int32_t* d_roots = s->d_deg_order;
-  const int32_t* h_roots = g->deg_order.data();
+  const int32_t* h_roots = nullptr;
   std::vector<int32_t> mine;
   if (world > 1) {
     for (int i = o->rank; i < n_roots; i += world) mine.push_back(g->deg_order[i]);
@@ -1408,35 +1410,56 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
     h_roots = mine.data();
     n_roots = (int)mine.size();
   }
-  // the items are the roots' out-edges: runs of equal out-degree number them
-  std::vector<NearStep> steps;
-  int64_t items = 0;
-  for (int i = 0; i < n_roots;) {
-    const int32_t d = (int32_t)(g->orow[h_roots[i] + 1] - g->orow[h_roots[i]]);
-    int j = i;
-    if (world == 1) j = (int)std::min<int64_t>(n_roots, g->cnt_ge[d]);
-    else
-      while (j < n_roots && g->orow[h_roots[j] + 1] - g->orow[h_roots[j]] == d) ++j;
-    steps.push_back(NearStep{(int32_t)items, i, d, 0});
-    items += (int64_t)(j - i) * d;
-    i = j;
-  }
-  if ((rc = ensure_ws_bytes(reinterpret_cast<void**>(&ws.d_parts), &ws.parts_cap, sizeof(NearStep) * (steps.size() + 1))))
-    return rc;
-  if (!steps.empty())
-    DM_CUDA(cudaMemcpyAsync(ws.d_parts, steps.data(), sizeof(NearStep) * steps.size(), cudaMemcpyHostToDevice,
+  // the items are the roots' out-edges, numbered through the runs of roots of equal out-degree: for
+  // a shard its own, else a prefix of the whole order's, laid out once
+  std::vector<int32_t> mine_steps;
+  auto runs = [&](const int32_t* roots, int n, std::vector<int32_t>& out) {
+    int64_t items = 0;
+    for (int i = 0, j; i < n; i = j) {
+      const int32_t d = (int32_t)(g->orow[roots[i] + 1] - g->orow[roots[i]]);
+      for (j = i + 1; j < n && g->orow[roots[j] + 1] - g->orow[roots[j]] == d;) ++j;
+      out.insert(out.end(), {(int32_t)items, i, d, 0});
+      items += (int64_t)(j - i) * d;
+    }
+    out.insert(out.end(), {(int32_t)items, n, 0, 0});
+  };
+  const void* d_steps = nullptr;
+  const std::vector<int32_t>* steps = &mine_steps;
+  if (world > 1) {
+    runs(h_roots, n_roots, mine_steps);
+    if ((rc = ensure_ws_bytes(reinterpret_cast<void**>(&ws.d_parts), &ws.parts_cap, sizeof(int32_t) * mine_steps.size())))
+      return rc;
+    DM_CUDA(cudaMemcpyAsync(ws.d_parts, mine_steps.data(), sizeof(int32_t) * mine_steps.size(), cudaMemcpyHostToDevice,
                             ctx.stream));
+    d_steps = ws.d_parts;
+  } else {
+    steps = &g->near_steps;
+    if (g->near_steps.empty())
+      runs(g->deg_order.data(), 1 <= g->max_out_degree ? (int)g->cnt_ge[1] : 0, g->near_steps);
+    if (!s->d_near) {
+      const size_t bytes = sizeof(int32_t) * g->near_steps.size();
+      void* p = nullptr;
+      DM_CUDA(gbuf_alloc(&p, bytes));
+      s->d_near = p;
+      DM_CUDA(cudaMemcpyAsync(p, g->near_steps.data(), bytes, cudaMemcpyHostToDevice, ctx.stream));
+    }
+    d_steps = s->d_near;
+  }
+  int n_steps = 0;
+  while (4 * (size_t)(n_steps + 1) < steps->size() && (*steps)[4 * n_steps + 2] >= need) ++n_steps;
+  const int items = (*steps)[4 * (size_t)n_steps];
   NearLaunch L;
   L.dag = GraphView{s->dg.d_orow, s->dg.d_odeg, s->dg.d_oadj, g->n};
   L.in_end = s->d_in_end;
   L.in_deg = s->d_in_deg;
   L.in = s->d_in;
   L.roots = d_roots;
-  L.steps = ws.d_parts;
-  L.n_steps = (int)steps.size();
-  L.n_items = (int)items;
+  L.steps = d_steps;
+  L.n_steps = n_steps;
+  L.n_items = items;
   L.c = c;
-  L.ctr = ws.d_ctr;
+  L.ctr = ws.d_ctr + 1;
+  L.out = ws.h_out;
   if (g->near_rows < 0) {
     // the largest universe and rows that an edge of this graph can have
     g->near_list = 0;
@@ -1457,22 +1480,21 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
     if ((rc = ensure_ws_bytes(&ws.d_scratch, &ws.scratch_cap, per_warp * ctx.arena_warps))) return rc;
     L.arena = reinterpret_cast<int32_t*>(ws.d_scratch);
   }
-  if ((rc = init_counters(ws, (int)items, ctx.stream))) return rc;
+  if (items == 0) std::memset(ws.h_out, 0, sizeof(DevCounters));  // no launch
   DM_CUDA(cudaEventRecord(ws.k0, ctx.stream));
   int grid = 0;
   Reporter reporter;
   if (items > 0) {
     if ((rc = near_clique_launch(L, ctx, &grid))) return rc;
-    if ((rc = reporter.start(o, ctx.device, ws.d_ctr, grid * 8, items))) return rc;
+    if ((rc = reporter.start(o, ctx.device, L.ctr, grid * 8, items, 0, items))) return rc;
   }
   DM_CUDA(cudaEventRecord(ws.k1, ctx.stream));
-  DM_CUDA(cudaMemcpyAsync(ws.h_out, ws.d_ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, ctx.stream));
   DM_CUDA(cudaStreamSynchronize(ctx.stream));
   const DevCounters h = *ws.h_out;
   if ((rc = reset_queue(ws, h, ctx.stream))) return rc;
   float kms = 0, pms = 0;
   cudaEventElapsedTime(&kms, ws.k0, ws.k1);
-  cudaEventElapsedTime(&pms, ws.ev0, ws.k0);
+  if (prepares) cudaEventElapsedTime(&pms, ws.ev0, ws.k0);
   if (h.err) return fail(kernel_status(h.err), "near-clique kernel reported error " + std::to_string(h.err));
   *count = h.count;
   if (st) {

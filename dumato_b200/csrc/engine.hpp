@@ -170,7 +170,8 @@ struct NearLaunch {
   int n_steps = 0;
   int n_items = 0;                 // out-edges of the roots
   int c = 2;                       // clique size n - 2
-  DevCounters* ctr = nullptr;
+  DevCounters* ctr = nullptr;      // self-clearing
+  DevCounters* out = nullptr;      // page-locked host copy, written by the kernel
   int32_t* arena = nullptr;        // arena_ints per warp, or null
   size_t arena_ints = 0;
   int list_cap = 0;

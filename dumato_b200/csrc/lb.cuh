@@ -171,6 +171,27 @@ static __device__ __noinline__ bool q_pop(const LBArgs& lb, int home, int& root,
   return false;
 }
 
+// End of a launch on self-clearing counters (all threads of every block, after the block's last
+// adds to them): the last block hands the counters to the host (out: page-locked memory) and
+// zeroes them for the next launch, so a call needs no copy before and none after the kernel (each
+// took 3 to 5 us of a call of 45 us whose kernel runs for 13).
+static __device__ __forceinline__ void counters_to_host(DevCounters* c, DevCounters* out) {
+  __shared__ int last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&c->blocks_done, 1) == (int)gridDim.x - 1 ? 1 : 0;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  volatile unsigned* v = reinterpret_cast<volatile unsigned*>(c);
+  for (int i = threadIdx.x; i < (int)(sizeof(DevCounters) / sizeof(unsigned)); i += blockDim.x) {
+    reinterpret_cast<unsigned*>(out)[i] = v[i];
+    v[i] = 0u;
+  }
+}
+
 // Test hook: waits for test_gate, which nothing sets, until the bounded wait gives up.
 static __device__ __noinline__ void lb_stall(const LBArgs& lb) {
   const long long ts = global_ns();
