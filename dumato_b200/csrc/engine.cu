@@ -851,8 +851,10 @@ static int upload_clique_image(dm_graph* g, DeviceSlot* s, cudaStream_t st) {
   if (rc) return rc;
   void* base = nullptr;
   cudaError_t e = gbuf_alloc(&base, g->img.size());
-  // the first copy goes through the staging buffers; a graph uploaded again is page-locked (once)
-  if (e == cudaSuccess && !g->img_used) {
+  // an image of more than a staging piece goes through the staging buffers the first time and is
+  // page-locked (once) when it is uploaded again: page-locking 8 MB for a single copy took longer
+  // than copying it; a small one is page-locked at once, so that no later upload pays for it
+  if (e == cudaSuccess && !g->img_used && g->img.size() > STAGE_BYTES) {
     Stager stager(s->dg.device, st);
     e = stager.upload(base, g->img.data(), g->img.size());
     g->img_used = true;
