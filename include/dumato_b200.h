@@ -226,7 +226,10 @@ DM_API int dm_count_cliques_upto(dm_graph* g, int32_t kmax, const dm_opts* opts,
    sum over (n-2)-cliques C of t(t-1)/2 with t the size of C's common neighbourhood. */
 DM_API int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* opts, uint64_t* count, dm_stats* stats);
 /* Connected induced k-vertex subgraphs per class of dict (k in [3, 7]).
-   class_counts has n_classes entries (dm_dictionary_shape). */
+   class_counts has n_classes entries (dm_dictionary_shape). Whole graphs of k = 3, 4 are counted
+   from closed-form sums over edges, triangles, 4-cliques and 4-cycles; a shard, a subtree log, a
+   schedule, an explicit vwarp or mode, a report or a test flag asks for the enumeration (the same
+   counts). */
 DM_API int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_opts* opts,
                     uint64_t* class_counts, dm_stats* stats);
 
