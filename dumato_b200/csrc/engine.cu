@@ -1701,7 +1701,7 @@ int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_
   const int vwarp = (ctx.vwarp == 8 || ctx.vwarp == 16) ? ctx.vwarp : 32;
   const size_t per_warp = motif_arena_stride(k, maxdeg, vwarp) * sizeof(int2);
   const size_t budget = (size_t)8 << 30;
-  // (the kernel keeps 32 warps per SM)
+  // (the kernel keeps at most 32 warps per SM)
   ctx.arena_warps = (int)std::min<size_t>((size_t)ctx.num_sms * 32, std::max<size_t>(8, budget / per_warp));
   // vertex bitmaps, zero between calls; past 2 GB they get up to a quarter of the free memory (at
   // most 8 GB), and the launch as many warps as that holds

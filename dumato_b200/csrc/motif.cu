@@ -28,8 +28,15 @@ struct MotifArgs {
 // 13,800 vertices for k <= 5, 9,200 above); larger graphs keep them in global memory.
 constexpr size_t MOTIF_SMEM_BITS_MAX = 54 * 1024;
 
+// Blocks per SM the registers are sized for: three for k >= 5 (80 registers; with four, 64 registers
+// and 120 bytes of spills per thread, k = 5 took 3.79 ms instead of 3.53 on a Chung-Lu graph of 3,000
+// vertices and 0.72 instead of 0.58 on a random graph of 2,000, k = 6 there 4.24 instead of 4.19),
+// four for k = 4, whose shorter chains want the warps (5.5 ms, 5.8 with three, on a Chung-Lu
+// graph of 18,700 vertices).
+__host__ __device__ constexpr int motif_min_blocks(int K) { return K >= 5 ? 3 : 4; }
+
 template <int K, int W>
-__global__ void __launch_bounds__(32 * MOTIF_WARPS, 4) motif_kernel(const __grid_constant__ MotifArgs a) {
+__global__ void __launch_bounds__(32 * MOTIF_WARPS, motif_min_blocks(K)) motif_kernel(const __grid_constant__ MotifArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   unsigned long long* bhist = reinterpret_cast<unsigned long long*>(smem);
   unsigned char* wbase = smem + sizeof(unsigned long long) * ((a.n_classes + 1) & ~1);

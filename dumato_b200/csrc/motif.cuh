@@ -29,7 +29,7 @@
 // masks looked up and flushed) took 12.6 ms for k = 5 on a Chung-Lu graph of 3,000 vertices and
 // 18,000 edges, 10.4 ms for k = 6 on a random graph of 2,000 / 10,000, 387 ms for a batch of 24
 // graphs; the sweep took 6.5, 5.3 and 86 ms while the sets were sorted lists in global memory that
-// masks and adjacency were searched in, and takes 3.8, 4.2 and 51 ms with one bitmap per mask bit
+// masks and adjacency were searched in, and takes 3.5, 4.2 and 51 ms with one bitmap per mask bit
 // and the sets of level k-3 in shared memory.
 //
 // Virtual warps (the reference's DM_WCV variant, src/DM_WCV/DuMatoGPU.cu:12-37): with W < 32
