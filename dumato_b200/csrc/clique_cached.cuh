@@ -306,32 +306,47 @@ __device__ __forceinline__ unsigned edges_inside(const Bits<NW>& T, const uint64
 
 // 5- and 6-cliques of a wide root (rows of two or more words), items [tw.range) of its local
 // edges (c1, c2). With S = row[c1] & row[c2], a 5-clique is an edge inside S, a 6-clique an edge
-// inside T = S & row[c3] for a member c3 of S. A warp takes TAKE items together; for k = 6 the (item,
+// inside T = S & row[c3] for a member c3 of S. A warp takes 8 or 32 items together; for k = 6 the (item,
 // c3) pairs of their sets are laid end to end over the lanes through the prefix of their sizes,
 // and each lane counts the edges inside its T in a loop of its own.
 //
 // The lockstep walk pays about 100 instructions of stack, counters and selects for every node,
 // and at these sizes (out-degrees to 171, 4.5e8 of 5.2e8 nodes of the k = 6 walk at its last level
 // on an R-MAT graph of 98,552 vertices) nearly all nodes are last ones, whose whole work is one AND
-// and popcount per word: 6-cliques of that graph took 6.8 ms per call, now 3.3 (3.6 with 32 items
-// at a time, 0.32 instead of 0.14 of the warp time idle). Rows of one word stay with the walk: their sets are too
-// small to fill a loop.
+// and popcount per word: 6-cliques of that graph took 6.8 ms per call, now 2.95. Rows of one word
+// stay with the walk: their sets are too small to fill a loop. So do k >= 7 and the fused count, for
+// which the pairs would have to be laid out once more per level; that form has not been built.
+//
+// How often a task looks up, in SM cycles. Progress, and the demand for work with it, every
+// WIDE_CHECK: at every batch the adds of some thousand warps to one word set the pace on light tasks.
+// Items are handed out only while the rest of the task, at its pace so far, is worth WIDE_REST: a
+// donated range costs its receiver the staging of the block and the row prefix again. On random graphs of
+// 1,500 vertices with edge probability 0.1 (out-degrees to 131, sets mostly empty) 5-, 6-cliques took
+// 0.148, 0.277 ms with a look at every batch and ranges split to the last, 0.080, 0.081 now (the walk
+// 0.089, 0.095); 0.25 as long a WIDE_REST 0.128, 0.135; 0.5 or 2 times WIDE_CHECK the same within 5 %.
+constexpr long long WIDE_CHECK = 8192, WIDE_REST = 64000;
 template <int K, int NW>
 __device__ __forceinline__ unsigned long long wide_run(const CachedArgs& a, const TaskWords& tw, const uint64_t* rows,
                                                        const int32_t* sE, int root, int d, bool eager, CheckState& cs) {
   const int lane = lane_id();
   const LBArgs& lb = a.c.lb;
   const long long t_start = lane == 0 ? clock64() : 0;
-  // items taken together: a 6-clique item holds some hundred pairs at these sizes, so few of them
-  // fill the lanes, and ranges stay divisible for idle warps almost to their end
-  constexpr int TAKE = K == 6 ? 8 : 32;
-  constexpr int need = TAKE;
+  const bool at_once = lb.donate_after_ns == 0;  // (a test's donations)
+  long long t_check = t_start + (at_once ? 0 : WIDE_CHECK);
+  int taken = 0, told = 0;  // items taken, and those reported as progress
+  // items taken together: an item's set holds about (E/d)^2 / d members (E local edges of d
+  // members). From 8 members on a 6-clique item has pairs enough that eight items fill the lanes, and
+  // ranges stay divisible for idle warps almost to their end (R-MAT graph above: 3.6 ms with 32, 0.32
+  // instead of 0.14 of the warp time idle); smaller sets need an item on every lane (6-cliques of a
+  // random graph of 900 vertices with edge probability 0.25: 0.77 ms with 8, 0.33 with 32)
+  const float mean = (float)sE[d] / (float)d;
+  const int take = K == 6 && mean * mean >= 8.f * (float)d ? 8 : 32;
   int xb = 0, xe = 0;  // lane 0: split-off items that no queue slot took
   unsigned long long cnt = 0;
   uint64_t* sets = tw.stk;  // k = 6: the items' sets, [word][lane]
   while (true) {
     unsigned long long old = 0ull;
-    if (lane == 0) old = atomicAdd(tw.range, (unsigned long long)TAKE);
+    if (lane == 0) old = atomicAdd(tw.range, (unsigned long long)take);
     old = __shfl_sync(FULL_MASK, old, 0);
     const int next = (int)(unsigned)old, end = (int)(unsigned)(old >> 32);
     if (next >= end) {
@@ -347,7 +362,7 @@ __device__ __forceinline__ unsigned long long wide_run(const CachedArgs& a, cons
     const int it = next + lane;
     Bits<NW> S;
     int p = 0;
-    if (lane < TAKE && it < end) {
+    if (lane < take && it < end) {
       const int c1 = lower_bound_bl<(NW == 2 ? 128 : 256)>(sE, d + 1, it + 1) - 1;
       const int c2 = select_row<NW>(rows + c1 * NW, it - sE[c1]);
 #pragma unroll
@@ -391,13 +406,20 @@ __device__ __forceinline__ unsigned long long wide_run(const CachedArgs& a, cons
       }
       __syncwarp();
     }
+    taken += take;
     if (lane == 0) {
-      atomicAdd(&lb.ctr->progress, (unsigned long long)TAKE);
-      if (lb.hungry_trigger > 0) {
-        if (next + TAKE < end)
-          lockstep_donate(lb, tw, cs, end - next - TAKE, need, root, t_start, 0, need, 0, nullptr, eager, xb, xe);
-        cs.hungry = vload(&lb.ctr->hungry);  // read after the next items: never waited for
-        cs.queued = vload(&lb.ctr->queued);
+      const long long now = clock64();
+      const int left = end - next - take;
+      if (left > 0 && ((now - t_start) * left >= WIDE_REST * taken || at_once))
+        lockstep_donate(lb, tw, cs, left, take, root, t_start, 0, take, 0, nullptr, eager, xb, xe);
+      if (now >= t_check) {
+        t_check = now + (at_once ? 0 : WIDE_CHECK);
+        atomicAdd(&lb.ctr->progress, (unsigned long long)(taken - told));
+        told = taken;
+        if (lb.hungry_trigger > 0) {
+          cs.hungry = vload(&lb.ctr->hungry);  // read after the next items: never waited for
+          cs.queued = vload(&lb.ctr->queued);
+        }
       }
     }
     __syncwarp();

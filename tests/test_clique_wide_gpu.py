@@ -48,3 +48,24 @@ def test_complete_graphs(dm, gpu, n):
     g = dm.Graph.from_edges(*np.triu_indices(n, 1))
     for k in (5, 6):
         assert dm.count_cliques(g, k)[0] == comb(n, k)
+
+
+@pytest.mark.parametrize("n,p", [(1500, 0.1), (300, 0.5)])
+def test_light_and_heavy_sets_vs_oracle(dm, orc, gpu, n, p):
+    """Wide roots whose sets are mostly empty (an item on every lane, and no ranges handed out for
+    tasks of some microseconds: a donation per root at most, where ranges split to the last made
+    more than two) and ones whose sets hold many members. Exact counts."""
+    rng = np.random.default_rng(n)
+    u, v = np.triu_indices(n, 1)
+    keep = rng.random(u.size) < p
+    g = dm.Graph.from_edges(u[keep], v[keep])
+    assert 64 < g.info().max_out_degree <= 256
+    og = orc.OracleGraph.from_pairs(*g.edges())
+    for k in (5, 6):
+        want, _ = orc.clique_dag_bytes(og, k)
+        assert dm.count_cliques(g, k, dm.Options(test_flags=dm.TEST_EAGER_DONATION))[0] == want
+        for _ in range(3):
+            got, st = dm.count_cliques(g, k)
+            assert got == want
+            if p < 0.2:
+                assert st.donations < n, st.donations
