@@ -729,6 +729,24 @@ int check_opts(const dm_opts* o) {
   return DM_OK;
 }
 
+// A counting call that returns an error waits for what it has enqueued (the launch, the clearing of
+// the counters and the queue): the next call on the graph's workspace may run on another stream,
+// and the self-clearing counters are not uploaded again. A good call ends with its own wait.
+class ErrorWait {
+ public:
+  explicit ErrorWait(cudaStream_t st) : st_(st) {}
+  ~ErrorWait() {
+    if (!done_) cudaStreamSynchronize(st_);
+  }
+  ErrorWait(const ErrorWait&) = delete;
+  ErrorWait& operator=(const ErrorWait&) = delete;
+  void done() { done_ = true; }
+
+ private:
+  cudaStream_t st_;
+  bool done_ = false;
+};
+
 // Descending out-degree order of all roots: computed once per graph (host), uploaded once
 // per device copy.
 static void host_deg_order(dm_graph* g) {
@@ -1075,6 +1093,7 @@ static int count_cliques_impl(dm_graph* g, int32_t k, const dm_opts* o, uint64_t
   ensure_oriented(g);
   DeviceSlot* s = slot_for(g, ctx.device);
   Workspace& ws = s->ws;
+  ErrorWait wait(ctx.stream);
   if ((rc = prepare_ws(ws, ctx.stream))) return rc;
   // (a plain call on a resident graph prepares nothing: no event, prep_ms 0)
   const bool prepares = !s->dg.has_oriented || s->index_state == 0 ||
@@ -1149,7 +1168,10 @@ static int count_cliques_impl(dm_graph* g, int32_t k, const dm_opts* o, uint64_t
   const bool use_index = want_index && s->index_state == 1 && d_desc != nullptr;
   // the plain task list on the index holds the parts of the split roots too (they lead it)
   if (use_index && d_desc == s->d_desc_deg && n_roots > 0) n_roots += g->idx_extra;
-  if (upto && (!use_index || max_d > INDEX_MAX_DEGREE || (o && o->subtree_counts))) return 1;
+  if (upto && (!use_index || max_d > INDEX_MAX_DEGREE || (o && o->subtree_counts))) {
+    if (!prepares) wait.done();  // nothing was enqueued
+    return 1;
+  }
   // triangles of the whole graph: the popcount of the index (an explicit staging, a report or a test
   // hook asks for the task kernel)
   const bool flat = k == 3 && !upto && use_index && d_desc == s->d_desc_deg && max_d <= INDEX_MAX_DEGREE &&
@@ -1269,6 +1291,7 @@ static int count_cliques_impl(dm_graph* g, int32_t k, const dm_opts* o, uint64_t
   if (h.err)
     return fail(kernel_status(h.err),
                 "clique kernel reported error " + std::to_string(h.err));
+  wait.done();
   *count = h.count;
   if (upto) {
     for (int j = 3; j <= k; ++j) upto[j - 3] = h.count_k[j];
@@ -1387,6 +1410,7 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
   ensure_oriented(g);
   DeviceSlot* s = slot_for(g, ctx.device);
   Workspace& ws = s->ws;
+  ErrorWait wait(ctx.stream);
   if ((rc = prepare_ws(ws, ctx.stream))) return rc;
   const int world = (o && o->world_size > 1) ? o->world_size : 1;
   const bool prepares = !s->dg.has_oriented || !s->d_deg_order || !s->d_in || !s->d_near || world > 1;
@@ -1498,6 +1522,7 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
   cudaEventElapsedTime(&kms, ws.k0, ws.k1);
   if (prepares) cudaEventElapsedTime(&pms, ws.ev0, ws.k0);
   if (h.err) return fail(kernel_status(h.err), "near-clique kernel reported error " + std::to_string(h.err));
+  wait.done();
   *count = h.count;
   if (st) {
     std::memset(st, 0, sizeof(*st));
@@ -1527,12 +1552,16 @@ static int motif_census(dm_graph* g, int k, const dm_dictionary* dict, const int
   DeviceSlot* s = slot_for(g, ctx.device);
   Workspace& ws = s->ws;
   int rc;
+  ErrorWait wait(ctx.stream);
   if ((rc = prepare_ws(ws, ctx.stream))) return rc;
   const bool prepares = !s->dg.has_oriented || s->index_state == 0 || !s->d_udeg || (k == 4 && !s->d_in);
   if (prepares) DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
   if (!s->dg.has_oriented && (rc = upload_clique_image(g, s, ctx.stream))) return rc;
   if ((rc = ensure_index(g, s, ctx))) return rc;
-  if (s->index_state != 1) return 1;
+  if (s->index_state != 1) {
+    if (!prepares) wait.done();  // nothing was enqueued
+    return 1;
+  }
   if ((rc = ensure_census(g, s, k, ctx))) return rc;
   CensusLaunch L;
   if (k == 4) {
@@ -1569,6 +1598,7 @@ static int motif_census(dm_graph* g, int k, const dm_dictionary* dict, const int
   }
   DM_CUDA(cudaEventRecord(ws.k1, ctx.stream));
   DM_CUDA(cudaStreamSynchronize(ctx.stream));
+  wait.done();
   uint64_t sums[CENSUS_SUMS], types[6];
   for (int i = 0; i < CENSUS_SUMS; ++i) sums[i] = ws.h_sums[i];
   census_classes(k, sums, types);
@@ -1613,6 +1643,7 @@ int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_
   std::lock_guard<std::mutex> lk(g->mu);
   DeviceSlot* s = slot_for(g, ctx.device);
   Workspace& ws = s->ws;
+  ErrorWait wait(ctx.stream);
   if ((rc = prepare_ws(ws, ctx.stream))) return rc;
   DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
   if (!s->dg.has_undirected) {
@@ -1787,6 +1818,7 @@ int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_
   if (h.err)
     return fail(kernel_status(h.err),
                 "motif kernel reported error " + std::to_string(h.err));
+  wait.done();
   if (st) {
     std::memset(st, 0, sizeof(*st));
     st->kernel_ms = kms;
