@@ -47,6 +47,7 @@ static CachedArgs cached_args(const CliqueLaunch& L, LaunchCtx& ctx) {
   a.blocks = reinterpret_cast<const uint4*>(L.blocks);
   a.boff = L.boff;
   a.out = L.out;
+  a.next = L.next;
   a.c.lb.cursor0 = L.n_static;
   a.c.lb.pending0 = L.n_roots;
   a.static_chunk = L.static_chunk;

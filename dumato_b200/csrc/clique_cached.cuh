@@ -189,6 +189,7 @@ struct CachedArgs {
   const uint4* blocks;         // the clique index
   const uint32_t* boff;        // block offset per root (rank space), for donated tasks
   DevCounters* out;            // page-locked host memory: the counters at the end of the launch
+  DevCounters* next;           // the next launch's counters, zeroed by this one
   int static_chunk;            // entries per warp dealt statically (at most CHUNK_MAX)
   int n_static;                // entries [0, n_static) are dealt statically, warp w taking
                                // w, w + T, w + 2T, ... (T warps): the heaviest entries of a
@@ -933,7 +934,7 @@ __global__ void __launch_bounds__(256, cached_min_blocks<M>()) clique_cached_ker
         if (blk_k[j]) atomicAdd(&a.c.lb.ctr->count_k[j], blk_k[j]);
     }
   }
-  counters_to_host(a.c.lb.ctr, a.out);
+  counters_to_host(a.c.lb.ctr, a.next, a.out);
 }
 
 }  // namespace dmb

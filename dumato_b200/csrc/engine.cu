@@ -31,7 +31,8 @@ const char* cuda_err_str(cudaError_t e) { return cudaGetErrorString(e); }
 
 // Per-(graph, device) workspace, reused across calls.
 struct Workspace {
-  DevCounters* d_ctr = nullptr;     // [0] initialised by every call, [1] self-clearing (index kernel)
+  DevCounters* d_ctr = nullptr;     // [0] initialised by every call; [1], [2] self-clearing, in turn:
+  int turn = 0;                     // a launch on [1 + turn] zeroes the other for the next one
   unsigned long long* d_sums = nullptr;  // census sums (CENSUS_BYTES behind d_ctr), self-clearing
   int32_t* d_tasks = nullptr;
   size_t tasks_cap = 0;
@@ -72,7 +73,7 @@ struct Workspace {
   DevCounters* h_out = nullptr;     // pinned: the counters read back after the kernel
   unsigned long long* h_sums = nullptr;  // pinned (behind h_out): the census sums of a call
 };
-constexpr size_t CTR_BYTES = 2 * sizeof(DevCounters) + CENSUS_BYTES;
+constexpr size_t CTR_BYTES = 3 * sizeof(DevCounters) + CENSUS_BYTES;
 
 
 // Empty state: every shard's positions at 0, slot j of a shard carrying sequence j.
@@ -621,7 +622,7 @@ static int prepare_ws(Workspace& ws, cudaStream_t st) {
   if (!ws.d_ctr) {
     DM_CUDA(cudaMalloc(&ws.d_ctr, CTR_BYTES));
     DM_CUDA(cudaMemsetAsync(ws.d_ctr, 0, CTR_BYTES, st));
-    ws.d_sums = reinterpret_cast<unsigned long long*>(ws.d_ctr + 2);
+    ws.d_sums = reinterpret_cast<unsigned long long*>(ws.d_ctr + 3);
   }
   if (!ws.h_init) DM_CUDA(cudaMallocHost(&ws.h_init, sizeof(DevCounters)));
   if (!ws.h_out) {
@@ -1225,8 +1226,9 @@ static int count_cliques_impl(dm_graph* g, int32_t k, const dm_opts* o, uint64_t
   int grid = 0;
   DevCounters* ctr = ws.d_ctr;
   if (use_index) {
-    ctr = ws.d_ctr + 1;
+    ctr = ws.d_ctr + 1 + ws.turn;
     L.ctr = ctr;
+    L.next = ws.d_ctr + 2 - ws.turn;
     L.out = ws.h_out;
     // a root's block is staged in one round trip, so tasks are short: a task may donate
     // after 2 us instead of 20
@@ -1264,6 +1266,7 @@ static int count_cliques_impl(dm_graph* g, int32_t k, const dm_opts* o, uint64_t
   } else if (n_roots > 0) {
     rc = use_index ? clique_cached_launch(L, ctx, grid) : clique_launch(L, ctx, &grid);
     if (rc) return rc;
+    if (use_index) ws.turn ^= 1;
     if ((rc = reporter.start(o, ctx.device, ctr, grid * 8, n_roots, use_index ? L.n_static : 0,
                              use_index ? n_roots : 0)))
       return rc;
@@ -1484,7 +1487,8 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
   L.n_steps = n_steps;
   L.n_items = items;
   L.c = c;
-  L.ctr = ws.d_ctr + 1;
+  L.ctr = ws.d_ctr + 1 + ws.turn;
+  L.next = ws.d_ctr + 2 - ws.turn;
   L.out = ws.h_out;
   if (g->near_rows < 0) {
     // the largest universe and rows that an edge of this graph can have
@@ -1512,6 +1516,7 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
   Reporter reporter;
   if (items > 0) {
     if ((rc = near_clique_launch(L, ctx, &grid))) return rc;
+    ws.turn ^= 1;
     if ((rc = reporter.start(o, ctx.device, L.ctr, grid * 8, items, 0, items))) return rc;
   }
   DM_CUDA(cudaEventRecord(ws.k1, ctx.stream));

@@ -144,6 +144,7 @@ struct CliqueLaunch {
   const void* blocks = nullptr;     // the index (16-byte units)
   const uint32_t* boff = nullptr;   // block offset per root
   DevCounters* out = nullptr;       // page-locked host copy of the counters, written by the kernel
+  DevCounters* next = nullptr;      // the next launch's counters, zeroed by the kernel
   int static_chunk = 1;             // warp w starts with entries [w * static_chunk, +static_chunk)
   int n_static = 0;                 // entries dealt statically; the root cursor starts here
   bool tma = true;                  // stage blocks by bulk asynchronous copies (else 16-byte loads)
@@ -172,6 +173,7 @@ struct NearLaunch {
   int c = 2;                       // clique size n - 2
   DevCounters* ctr = nullptr;      // self-clearing
   DevCounters* out = nullptr;      // page-locked host copy, written by the kernel
+  DevCounters* next = nullptr;     // the next launch's counters, zeroed by the kernel
   int32_t* arena = nullptr;        // arena_ints per warp, or null
   size_t arena_ints = 0;
   int list_cap = 0;

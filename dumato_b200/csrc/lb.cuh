@@ -173,9 +173,10 @@ static __device__ __noinline__ bool q_pop(const LBArgs& lb, int home, int& root,
 
 // End of a launch on self-clearing counters (all threads of every block, after the block's last
 // adds to them): the last block hands the counters to the host (out: page-locked memory) and
-// zeroes them for the next launch, so a call needs no copy before and none after the kernel (each
-// took 3 to 5 us of a call of 45 us whose kernel runs for 13).
-static __device__ __forceinline__ void counters_to_host(DevCounters* c, DevCounters* out) {
+// zeroes the block of counters that the next launch will use, so a call needs no copy before and none
+// after the kernel (each took 3 to 5 us of a call of 45 us whose kernel runs for 13). The launch's own
+// counters keep their final state until the launch after the next: a live report may still read them.
+static __device__ __forceinline__ void counters_to_host(DevCounters* c, DevCounters* next, DevCounters* out) {
   __shared__ int last;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -185,10 +186,10 @@ static __device__ __forceinline__ void counters_to_host(DevCounters* c, DevCount
   __syncthreads();
   if (!last) return;
   __threadfence();
-  volatile unsigned* v = reinterpret_cast<volatile unsigned*>(c);
+  const volatile unsigned* v = reinterpret_cast<const volatile unsigned*>(c);
   for (int i = threadIdx.x; i < (int)(sizeof(DevCounters) / sizeof(unsigned)); i += blockDim.x) {
     reinterpret_cast<unsigned*>(out)[i] = v[i];
-    v[i] = 0u;
+    reinterpret_cast<unsigned*>(next)[i] = 0u;
   }
 }
 

@@ -46,6 +46,7 @@ struct NearArgs {
   int n_steps, n_items;
   LBArgs lb;
   DevCounters* out;         // page-locked host memory: the counters at the end of the launch
+  DevCounters* next;        // the next launch's counters, zeroed by this one
   int32_t* arena;           // per warp: list, rows, sets that do not fit shared memory; or null
   size_t arena_ints;
   int list_cap;             // universe vertices an edge can have
@@ -192,7 +193,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) near_clique_kernel(const __gr
     if (total) atomicAdd(&ctr->count, total);
     atomicAdd(&ctr->tasks, ntasks);
   }
-  counters_to_host(ctr, a.out);
+  counters_to_host(ctr, a.next, a.out);
 }
 
 template <int C>
@@ -228,6 +229,7 @@ int near_clique_launch(const NearLaunch& L, LaunchCtx& ctx, int* grid) {
   a.lb.timeout_ns = (long long)ctx.timeout_ms * 1000000ll;
   a.lb.test_stall = ctx.test_stall;
   a.out = L.out;
+  a.next = L.next;
   a.arena = L.arena;
   a.arena_ints = L.arena_ints;
   a.list_cap = L.list_cap;

@@ -171,3 +171,19 @@ def test_fused_counts_fall_back_per_size(dm, orc, gpu):
     og2 = _og(orc, g2)
     got2, _ = dm.count_cliques_upto(g2, 5, dm.Options(mode=dm.MODE_LIST))
     assert got2 == {k: orc.clique_dag_bytes(og2, k)[0] for k in range(3, 6)}
+
+
+def test_live_reports_after_the_kernel(dm, gpu):
+    """A sample taken after the kernel has ended, while the call still copies its subtree log (8 bytes
+    for each of 6,000,000 vertices), shows the final state: every task dealt and settled."""
+    g = dm.Graph.generate(dm.GEN_ER, 6_000_000, 2_000_000, seed=1)
+    for k in (3, 4):
+        log = np.zeros(g.info().n_vertices, np.uint64)
+        for _ in range(3):
+            samples = []
+            dm.count_cliques(g, k, dm.Options(subtree_counts=log, report=samples.append, report_ms=1))
+            assert samples
+            for a, b in zip(samples, samples[1:]):
+                assert b["roots_claimed"] >= a["roots_claimed"] and b["pending"] <= a["pending"]
+            assert samples[-1]["pending"] == 0
+            assert samples[-1]["roots_claimed"] == samples[-1]["roots_total"]
