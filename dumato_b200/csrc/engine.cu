@@ -239,9 +239,31 @@ struct L2Window {
 // function. The thread stops after the call's stream has been synchronised.
 static std::map<int, cudaStream_t> g_report_streams;
 
+// Near-clique launches count a root's out-edges one by one; their roots from the number of items,
+// through the runs of roots of equal out-degree (NearStep; the entry behind the n runs holds the totals).
+struct ItemRuns {
+  const int32_t* steps = nullptr;
+  int n = 0;
+  int64_t items() const { return steps[4 * (size_t)n]; }
+  int64_t roots() const { return steps[4 * (size_t)n + 1]; }
+  // roots all of whose items are among the first e, and (begun) those any of whose items are
+  int64_t done(int64_t e, bool begun) const {
+    if (e >= items()) return roots();
+    if (e <= 0) return 0;
+    int lo = 0, hi = n;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) / 2;
+      if (steps[4 * (size_t)mid] <= e) lo = mid; else hi = mid;
+    }
+    const int32_t* s = steps + 4 * (size_t)lo;
+    return s[1] + (e - s[0] + (begun ? s[2] - 1 : 0)) / s[2];
+  }
+};
+
 class Reporter {
  public:
-  int start(const dm_opts* o, int dev, const DevCounters* ctr, int warps, int64_t roots, int cursor0 = 0, int pending0 = 0) {
+  int start(const dm_opts* o, int dev, const DevCounters* ctr, int warps, int64_t roots, int cursor0 = 0, int pending0 = 0,
+            ItemRuns runs = ItemRuns()) {
     if (!o || !o->report || o->report_ms <= 0) return DM_OK;
     {
       std::lock_guard<std::mutex> lk(g_dev_mu);
@@ -262,6 +284,7 @@ class Reporter {
     roots_ = roots;
     cursor0_ = cursor0;
     pending0_ = pending0;
+    runs_ = runs;
     t0_ = std::chrono::steady_clock::now();
     th_ = std::thread([this] { run(); });
     return DM_OK;
@@ -296,6 +319,12 @@ class Reporter {
       r.pending = (int64_t)snap_->pending + pending0_;
       r.donations = snap_->donations;
       r.progress = snap_->progress;
+      if (runs_.n) {
+        const int64_t settled = -(int64_t)snap_->pending;
+        r.roots_claimed = runs_.done(snap_->cursor, true);
+        r.pending = roots_ - runs_.done(settled, false);
+        r.progress += (uint64_t)settled;
+      }
       fn_(&r, user_);
     }
   }
@@ -309,6 +338,7 @@ class Reporter {
   int ms_ = 0, dev_ = 0, warps_ = 0;
   int64_t roots_ = 0;
   int cursor0_ = 0, pending0_ = 0;  // where a self-clearing launch counts from
+  ItemRuns runs_;
   std::chrono::steady_clock::time_point t0_;
 };
 
@@ -1517,7 +1547,7 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
   if (items > 0) {
     if ((rc = near_clique_launch(L, ctx, &grid))) return rc;
     ws.turn ^= 1;
-    if ((rc = reporter.start(o, ctx.device, L.ctr, grid * 8, items, 0, items))) return rc;
+    if ((rc = reporter.start(o, ctx.device, L.ctr, grid * 8, n_roots, 0, 0, ItemRuns{steps->data(), n_steps}))) return rc;
   }
   DM_CUDA(cudaEventRecord(ws.k1, ctx.stream));
   DM_CUDA(cudaStreamSynchronize(ctx.stream));
@@ -1533,7 +1563,7 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
     std::memset(st, 0, sizeof(*st));
     st->kernel_ms = kms;
     st->prep_ms = pms;
-    st->tasks = h.tasks;
+    st->tasks = (uint64_t)n_roots;
     st->idle_polls = h.idle_polls;
     st->mode_used = DM_MODE_LIST;
     st->vwarp_used = 32;

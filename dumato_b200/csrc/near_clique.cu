@@ -59,13 +59,15 @@ constexpr int NEAR_LIST = 256;
 constexpr int NEAR_ROWS = 1024;
 constexpr int NEAR_SETS = 9;  // nested sets X (n = 13 chooses nine members from the candidates)
 constexpr int NEAR_WARP_INTS = NEAR_LIST + NEAR_ROWS + NEAR_SETS * (NEAR_LIST / 32);
+constexpr unsigned NEAR_TELL = 64;  // steps of an item between two reports of progress
 
 // Adds t (t - 1) / 2 over the cliques that extend the members chosen so far by LEFT more
 // candidates from index `start` on. X: the candidates and common neighbours left (null: the whole
-// universe); sets: room for the sets below. Warp-uniform but for the last member.
+// universe); sets: room for the sets below. Warp-uniform but for the last member. `nodes` counts the
+// members chosen before the last two; every NEAR_TELL of them are reported as progress.
 template <int LEFT>
 __device__ __forceinline__ void near_dfs(const uint32_t* rows, int W, int m, const uint32_t* X, uint32_t* sets, int start,
-                                         unsigned long long& total) {
+                                         unsigned long long& total, unsigned& nodes, DevCounters* ctr) {
   const int lane = lane_id();
   if constexpr (LEFT == 1) {
     for (int j = start + lane; j < m; j += 32) {
@@ -77,6 +79,9 @@ __device__ __forceinline__ void near_dfs(const uint32_t* rows, int W, int m, con
   } else {
     for (int j = start; j <= m - LEFT; ++j) {
       if (X && !((X[j >> 5] >> (j & 31)) & 1u)) continue;
+      if constexpr (LEFT >= 3) {
+        if (++nodes % NEAR_TELL == 0u && lane == 0) atomicAdd(&ctr->progress, (unsigned long long)NEAR_TELL);
+      }
       const uint32_t* Y = rows + (size_t)j * W;
       if (X) {
         for (int w = lane; w < W; w += 32) sets[w] = X[w] & Y[w];
@@ -91,7 +96,7 @@ __device__ __forceinline__ void near_dfs(const uint32_t* rows, int W, int m, con
         if (w == (m - 1) >> 5) b &= 0xffffffffu >> (31 - ((m - 1) & 31));
         left += __popc(b);
       }
-      if (left >= LEFT - 1) near_dfs<LEFT - 1>(rows, W, m, Y, X ? sets + W : sets, j + 1, total);
+      if (left >= LEFT - 1) near_dfs<LEFT - 1>(rows, W, m, Y, X ? sets + W : sets, j + 1, total, nodes, ctr);
       __syncwarp();
     }
   }
@@ -106,7 +111,8 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) near_clique_kernel(const __gr
   int32_t* own = smem[wib];
   int32_t* arena = a.arena ? a.arena + (size_t)(blockIdx.x * NEAR_WARPS + wib) * a.arena_ints : nullptr;
   DevCounters* ctr = a.lb.ctr;
-  unsigned long long total = 0, ntasks = 0;
+  unsigned long long total = 0;
+  unsigned nodes = 0;
   while (true) {
     int first = 0, count = 0;
     if (lane == 0) {
@@ -118,7 +124,6 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) near_clique_kernel(const __gr
     first = __shfl_sync(FULL_MASK, first, 0);
     count = __shfl_sync(FULL_MASK, count, 0);
     if (count <= 0) break;
-    ntasks += count;
     for (int e = first; e < first + count; ++e) {
       // item e: out-edge i of root o, found through the runs of roots of equal out-degree
       int lo = 0, hi = a.n_steps;
@@ -179,9 +184,10 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) near_clique_kernel(const __gr
             const unsigned bits = __ballot_sync(FULL_MASK, adj);
             if (lane == 0) rows[j * W + w] = bits;
           }
+          if ((w & 63) == 63 && lane == 0) atomicAdd(&ctr->progress, 64ull);
         }
         __syncwarp();
-        near_dfs<C - 2>(rows, W, m, nullptr, sets, 0, total);
+        near_dfs<C - 2>(rows, W, m, nullptr, sets, 0, total, nodes, ctr);
       }
       __syncwarp();
     }
@@ -189,10 +195,7 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) near_clique_kernel(const __gr
   }
   if (lane == 0 && a.lb.test_stall) lb_stall(a.lb);
   total = warp_sum_u64(total);
-  if (lane == 0) {
-    if (total) atomicAdd(&ctr->count, total);
-    atomicAdd(&ctr->tasks, ntasks);
-  }
+  if (lane == 0 && total) atomicAdd(&ctr->count, total);
   counters_to_host(ctr, a.next, a.out);
 }
 

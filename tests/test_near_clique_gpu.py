@@ -58,3 +58,33 @@ def test_near_cliques_match_reference_binaries(dm, gpu):
             seen += 1
     if seen == 0:
         pytest.skip("no reference q_n counts in the fixture")
+
+
+@pytest.mark.parametrize("q,world", [(4, 1), (5, 1), (6, 1), (6, 3), (8, 1)])
+def test_near_clique_reports_and_statistics(dm, orc, gpu, q, world):
+    """Tasks and live reports count root tasks, as for the other entry points, and progress advances."""
+    rng = np.random.default_rng(3)
+    u, v = np.triu_indices(900, 1)
+    keep = rng.random(u.size) < 0.25
+    g = dm.Graph.from_edges(u[keep], v[keep])
+    src, dst = g.edges()
+    deg = np.bincount(np.concatenate([src, dst]), minlength=900)
+    rank = np.empty(900, int)
+    rank[np.lexsort((np.arange(900), deg))] = np.arange(900)
+    out = np.bincount(np.minimum(rank[src], rank[dst]), minlength=900)
+    eligible = int((out >= q - 3).sum())
+    roots = len(range(0, eligible, world))
+    for _ in range(3):
+        samples = []
+        o = dm.Options(report=samples.append, report_ms=1, rank=0, world_size=world)
+        got, st = dm.count_near_cliques(g, q, o)
+        assert st.tasks == roots
+        for a, b in zip(samples, samples[1:]):
+            assert b["roots_claimed"] >= a["roots_claimed"] and b["pending"] <= a["pending"]
+            assert b["progress"] >= a["progress"]
+        for s in samples:
+            assert s["roots_total"] == roots and 0 <= s["roots_claimed"] <= roots and 0 <= s["pending"] <= roots
+        if len(samples) > 2:
+            assert samples[-1]["progress"] > 0
+    if world == 1 and q <= 5:
+        assert got == orc.near_cliques(orc.OracleGraph.from_pairs(src, dst), q)
