@@ -104,8 +104,10 @@ struct dm_graph {
   std::vector<int32_t> udeg;          // undirected degree by rank (census)
   int32_t n_deg01 = 0;                // vertices of degree 0 or 1: the lowest ranks
   std::vector<int32_t> near_steps;    // runs of equal out-degree of deg_order (engine.hpp NearStep)
+  std::vector<int64_t> near_pairs;    // first pair of out-neighbours of each run, and their number
   int32_t near_list = 0;              // near-clique arena bounds: largest universe, and rows of an
-  int64_t near_rows = -1;             // edge (-1: not computed)
+  int64_t near_rows = 0;              // edge
+  int64_t near_work = 0;              // sum over the edges of the degree of their lower end
   std::vector<void*> pinned;          // host arrays registered with the CUDA driver
   // device copies
   std::mutex mu;

@@ -1431,6 +1431,57 @@ static int ensure_census(dm_graph* g, DeviceSlot* s, int k, LaunchCtx& ctx) {
   return DM_OK;
 }
 
+// Runs of roots of equal out-degree in a descending order (NearStep), closed by the totals.
+static void near_runs(const dm_graph* g, const int32_t* roots, int n, std::vector<int32_t>& out) {
+  int64_t items = 0;
+  for (int i = 0, j; i < n; i = j) {
+    const int32_t d = (int32_t)(g->orow[roots[i] + 1] - g->orow[roots[i]]);
+    for (j = i + 1; j < n && g->orow[roots[j] + 1] - g->orow[roots[j]] == d;) ++j;
+    out.insert(out.end(), {(int32_t)items, i, d, 0});
+    items += (int64_t)(j - i) * d;
+  }
+  out.insert(out.end(), {(int32_t)items, n, 0, 0});
+}
+
+// Near-clique tables of a graph and of its device copy, laid out once: the runs of the whole order, the
+// first pair of out-neighbours of each, and the bounds of an edge's universe and rows.
+static int ensure_near(dm_graph* g, DeviceSlot* s, LaunchCtx& ctx) {
+  int rc;
+  if ((rc = ensure_census(g, s, 3, ctx))) return rc < 0 ? rc : fail(DM_ENOMEM, "no device memory for the degrees");
+  if (g->near_steps.empty()) {
+    for (int32_t r = 0; r < g->n; ++r) {
+      const int d = (int)(g->orow[r + 1] - g->orow[r]);
+      if (d < 1) continue;
+      g->near_list = std::max(g->near_list, g->udeg[r]);
+      g->near_rows = std::max(g->near_rows, (int64_t)near_clique_rows(d, g->udeg[r]));
+      g->near_work += (int64_t)d * g->udeg[r];
+    }
+    near_runs(g, g->deg_order.data(), 1 <= g->max_out_degree ? (int)g->cnt_ge[1] : 0, g->near_steps);
+    int64_t pairs = 0;
+    for (size_t i = 0; i < g->near_steps.size(); i += 4) {
+      g->near_pairs.push_back(pairs);
+      if (i + 4 == g->near_steps.size()) break;
+      const int64_t d = g->near_steps[i + 2];
+      pairs += (g->near_steps[i + 5] - g->near_steps[i + 1]) * (d * (d - 1) / 2);
+    }
+  }
+  if (s->d_near) return DM_OK;
+  const size_t a = sizeof(int32_t) * g->near_steps.size(), b = sizeof(int64_t) * g->near_pairs.size();
+  void* p = nullptr;
+  DM_CUDA(gbuf_alloc(&p, a + b));
+  s->d_near = p;
+  DM_CUDA(cudaMemcpyAsync(p, g->near_steps.data(), a, cudaMemcpyHostToDevice, ctx.stream));
+  DM_CUDA(cudaMemcpyAsync(static_cast<char*>(p) + a, g->near_pairs.data(), b, cudaMemcpyHostToDevice, ctx.stream));
+  return DM_OK;
+}
+
+// q_4 by triangles (two launches) or edge by edge (one)? The edge-by-edge form takes near_work search
+// steps. Measured either side of the line, edges / triangles in us per call: work 33,000 (R-MAT 500 /
+// 2,000) 32 / 43, 104,000 (complete graph of 60) 31 / 42, 193,000 (R-MAT 1,377 / 8,000) 55 / 45,
+// 593,000 (random 20,000 / 80,000) 208 / 46. A shard takes its share of the edges but all triangles:
+// 265,000 (Chung-Lu 3,000 / 18,000) 59 / 65, 593,000 134 / 87.
+constexpr int64_t NEAR4_STEPS = 150'000, NEAR4_SHARD_STEPS = 500'000;
+
 int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* count, dm_stats* st) {
   if (!g || !count) return fail(DM_EINVAL, "dm_count_near_cliques: null argument");
   if (n < 4 || n > 13) return fail(DM_EINVAL, "dm_count_near_cliques: n must be in [4, 13]");
@@ -1446,11 +1497,14 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
   ErrorWait wait(ctx.stream);
   if ((rc = prepare_ws(ws, ctx.stream))) return rc;
   const int world = (o && o->world_size > 1) ? o->world_size : 1;
-  const bool prepares = !s->dg.has_oriented || !s->d_deg_order || !s->d_in || !s->d_near || world > 1;
+  const bool prepares = !s->dg.has_oriented || !s->d_deg_order || !s->d_near || (n > 4 && !s->d_in) || world > 1;
   if (prepares) DM_CUDA(cudaEventRecord(ws.ev0, ctx.stream));
   if (!s->dg.has_oriented && (rc = upload_clique_image(g, s, ctx.stream))) return rc;
   if ((rc = ensure_deg_order(g, s, ctx.stream))) return rc;
-  if ((rc = ensure_census(g, s, 4, ctx))) return rc < 0 ? rc : fail(DM_ENOMEM, "no device memory for the in-lists");
+  if ((rc = ensure_near(g, s, ctx))) return rc;
+  const bool by_triangles = n == 4 && g->near_work >= (world > 1 ? NEAR4_SHARD_STEPS : NEAR4_STEPS);
+  if (!by_triangles && (rc = ensure_census(g, s, 4, ctx)))
+    return rc < 0 ? rc : fail(DM_ENOMEM, "no device memory for the in-lists");
   const int c = n - 2;
   const int need = c - 1;  // out-neighbours a root needs to start a c-clique
   int n_roots = need <= g->max_out_degree ? (int)g->cnt_ge[need] : 0;
@@ -1472,37 +1526,16 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
   // the items are the roots' out-edges, numbered through the runs of roots of equal out-degree: for
   // a shard its own, else a prefix of the whole order's, laid out once
   std::vector<int32_t> mine_steps;
-  auto runs = [&](const int32_t* roots, int n, std::vector<int32_t>& out) {
-    int64_t items = 0;
-    for (int i = 0, j; i < n; i = j) {
-      const int32_t d = (int32_t)(g->orow[roots[i] + 1] - g->orow[roots[i]]);
-      for (j = i + 1; j < n && g->orow[roots[j] + 1] - g->orow[roots[j]] == d;) ++j;
-      out.insert(out.end(), {(int32_t)items, i, d, 0});
-      items += (int64_t)(j - i) * d;
-    }
-    out.insert(out.end(), {(int32_t)items, n, 0, 0});
-  };
-  const void* d_steps = nullptr;
-  const std::vector<int32_t>* steps = &mine_steps;
-  if (world > 1) {
-    runs(h_roots, n_roots, mine_steps);
+  const void* d_steps = s->d_near;
+  const std::vector<int32_t>* steps = &g->near_steps;
+  if (world > 1 && !by_triangles) {
+    near_runs(g, h_roots, n_roots, mine_steps);
+    steps = &mine_steps;
     if ((rc = ensure_ws_bytes(reinterpret_cast<void**>(&ws.d_parts), &ws.parts_cap, sizeof(int32_t) * mine_steps.size())))
       return rc;
     DM_CUDA(cudaMemcpyAsync(ws.d_parts, mine_steps.data(), sizeof(int32_t) * mine_steps.size(), cudaMemcpyHostToDevice,
                             ctx.stream));
     d_steps = ws.d_parts;
-  } else {
-    steps = &g->near_steps;
-    if (g->near_steps.empty())
-      runs(g->deg_order.data(), 1 <= g->max_out_degree ? (int)g->cnt_ge[1] : 0, g->near_steps);
-    if (!s->d_near) {
-      const size_t bytes = sizeof(int32_t) * g->near_steps.size();
-      void* p = nullptr;
-      DM_CUDA(gbuf_alloc(&p, bytes));
-      s->d_near = p;
-      DM_CUDA(cudaMemcpyAsync(p, g->near_steps.data(), bytes, cudaMemcpyHostToDevice, ctx.stream));
-    }
-    d_steps = s->d_near;
   }
   int n_steps = 0;
   while (4 * (size_t)(n_steps + 1) < steps->size() && (*steps)[4 * n_steps + 2] >= need) ++n_steps;
@@ -1520,19 +1553,21 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
   L.ctr = ws.d_ctr + 1 + ws.turn;
   L.next = ws.d_ctr + 2 - ws.turn;
   L.out = ws.h_out;
-  if (g->near_rows < 0) {
-    // the largest universe and rows that an edge of this graph can have
-    g->near_list = 0;
-    g->near_rows = 0;
-    for (int32_t r = 0; r < g->n; ++r) {
-      const int d = (int)(g->orow[r + 1] - g->orow[r]);
-      if (d < 1) continue;
-      g->near_list = std::max(g->near_list, g->udeg[r]);
-      g->near_rows = std::max(g->near_rows, (int64_t)near_clique_rows(d, g->udeg[r]));
-    }
+  if (by_triangles) {
+    L.tri_words = g->img_adj_ints;
+    if ((rc = ensure_ws_bytes(reinterpret_cast<void**>(&ws.d_census), &ws.census_cap, sizeof(unsigned) * L.tri_words)))
+      return rc;
+    L.tri = reinterpret_cast<unsigned*>(ws.d_census);
+    L.pair_step = reinterpret_cast<const long long*>(static_cast<const char*>(s->d_near) +
+                                                     sizeof(int32_t) * g->near_steps.size());
+    L.n_pairs = g->near_pairs[n_steps];
+    L.roots = s->d_deg_order;
+    L.shard = world > 1 ? d_roots : nullptr;
+    L.shard_roots = n_roots;
+    L.n_items = n_roots;
   }
   ctx.arena_warps = ctx.num_sms * 64;
-  if (g->near_rows > 0) {
+  if (g->near_rows > 0 && !by_triangles) {
     L.list_cap = g->near_list + 32;
     L.arena_ints = ((size_t)L.list_cap + (size_t)g->near_rows + 63) / 64 * 64;
     const size_t per_warp = L.arena_ints * sizeof(int32_t);
@@ -1547,7 +1582,10 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
   if (items > 0) {
     if ((rc = near_clique_launch(L, ctx, &grid))) return rc;
     ws.turn ^= 1;
-    if ((rc = reporter.start(o, ctx.device, L.ctr, grid * 8, n_roots, 0, 0, ItemRuns{steps->data(), n_steps}))) return rc;
+    // (by triangles every root is dealt at the start, and all are settled by the sum at the end)
+    rc = by_triangles ? reporter.start(o, ctx.device, L.ctr, grid * 8, n_roots, n_roots, n_roots)
+                      : reporter.start(o, ctx.device, L.ctr, grid * 8, n_roots, 0, 0, ItemRuns{steps->data(), n_steps});
+    if (rc) return rc;
   }
   DM_CUDA(cudaEventRecord(ws.k1, ctx.stream));
   DM_CUDA(cudaStreamSynchronize(ctx.stream));

@@ -177,6 +177,15 @@ struct NearLaunch {
   int32_t* arena = nullptr;        // arena_ints per warp, or null
   size_t arena_ints = 0;
   int list_cap = 0;
+  // q_4 by triangles (else null): a counter per padded DAG entry, the first pair of out-neighbours of
+  // each run of the whole order (roots, steps), and the shard's roots (null: all). n_items then
+  // is the number of root tasks.
+  unsigned* tri = nullptr;
+  size_t tri_words = 0;
+  const long long* pair_step = nullptr;
+  long long n_pairs = 0;
+  const int32_t* shard = nullptr;
+  int shard_roots = 0;
 };
 // A run of roots of equal out-degree: its first item (out-edge), first root, out-degree.
 struct NearStep {

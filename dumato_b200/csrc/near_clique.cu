@@ -59,6 +59,7 @@ constexpr int NEAR_LIST = 256;
 constexpr int NEAR_ROWS = 1024;
 constexpr int NEAR_SETS = 9;  // nested sets X (n = 13 chooses nine members from the candidates)
 constexpr int NEAR_WARP_INTS = NEAR_LIST + NEAR_ROWS + NEAR_SETS * (NEAR_LIST / 32);
+constexpr int PAIR_CHUNK = 256;       // pairs of out-neighbours a warp takes together (q_4)
 constexpr unsigned NEAR_TELL = 64;  // steps of an item between two reports of progress
 
 // Adds t (t - 1) / 2 over the cliques that extend the members chosen so far by LEFT more
@@ -217,6 +218,116 @@ static int launch_near(const NearArgs& a, LaunchCtx& ctx, int* grid_out) {
   return DM_OK;
 }
 
+// ---------------- q_4: pairs of triangles on an edge ----------------
+
+// q_4 = sum over edges of t (t - 1) / 2 with t the triangles on the edge. Every triangle is found once
+// on the DAG, from its lowest vertex r: a pair (v, y) of r's out-neighbours, v < y, joined by an edge,
+// which is found at its place in v's row; it adds one to the counters of its three edges. The pairs of
+// all roots are numbered end to end (pair_step: the first pair of each run of roots of equal
+// out-degree), so a root of any size spreads over the grid.
+//
+// Bound by the dependent loads of the searches, one per pair of out-neighbours. Edge by edge
+// (near_clique_kernel<2>), every neighbour of a vertex is searched for each of its out-edges and every
+// triangle is met three times: q_4 takes 6.9 ms on an R-MAT graph of 98,552 vertices / 1.08M edges,
+// 0.52 on a Chung-Lu graph of 18,700 / 198,000 and 13.7 on a random graph of 4,000 with edge
+// probability 0.1, here 0.31, 0.053 and 1.3 (a warp per root, merging undirected lists, took
+// 3.5, 0.36 and 3.5). On small graphs one launch is faster than two (engine.cu NEAR4_STEPS).
+__global__ void __launch_bounds__(256) near_triangle_kernel(const __grid_constant__ NearArgs a, unsigned* tri,
+                                                            const long long* pair_step, long long n_pairs) {
+  const int lane = lane_id();
+  const long long warps = (long long)gridDim.x * NEAR_WARPS;
+  unsigned chunks = 0;
+  for (long long q0 = ((long long)blockIdx.x * NEAR_WARPS + warp_in_block()) * PAIR_CHUNK; q0 < n_pairs;
+       q0 += warps * PAIR_CHUNK) {
+    // the run of the chunk's first pair
+    int s = 0, hi = a.n_steps;
+    while (hi - s > 1) {
+      const int mid = (s + hi) >> 1;
+      if (__ldg(pair_step + mid) <= q0) s = mid; else hi = mid;
+    }
+    for (int c = 0; c < PAIR_CHUNK; c += 32) {
+      const long long q = q0 + c + lane;
+      if (q >= n_pairs) break;
+      while (__ldg(pair_step + s + 1) <= q) ++s;
+      const int4 st = __ldg(a.steps + s);
+      const int d = st.z;
+      const long long rel = q - __ldg(pair_step + s);
+      const unsigned P = (unsigned)((long long)d * (d - 1) / 2);
+      unsigned o, p;
+      if (rel <= 0xffffffffll) {
+        o = (unsigned)rel / P;
+        p = (unsigned)rel - o * P;
+      } else {
+        o = (unsigned)(rel / P);
+        p = (unsigned)(rel - (long long)o * P);
+      }
+      // p = m (m - 1) / 2 + b with 0 <= b < m: v is the m-th out-neighbour from the end
+      unsigned m = (unsigned)((1.f + sqrtf(1.f + 8.f * (float)p)) * 0.5f);
+      while ((unsigned long long)m * (m - 1) / 2 > p) --m;
+      while ((unsigned long long)m * (m + 1) / 2 <= p) ++m;
+      const int i = d - 1 - (int)m, j = i + 1 + (int)(p - (unsigned)((unsigned long long)m * (m - 1) / 2));
+      const int rr = __ldg(a.dag.row + __ldg(a.roots + st.y + (int)o));
+      const int v = __ldg(a.dag.adj + rr + i), y = __ldg(a.dag.adj + rr + j);
+      const int rv = __ldg(a.dag.row + v), nv = __ldg(a.dag.deg + v);
+      const int at = lower_bound(a.dag.adj + rv, 0, nv, y);
+      if (at < nv && __ldg(a.dag.adj + rv + at) == y) {
+        atomicAdd(tri + rr + i, 1u);
+        atomicAdd(tri + rr + j, 1u);
+        atomicAdd(tri + rv + at, 1u);
+      }
+    }
+    __syncwarp();
+    if ((++chunks & 63u) == 0u && lane == 0) atomicAdd(&a.lb.ctr->progress, 64ull * PAIR_CHUNK);
+  }
+}
+
+// The sum over all edges (padding holds no triangle), or over those of the listed roots (a shard).
+__global__ void __launch_bounds__(256) near_pairs_kernel(const __grid_constant__ NearArgs a, const unsigned* tri, int64_t n,
+                                                         const int32_t* roots, int n_roots) {
+  const int t = blockIdx.x * 256 + threadIdx.x, T = gridDim.x * 256;
+  auto pairs = [](unsigned x) -> unsigned long long {
+    return (x & 1) ? (unsigned long long)x * ((x - 1) >> 1) : (unsigned long long)(x >> 1) * (x - 1u);
+  };
+  unsigned long long total = 0;
+  if (roots) {
+    for (int i = t >> 5; i < n_roots; i += T >> 5) {
+      const int r = __ldg(roots + i), b = __ldg(a.dag.row + r), d = __ldg(a.dag.deg + r);
+      for (int j = lane_id(); j < d; j += 32) total += pairs(tri[b + j]);
+    }
+  } else {
+    for (int64_t i = t; i < n; i += T) total += pairs(tri[i]);
+  }
+  if (lane_id() == 0 && a.lb.test_stall) lb_stall(a.lb);
+  total = warp_sum_u64(total);
+  if (lane_id() == 0 && total) atomicAdd(&a.lb.ctr->count, total);
+  if (t == 0) {
+    atomicSub(&a.lb.ctr->pending, a.n_items);
+    atomicAdd(&a.lb.ctr->progress, (unsigned long long)a.n_items);
+  }
+  counters_to_host(a.lb.ctr, a.next, a.out);
+}
+
+static int launch_near4(const NearArgs& a, const NearLaunch& L, LaunchCtx& ctx, int* grid_out) {
+  auto grid_for = [&](int64_t blocks) {
+    if (ctx.threads > 0) blocks = std::min<int64_t>(blocks, (ctx.threads + 255) / 256);
+    return (int)std::max<int64_t>(1, std::min<int64_t>(blocks, ctx.num_sms * 8));
+  };
+  DM_CUDA(cudaMemsetAsync(L.tri, 0, sizeof(unsigned) * L.tri_words, ctx.stream));
+  const int grid = grid_for((L.n_pairs + PAIR_CHUNK * NEAR_WARPS - 1) / (PAIR_CHUNK * NEAR_WARPS));
+  if (L.n_pairs > 0) {
+    near_triangle_kernel<<<grid, 256, 0, ctx.stream>>>(a, L.tri, L.pair_step, L.n_pairs);
+    ctx.launches++;
+    DM_CUDA(cudaGetLastError());
+  }
+  const int64_t work = L.shard ? (int64_t)L.shard_roots * 32 : (int64_t)L.tri_words;
+  near_pairs_kernel<<<grid_for((work + 1023) / 1024), 256, 0, ctx.stream>>>(a, L.tri, (int64_t)L.tri_words, L.shard,
+                                                                           L.shard_roots);
+  ctx.launches++;
+  *grid_out = grid;
+  DM_CUDA(cudaGetLastError());
+  return DM_OK;
+}
+
 int near_clique_launch(const NearLaunch& L, LaunchCtx& ctx, int* grid) {
   NearArgs a;
   a.dag = L.dag;
@@ -236,6 +347,7 @@ int near_clique_launch(const NearLaunch& L, LaunchCtx& ctx, int* grid) {
   a.arena = L.arena;
   a.arena_ints = L.arena_ints;
   a.list_cap = L.list_cap;
+  if (L.tri) return launch_near4(a, L, ctx, grid);
   switch (L.c) {
     case 2: return launch_near<2>(a, ctx, grid);
     case 3: return launch_near<3>(a, ctx, grid);
