@@ -177,6 +177,7 @@ struct NearLaunch {
   int32_t* arena = nullptr;        // arena_ints per warp, or null
   size_t arena_ints = 0;
   int list_cap = 0;
+  int max_claim = 1;               // larger claims than the guided ones, up to these (<= 32)
   // q_4 by triangles (else null): a counter per padded DAG entry, the first pair of out-neighbours of
   // each run of the whole order (roots, steps), and the shard's roots (null: all). n_items then
   // is the number of root tasks.

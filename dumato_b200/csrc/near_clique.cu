@@ -16,7 +16,10 @@
 // X = the universe cap the rows of the members chosen so far holds both the candidates left and
 // the common neighbours, and t_C = popc(X & row of the last member), one last member per lane.
 // Edges are numbered by descending out-degree of r, so the heaviest start first, and claimed in
-// runs from a cursor.
+// runs from a cursor. A claim is laid out with an edge per lane, and where out-degrees are small the
+// candidates of all its edges are searched side by side first, since most edges of a sparse graph have
+// too few: one edge after the other, q_5 of a random graph of 50,000 / 200,000 took 320 us, now 129
+// (claims of one to three edges go on directly: q_6 of the R-MAT graph below 66 us, 70 with the search).
 //
 // Bound by the dependent loads of the membership searches that build the rows (one binary search
 // in an out-row per universe vertex and candidate, 32 side by side); the counting is AND + popc
@@ -50,6 +53,7 @@ struct NearArgs {
   int32_t* arena;           // per warp: list, rows, sets that do not fit shared memory; or null
   size_t arena_ints;
   int list_cap;             // universe vertices an edge can have
+  int max_claim;            // of light items a warp claims up to half its share, at most these (<= 32)
 };
 
 constexpr int NEAR_WARPS = 8;
@@ -60,6 +64,7 @@ constexpr int NEAR_ROWS = 1024;
 constexpr int NEAR_SETS = 9;  // nested sets X (n = 13 chooses nine members from the candidates)
 constexpr int NEAR_WARP_INTS = NEAR_LIST + NEAR_ROWS + NEAR_SETS * (NEAR_LIST / 32);
 constexpr int PAIR_CHUNK = 256;       // pairs of out-neighbours a warp takes together (q_4)
+constexpr int NEAR_LIGHT = 32;        // out-degrees up to which a claim's candidates are searched together
 constexpr unsigned NEAR_TELL = 64;  // steps of an item between two reports of progress
 
 // Adds t (t - 1) / 2 over the cliques that extend the members chosen so far by LEFT more
@@ -118,30 +123,76 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) near_clique_kernel(const __gr
     int first = 0, count = 0;
     if (lane == 0) {
       const int left = a.n_items - vload(&ctr->cursor);
-      const int chunk = max(1, min(16, left / (8 * total_warps)));
+      const int chunk = max(1, max(min(16, left / (8 * total_warps)), min(a.max_claim, left / (2 * total_warps))));
       first = left > 0 ? atomicAdd(&ctr->cursor, chunk) : a.n_items;
       count = min(chunk, a.n_items - first);
     }
     first = __shfl_sync(FULL_MASK, first, 0);
     count = __shfl_sync(FULL_MASK, count, 0);
     if (count <= 0) break;
-    for (int e = first; e < first + count; ++e) {
-      // item e: out-edge i of root o, found through the runs of roots of equal out-degree
+    // lane l: item first + l, out-edge i of a root, found through the runs of roots of equal out-degree
+    int my_d = 0, my_i = 0, my_nin = 0, my_row = 0, my_v = 0, my_rv = 0, my_nb = 0, my_in = 0;
+    if (lane < count) {
+      const int e = first + lane;
       int lo = 0, hi = a.n_steps;
       while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
         if (__ldg(&a.steps[mid].x) <= e) lo = mid; else hi = mid;
       }
       const int4 st = __ldg(a.steps + lo);
-      const int d = st.z;
-      const int o = st.y + (e - st.x) / d, i = (e - st.x) % d;
-      if (d - 1 - i < C - 2) continue;
-      const int r = __ldg(a.roots + o);
-      const int32_t* L = a.dag.adj + __ldg(a.dag.row + r);
-      const int v = __ldg(L + i);
-      const int32_t* B = a.dag.adj + __ldg(a.dag.row + v);
-      const int nb = __ldg(a.dag.deg + v);
-      const int nin = __ldg(a.in_deg + r);
+      my_d = st.z;
+      const int o = (e - st.x) / my_d;
+      my_i = (e - st.x) - o * my_d;
+      if (my_d - 1 - my_i >= C - 2) {
+        const int r = __ldg(a.roots + st.y + o);
+        my_row = __ldg(a.dag.row + r);
+        my_nin = __ldg(a.in_deg + r);
+        my_in = __ldg(a.in_end + r) - my_nin;
+        my_v = __ldg(a.dag.adj + my_row + my_i);
+        my_rv = __ldg(a.dag.row + my_v);
+        my_nb = __ldg(a.dag.deg + my_v);
+      }
+    }
+    bool mine = lane < count && my_d - 1 - my_i >= C - 2;
+    if (C > 2 && count >= 4 && __shfl_sync(FULL_MASK, my_d, 0) <= NEAR_LIGHT) {
+      // light items: all their candidates side by side first, and only those with enough of them on
+      const int len = mine ? my_d - 1 - my_i : 0;
+      int off = len;
+#pragma unroll
+      for (int s = 1; s < 32; s <<= 1) {
+        const int y = __shfl_up_sync(FULL_MASK, off, s);
+        if (lane >= s) off += y;
+      }
+      const int all = __shfl_sync(FULL_MASK, off, 31);
+      off -= len;
+      int found = 0;
+      for (int f0 = 0; f0 < all; f0 += 32) {
+        const int f = f0 + lane;
+        int j = 0;  // owner: the last item whose candidates start at or before f
+#pragma unroll
+        for (int h = 16; h >= 1; h >>= 1) {
+          const int x = __shfl_sync(FULL_MASK, off, j + h);
+          j = x <= f ? j + h : j;
+        }
+        const int at = __shfl_sync(FULL_MASK, my_row + my_i + 1 - off, j) + f;
+        const int rv = __shfl_sync(FULL_MASK, my_rv, j), nb = __shfl_sync(FULL_MASK, my_nb, j);
+        const bool hit = f < all && contains(a.dag.adj + rv, nb, __ldg(a.dag.adj + at));
+        const unsigned bal = __ballot_sync(FULL_MASK, hit);
+        const int a0 = min(max(off - f0, 0), 32), a1 = min(max(off + len - f0, 0), 32);
+        const unsigned upto1 = a1 >= 32 ? 0xffffffffu : (1u << a1) - 1u;
+        const unsigned upto0 = a0 >= 32 ? 0xffffffffu : (1u << a0) - 1u;
+        found += __popc(bal & upto1 & ~upto0);
+      }
+      mine = mine && found >= C - 2;
+    }
+    for (unsigned todo = __ballot_sync(FULL_MASK, mine); todo; todo &= todo - 1) {
+      const int src = __ffs(todo) - 1;
+      const int d = __shfl_sync(FULL_MASK, my_d, src), i = __shfl_sync(FULL_MASK, my_i, src);
+      const int nin = __shfl_sync(FULL_MASK, my_nin, src), v = __shfl_sync(FULL_MASK, my_v, src);
+      const int nb = __shfl_sync(FULL_MASK, my_nb, src);
+      const int32_t* L = a.dag.adj + __shfl_sync(FULL_MASK, my_row, src);
+      const int32_t* B = a.dag.adj + __shfl_sync(FULL_MASK, my_rv, src);
+      const int2* I = a.in + __shfl_sync(FULL_MASK, my_in, src);
       int32_t* uni = d + nin <= NEAR_LIST ? own : arena;
       // candidates: above v, and out-neighbours of both
       int m = 0;
@@ -158,7 +209,6 @@ __global__ void __launch_bounds__(32 * NEAR_WARPS) near_clique_kernel(const __gr
         const int y = j < i ? __ldg(L + j) : 0;
         u += compact(uni, u, y, j < i && contains(a.dag.adj + __ldg(a.dag.row + y), __ldg(a.dag.deg + y), v));
       }
-      const int2* I = a.in + (__ldg(a.in_end + r) - nin);
       for (int j0 = 0; j0 < nin; j0 += 32) {
         const int j = j0 + lane;
         const int y = j < nin ? __ldg(&I[j].x) : 0;
@@ -347,6 +397,7 @@ int near_clique_launch(const NearLaunch& L, LaunchCtx& ctx, int* grid) {
   a.arena = L.arena;
   a.arena_ints = L.arena_ints;
   a.list_cap = L.list_cap;
+  a.max_claim = L.max_claim;
   if (L.tri) return launch_near4(a, L, ctx, grid);
   switch (L.c) {
     case 2: return launch_near<2>(a, ctx, grid);

@@ -88,3 +88,49 @@ def test_near_clique_reports_and_statistics(dm, orc, gpu, q, world):
             assert samples[-1]["progress"] > 0
     if world == 1 and q <= 5:
         assert got == orc.near_cliques(orc.OracleGraph.from_pairs(src, dst), q)
+
+
+@pytest.mark.parametrize("kind", ["complete", "hub", "runs", "sparse"])
+def test_four_vertex_near_cliques_by_triangles(dm, orc, gpu, kind):
+    """q_4 of graphs above the size from which triangles are counted per edge, whole and in shards:
+    one run of roots per out-degree, a hub, long runs of equal out-degree (chunks of pairs that
+    cross runs), and hardly any triangle."""
+    rng = np.random.default_rng(2)
+    if kind == "complete":
+        g = dm.Graph.from_edges(*np.triu_indices(131, 1))
+    elif kind == "hub":
+        s, t = rng.integers(0, 5000, 60_000), rng.integers(0, 5000, 60_000)
+        g = dm.Graph.from_edges(np.concatenate([s, np.zeros(4000, int)]), np.concatenate([t, np.arange(1000, 5000)]))
+    elif kind == "runs":       # a circulant graph: each vertex joined to the next 40
+        n, w = 2003, 40
+        s = np.repeat(np.arange(n), w)
+        g = dm.Graph.from_edges(s, (s + np.tile(np.arange(1, w + 1), n)) % n)
+    else:
+        g = dm.Graph.generate(dm.GEN_ER, 60_000, 300_000, seed=3)
+    s, t = g.edges()
+    deg = np.bincount(np.concatenate([s, t]))
+    assert int(np.minimum(deg[s], deg[t]).sum()) >= 500_000  # the shards' line
+    want = orc.near_cliques(_og(orc, g), 4)
+    for o in (None, dm.Options(threads=256)):
+        assert dm.count_near_cliques(g, 4, o)[0] == want
+    assert sum(dm.count_near_cliques(g, 4, dm.Options(rank=r, world_size=3))[0] for r in range(3)) == want
+
+
+@pytest.mark.parametrize("n,m", [(20_000, 80_000), (50_000, 900_000)])
+def test_near_cliques_of_sparse_graphs(dm, orc, gpu, n, m):
+    """Light items: claims of up to 32 edges whose candidates are searched together, most of them with
+    too few; a few dense spots among them."""
+    rng = np.random.default_rng(n)
+    s, t = [rng.integers(0, n, m)], [rng.integers(0, n, m)]
+    for _ in range(40):
+        ids = rng.choice(n, 9, replace=False)
+        a, b = np.triu_indices(9, 1)
+        s.append(ids[a])
+        t.append(ids[b])
+    g = dm.Graph.from_edges(np.concatenate(s), np.concatenate(t))
+    assert g.info().max_degree <= 128
+    og = _og(orc, g)
+    for q in (5, 6, 9):
+        want = orc.near_cliques(og, q)
+        assert dm.count_near_cliques(g, q)[0] == want
+        assert sum(dm.count_near_cliques(g, q, dm.Options(rank=r, world_size=3))[0] for r in range(3)) == want
