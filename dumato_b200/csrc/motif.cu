@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(32 * MOTIF_WARPS, motif_min_blocks(K)) motif_k
   const size_t warp_bit_words = (size_t)c.bit_words * motif_bit_stride(K) * (32 / W);
   uint32_t* sbits = reinterpret_cast<uint32_t*>(wbase + motif_warp_smem<K, W>() * MOTIF_WARPS);
   for (int cl = threadIdx.x; cl < a.n_classes; cl += blockDim.x) bhist[cl] = 0;
+  motif_zero_sweeps<K, W>(ws);
   if (a.bits_smem)
     for (size_t i = threadIdx.x; i < warp_bit_words * MOTIF_WARPS; i += blockDim.x) sbits[i] = 0u;
   __syncthreads();

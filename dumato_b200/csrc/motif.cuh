@@ -118,6 +118,15 @@ __host__ __device__ constexpr size_t motif_warp_smem() {
   return sizeof(MotifShared) + (sizeof(MotifGroup) + sizeof(MotifSweep<K>) + sizeof(MotifLists<W>)) * (32 / W);
 }
 
+// Zeroes a warp's sweep counters (all 32 lanes; every sweep leaves them zero). Once per launch where the
+// memory holds nothing else, else before each task.
+template <int K, int W>
+__device__ __forceinline__ void motif_zero_sweeps(MotifShared* ws) {
+  unsigned* const s = reinterpret_cast<unsigned*>(reinterpret_cast<MotifGroup*>(ws + 1) + 32 / W);
+  for (int i = lane_id(); i < (int)(sizeof(MotifSweep<K>) / sizeof(unsigned)) * (32 / W); i += 32) s[i] = 0u;
+  __syncwarp();
+}
+
 // Everything a motif task needs besides its own (v0, range) or prefix.
 struct MotifCtx {
   GraphView g;                 // undirected CSR, rows sorted
@@ -294,11 +303,7 @@ __device__ __forceinline__ unsigned long long leaf_sweep(const MotifCtx& c, cons
   }
   if (c.sym && i0 < n) mask_hist<W>(E, i0, n, sw->rest, gl, gmask);
   __syncwarp(gmask);
-  // every (a, b) to a lane
-  for (int ab = gl; ab < MASKS * MASKS; ab += W) {
-    const int a = ab / MASKS, b = ab % MASKS;
-    const unsigned ra = sw->swept[a];
-    if (ra == 0) continue;
+  auto settle = [&](int a, int b, unsigned ra) {
     unsigned long long pairs = 0;
     if (c.sym) {
       const unsigned long long rb = sw->swept[b];
@@ -306,15 +311,34 @@ __device__ __forceinline__ unsigned long long leaf_sweep(const MotifCtx& c, cons
       else if (b > a) pairs = (unsigned long long)ra * rb;
       pairs += (unsigned long long)ra * sw->rest[b];
     }
-    const unsigned join = sw->joined[ab];
+    const unsigned join = sw->joined[a * MASKS + b];
     // (a pair joined in the order (a, b) may have been counted in the other order, or in another
     // range of E: the difference may be negative here, the class total is not)
     if (pairs != join) hist.add(__ldg(c.q2c + code(a, b)), pairs - join);
     if (join) {
-      sw->joined[ab] = 0u;
+      sw->joined[a * MASKS + b] = 0u;
       hist.add(__ldg(c.q2c + code(a, b | (1 << P))), (unsigned long long)join);
     }
     counted += pairs;
+  };
+  if constexpr (MASKS * MASKS <= 4 * W) {
+    // every (a, b) to a lane
+    for (int ab = gl; ab < MASKS * MASKS; ab += W) {
+      const unsigned ra = sw->swept[ab / MASKS];
+      if (ra) settle(ab / MASKS, ab % MASKS, ra);
+    }
+  } else {
+    // only the masks that were swept (few of them: most sets are small), their b over the lanes: up to
+    // 1,024 pairs were looked at per prefix for k = 7
+    unsigned present = 0;
+#pragma unroll
+    for (int m = 0; m < MASKS; m += W)
+      present |= (__ballot_sync(gmask, m + gl < MASKS && sw->swept[m + gl] != 0u) >> gsrc) << m;
+    for (; present; present &= present - 1) {
+      const int a = __ffs(present) - 1;
+      const unsigned ra = sw->swept[a];
+      for (int b = gl; b < MASKS; b += W) settle(a, b, ra);
+    }
   }
   for (int a = gl; a < MASKS; a += W) {
     const unsigned fr = sw->fresh[a];
@@ -451,7 +475,7 @@ __device__ __forceinline__ void leaf_pairs(const MotifCtx& c, unsigned* mh, cons
 
 // Runs one task on the calling warp (all 32 lanes). level 0: second vertices [bb, ee) of v0
 // (task_range encoding); level L >= 1: replay path[0..L-1], then expand positions [bb, ee) of
-// E_L (group 0 only). Adds the task's subgraphs to hist; nodes counts expansions (every
+// E_L (group 0 only). The sweep counters are zero (motif_zero_sweeps). Adds the task's subgraphs to hist; nodes counts expansions (every
 // lane of a group counts the same nodes; the caller keeps group leaders' counts only).
 template <int K, int W>
 __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHist& hist, MotifShared* ws,
@@ -504,7 +528,6 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHis
     sg->quick[0] = 0;
     sg->spill_lo = sg->spill_hi = 0;
   }
-  for (int m = gl; m < (int)(sizeof(MotifSweep<K>) / sizeof(unsigned)); m += W) reinterpret_cast<unsigned*>(sw)[m] = 0u;
   if constexpr (use_bits)
     for (int i = gl; i < n0; i += W) bits.set(__ldg(E0 + i), 0);
   MotifDemand dm;  // group leader
