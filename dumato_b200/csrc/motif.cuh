@@ -73,7 +73,6 @@ struct alignas(16) MotifSweep {
   static constexpr int MASKS = 1 << (K > 3 ? K - 2 : 2);
   unsigned swept[MASKS], rest[MASKS], fresh[MASKS];
   unsigned joined[K > 3 ? MASKS * MASKS : 1];
-  unsigned mh[8];              // k = 3: leaf-mask histogram
 };
 
 // 64-bit class counters: in shared memory (w, as pairs of 32-bit words, low word first: a 64-bit
@@ -115,13 +114,16 @@ struct alignas(16) MotifLists {
 // A warp's shared memory: MotifShared | a MotifGroup, a MotifSweep and a MotifLists per group.
 template <int K, int W>
 __host__ __device__ constexpr size_t motif_warp_smem() {
-  return sizeof(MotifShared) + (sizeof(MotifGroup) + sizeof(MotifSweep<K>) + sizeof(MotifLists<W>)) * (32 / W);
+  // (k = 3 sweeps nothing and keeps no lists)
+  return sizeof(MotifShared) +
+         (sizeof(MotifGroup) + (K > 3 ? sizeof(MotifSweep<K>) + sizeof(MotifLists<W>) : 0)) * (32 / W);
 }
 
 // Zeroes a warp's sweep counters (all 32 lanes; every sweep leaves them zero). Once per launch where the
 // memory holds nothing else, else before each task.
 template <int K, int W>
 __device__ __forceinline__ void motif_zero_sweeps(MotifShared* ws) {
+  if constexpr (K == 3) return;
   unsigned* const s = reinterpret_cast<unsigned*>(reinterpret_cast<MotifGroup*>(ws + 1) + 32 / W);
   for (int i = lane_id(); i < (int)(sizeof(MotifSweep<K>) / sizeof(unsigned)) * (32 / W); i += 32) s[i] = 0u;
   __syncwarp();
@@ -354,21 +356,6 @@ __device__ __forceinline__ unsigned long long leaf_sweep(const MotifCtx& c, cons
   return counted;
 }
 
-// k = 3: flushes the group's leaf-mask histogram (masks below 4) into the class counters.
-template <int W>
-__device__ __forceinline__ void flush_masks(unsigned* mh, const int32_t* q2c, const ClassHist& hist,
-                                            unsigned long long& task_cnt, int gl, unsigned gmask) {
-  for (int m = gl; m < 4; m += W) {
-    const unsigned c = mh[m];
-    if (c) {
-      mh[m] = 0;
-      hist.add(__ldg(q2c + m), (unsigned long long)c);
-      task_cnt += c;
-    }
-  }
-  __syncwarp(gmask);
-}
-
 // The group leader's view of the demand for work: the hungry and queued counters as loaded at the
 // previous check. The loads complete while the group works on, so a check never waits for them.
 struct MotifDemand {
@@ -432,45 +419,44 @@ __device__ __forceinline__ void motif_donate(const LBArgs& lb, MotifShared* ws, 
   }
 }
 
-// k = 3: the subgraphs (v0, w, x) with w the member of E_0 = N(v0) above v0 at index it.
+// k = 3: the subgraphs (v0, w, x) with w the member of E_0 = N(v0) above v0 at index it, by leaf mask
+// m in s[m - 1]. A lane's own sums may be negative; the group's are the counts. One pass over E_0 or
+// over N(w) above v0, whichever searches less, gives both the neighbours of w in E_0 and those of them
+// after w. The lanes meet after every search: drifting apart they loaded one row in more and smaller pieces
+// (k = 3 of a Chung-Lu graph of 18,700 vertices with groups of 8 / 16 / 32 lanes: 1.83 / 1.38 / 0.82 ms per
+// call with a pass for each and no meeting, 0.62 / 0.50 / 0.54 now).
 template <int W>
-__device__ __forceinline__ void leaf_pairs(const MotifCtx& c, unsigned* mh, const int32_t* E0, int n0, int it, int v0,
-                                           const ClassHist& hist, unsigned long long& task_cnt, int gl,
-                                           unsigned gmask) {
+__device__ __forceinline__ void leaf_pairs(const MotifCtx& c, const int32_t* E0, int n0, int it, int v0, int gl,
+                                           unsigned gmask, long long (&s)[3]) {
   const int w = __ldg(E0 + it);
   const int32_t* Nw = c.g.adj + __ldg(c.g.row + w);
   const int dw = __ldg(c.g.deg + w);
-  const int start = it + 1, n_inh = n0 - start;
   const int sw0 = lower_bound(Nw, 0, dw, v0 + 1);
   const int above = dw - sw0;
-  const int gt = lower_bound(Nw, 0, dw, w + 1);
-  const int dgt = dw - gt;
-  // members of E_0 after w that are adjacent to w: probe each of them in N(w), or each
-  // neighbour above w in E_0, whichever side is cheaper
-  unsigned adj = 0;
-  if ((long long)dgt * ilog2p1(n_inh) < (long long)n_inh * ilog2p1(dw)) {
-    for (int i = gt + gl; i < dw; i += W) adj += contains(E0 + start, n_inh, Nw[i]) ? 1u : 0u;
+  int adj = 0, inter = 0;
+  if ((long long)n0 * ilog2p1(above) <= (long long)above * ilog2p1(n0)) {
+    for (int i0 = 0; i0 < n0; i0 += W) {
+      const int i = i0 + gl;
+      if (i < n0 && contains(Nw + sw0, above, __ldg(E0 + i))) {
+        ++inter;
+        adj += i > it ? 1 : 0;
+      }
+      __syncwarp(gmask);
+    }
   } else {
-    for (int i = start + gl; i < n0; i += W) adj += contains(Nw, dw, __ldg(E0 + i)) ? 1u : 0u;
+    for (int i0 = sw0; i0 < dw; i0 += W) {
+      const int i = i0 + gl;
+      const int x = i < dw ? Nw[i] : 0;
+      if (i < dw && contains(E0, n0, x)) {
+        ++inter;
+        adj += x > w ? 1 : 0;
+      }
+      __syncwarp(gmask);
+    }
   }
-  // new vertices: N(w) above v0 minus N(v0)
-  unsigned inter = 0;
-  if (n0 <= above) {
-    for (int i = gl; i < n0; i += W) inter += contains(Nw, dw, __ldg(E0 + i)) ? 1u : 0u;
-  } else {
-    for (int i = sw0 + gl; i < dw; i += W) inter += contains(E0, n0, Nw[i]) ? 1u : 0u;
-  }
-  for (int o = W / 2; o > 0; o >>= 1) {
-    adj += __shfl_xor_sync(gmask, adj, o);
-    inter += __shfl_xor_sync(gmask, inter, o);
-  }
-  if (gl == 0) {
-    mh[1] = (unsigned)n_inh - adj;
-    mh[2] = (unsigned)above - inter;
-    mh[3] = adj;
-  }
-  __syncwarp(gmask);
-  flush_masks<W>(mh, c.q2c, hist, task_cnt, gl, gmask);
+  s[0] += (gl == 0 ? n0 - it - 1 : 0) - adj;
+  s[1] += (gl == 0 ? above : 0) - inter;
+  s[2] += adj;
 }
 
 // Runs one task on the calling warp (all 32 lanes). level 0: second vertices [bb, ee) of v0
@@ -508,6 +494,7 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHis
   auto ext_of = [&](int t) -> int2* { return t == K - 3 && top_small ? sl->ext : ext_at(t); };
   auto run_of = [&](int t) -> int* { return t == K - 3 && top_small ? sl->run : run_at(t); };
   unsigned long long task_cnt = 0;
+  long long pairs3[3] = {0, 0, 0};  // k = 3
   const long long t_start = global_ns();
   // E_0 = run 0 = N(v0) above v0: a suffix of the sorted CSR row
   const int32_t* row0 = c.g.adj + __ldg(c.g.row + v0);
@@ -531,7 +518,10 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHis
   if constexpr (use_bits)
     for (int i = gl; i < n0; i += W) bits.set(__ldg(E0 + i), 0);
   MotifDemand dm;  // group leader
-  if (gl == 0) motif_sample(c.lb, dm);
+  if (K > 3 && gl == 0) motif_sample(c.lb, dm);
+  // k = 3: no look at the demand before a donation is allowed, then one every 2,048 cycles (a look waits
+  // for words that every idle warp polls)
+  long long look = clock64() + (c.lb.donate_after_ns == 0 ? 0 : 2 * c.lb.donate_after_ns);
   unsigned long long checked = nodes;
   __syncwarp();
   // drops the bits of levels from..bdepth (the group's lanes, then a group barrier)
@@ -570,8 +560,17 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHis
           if (sg->spill_lo < sg->spill_hi) it = sg->spill_lo++;
         } else if (sg->spill_lo >= sg->spill_hi) {
           int ob = 0, oe = 0;
-          if (motif_wanted(c.lb, ws, dm, t_start) &&
-              range_split_donate(c.lb, &ws->range, v0, &ws->donations_left, &ws->busy, ob, oe, n0, 0, 0, nullptr)) {
+          bool kept = false;
+          if constexpr (K == 3) {
+            if (clock64() >= look) {
+              kept = range_maybe_donate(c.lb, &ws->range, v0, &ws->donations_left, t_start, &ws->busy, ob, oe, n0);
+              look = clock64() + (c.lb.donate_after_ns == 0 ? 0 : 2048);
+            }
+          } else {
+            kept = motif_wanted(c.lb, ws, dm, t_start) &&
+                   range_split_donate(c.lb, &ws->range, v0, &ws->donations_left, &ws->busy, ob, oe, n0, 0, 0, nullptr);
+          }
+          if (kept) {
             sg->spill_lo = ob;
             sg->spill_hi = oe;
           }
@@ -583,7 +582,7 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHis
     if constexpr (K == 3) {
       ++nodes;
       if (gl == 0 && (nodes & 255) == 0) atomicAdd(&c.lb.ctr->progress, 256ull);
-      leaf_pairs<W>(c, sw->mh, E0, n0, it, v0, hist, task_cnt, gl, gmask);
+      leaf_pairs<W>(c, E0, n0, it, v0, gl, gmask, pairs3);
     } else {
       // prefix (v0, w1); the members of E_0 after w1 are the inherited part
       int t = 0;
@@ -753,6 +752,16 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHis
   if constexpr (use_bits)
     for (int i = gl; i < n0; i += W) bits.clear(__ldg(E0 + i), 0);
   __syncwarp();
+  if constexpr (K == 3) {
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const unsigned long long x = warp_sum_u64((unsigned long long)pairs3[m]);
+      if (lane == 0 && x) {
+        hist.add(__ldg(c.q2c + m + 1), x);
+        task_cnt += x;
+      }
+    }
+  }
   if (c.per_root) {
     const unsigned long long tsum = warp_sum_u64(task_cnt);
     if (lane == 0 && tsum) atomicAdd(c.per_root + v0, tsum);
