@@ -24,8 +24,12 @@ struct MotifArgs {
   int bits_smem;               // the bitmaps live in shared memory (zeroed at launch), not in `bits`
 };
 
-// Shared-memory budget of one block's vertex bitmaps (three blocks per SM then still fit; up to
-// 13,800 vertices for k <= 5, 9,200 above); larger graphs keep them in global memory.
+// Shared-memory budget of one block's vertex bitmaps (for 32 lanes, graphs of up to 13,800 vertices for
+// k <= 5, 9,200 above); larger graphs keep them in global memory. Three blocks per SM fit beside them for
+// k = 5 with 32 lanes; k = 6 from 50 KB of bitmaps on, k = 7 and narrower groups (whose state takes 28
+// to 95 KB of a block) run with two, which is still faster than bitmaps in global memory: k = 7,
+// random graph of 8,000 / 10,000, 32 lanes 1.61 ms with two blocks, 1.80 with three and global ones;
+// k = 6, 9,000 / 16,000 1.18 and 1.24; k = 6, 2,000 / 6,000, 8 lanes 4.98 and 5.86.
 constexpr size_t MOTIF_SMEM_BITS_MAX = 54 * 1024;
 
 // Blocks per SM the registers are sized for: three for k >= 5 (80 registers; with four, 64 registers

@@ -59,3 +59,20 @@ def test_near_cliques_of_wide_universes(dm, orc, gpu, q):
     assert dm.count_near_cliques(g, q)[0] == want
     assert sum(dm.count_near_cliques(g, q, dm.Options(rank=r, world_size=3))[0] for r in range(3)) == want
     assert dm.count_near_cliques(g, q, dm.Options(threads=256))[0] == want
+
+
+@pytest.mark.parametrize("vwarp,blades", [(8, 20), (16, 20), (32, 130)])
+def test_seven_vertices_of_a_windmill(dm, gpu, vwarp, blades):
+    """k = 7 sets of up to 2 blades - 4 members, more than 255 (where the 16-bit pair counters are left
+    out) or fewer, with joined pairs: triangles sharing one vertex. A connected 7-subgraph is the
+    centre and six rim vertices with j of the rim edges: C(b, j) C(b - j, 6 - 2j) 2^(6 - 2j) of them."""
+    from math import comb
+
+    rim = 1 + np.arange(2 * blades)
+    u = np.concatenate([np.zeros(2 * blades, int), rim[::2]])
+    v = np.concatenate([rim, rim[1::2]])
+    g = dm.Graph.from_edges(u, v)
+    d = dm.Dictionary.generate(7)
+    got, _ = dm.count_motifs(g, 7, d, dm.Options(vwarp=vwarp))
+    want = [comb(blades, j) * comb(blades - j, 6 - 2 * j) * 2 ** (6 - 2 * j) for j in range(4)]
+    assert sorted(int(x) for x in got if x) == sorted(want)
