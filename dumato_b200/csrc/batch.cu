@@ -511,7 +511,7 @@ int dm_batch_create(const dm_query* queries, int32_t n, const dm_opts* opts, int
   for (size_t i = 0; i < roots.size(); ++i) hroots[i] = roots[i].second;
   if (padj.empty()) padj.assign(4, INT32_MAX);
   auto upload = [&](void** dst, const void* src, size_t bytes) -> int {
-    DM_CUDA(cudaMalloc(dst, std::max<size_t>(bytes, 16)));
+    DM_CUDA(device_alloc(dst, std::max<size_t>(bytes, 16)));
     if (bytes) DM_CUDA(cudaMemcpyAsync(*dst, src, bytes, cudaMemcpyHostToDevice, b->stream));
     return DM_OK;
   };
@@ -575,13 +575,13 @@ int dm_batch_create(const dm_query* queries, int32_t n, const dm_opts* opts, int
     const int thr = desc[i].trigger;
     desc[i].trigger = thr >= 100 ? 0 : std::max(1, (thr * warps + 99) / 100);
   }
-  ce = cudaMalloc(&b->d_arena, arena_bytes * (size_t)warps);
+  ce = device_alloc(reinterpret_cast<void**>(&b->d_arena), arena_bytes * (size_t)warps);
   if (ce != cudaSuccess)
     return fail_release(b, fail(DM_ECUDA, std::string("dm_batch_create: arena: ") + cudaGetErrorString(ce)));
   // vertex bitmaps of the motif queries, per warp (zeroed here; every task leaves them zero)
   if (bits_words) {
     b->bits_bytes = bits_words * sizeof(uint32_t) * (size_t)warps;
-    ce = cudaMalloc(&b->d_bits, b->bits_bytes);
+    ce = device_alloc(reinterpret_cast<void**>(&b->d_bits), b->bits_bytes);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(b->d_bits, 0, b->bits_bytes, b->stream);
     if (ce != cudaSuccess)
       return fail_release(b, fail(DM_ECUDA, std::string("dm_batch_create: bitmaps: ") + cudaGetErrorString(ce)));

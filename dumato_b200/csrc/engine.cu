@@ -22,6 +22,7 @@
 #include <thread>
 #include <vector>
 
+#include "buf_pool.hpp"
 #include "engine.hpp"
 #include "lb.cuh"
 
@@ -393,46 +394,86 @@ static DeviceSlot* slot_for(dm_graph* g, int dev) {
   return s;
 }
 
-// Device buffers owned by graphs (CSR copies, root orders, the clique index) go back to a
-// per-device pool when a graph's device copy is released, and the next upload of the same
-// or another graph takes them from there (best fit, at most twice the size asked for), so
-// re-uploading a graph costs copies, not cudaMalloc/cudaFree. The pool holds at most 4 GB.
+// Device buffers owned by graphs (CSR copies, root orders, the clique index) and by a file being read go
+// back to a per-device pool, and the next upload of the same or another graph takes them from there, so
+// re-uploading a graph costs copies, not cudaMalloc/cudaFree. A pool holds at most 4 GB. It and the
+// kept workspaces are given back when an allocation of this library finds no room.
 static std::mutex g_buf_mu;
-static std::map<void*, size_t> g_buf_size;
-static std::map<int, std::multimap<size_t, void*>> g_buf_pool;
-static size_t g_buf_pooled = 0;
+static std::map<int, BufPool> g_buf_pool;
 constexpr size_t BUF_POOL_MAX = (size_t)4 << 30;
+
+// (g_buf_mu held)
+static BufPool& buf_pool(int dev) {
+  auto it = g_buf_pool.find(dev);
+  if (it == g_buf_pool.end())
+    it = g_buf_pool
+             .emplace(dev, BufPool(
+                               BUF_POOL_MAX,
+                               [](void** p, size_t n) {
+                                 const cudaError_t e = cudaMalloc(p, n);
+                                 if (e != cudaSuccess) cudaGetLastError();
+                                 return (int)e;
+                               },
+                               [](void* p) { cudaFree(p); }))
+             .first;
+  return it->second;
+}
+
+// Frees the workspaces kept for the next graph; false when there were none.
+static bool drop_workspaces(int dev) {
+  std::vector<Workspace> kept;
+  {
+    std::lock_guard<std::mutex> lk(g_dev_mu);
+    kept.swap(g_ws_pool[dev]);
+  }
+  for (Workspace& w : kept) free_workspace(w);
+  return !kept.empty();
+}
 
 cudaError_t gbuf_alloc(void** p, size_t bytes) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   bytes = (std::max<size_t>(bytes, 256) + 255) / 256 * 256;
-  std::lock_guard<std::mutex> lk(g_buf_mu);
-  auto& pool = g_buf_pool[dev];
-  auto it = pool.lower_bound(bytes);
-  if (it != pool.end() && it->first <= 2 * bytes) {
-    *p = it->second;
-    g_buf_pooled -= it->first;
-    pool.erase(it);
-    return cudaSuccess;
+  for (int again = 0;; ++again) {
+    {
+      std::lock_guard<std::mutex> lk(g_buf_mu);
+      e = (cudaError_t)buf_pool(dev).take(p, bytes);
+    }
+    if (e != cudaErrorMemoryAllocation || again || !drop_workspaces(dev)) return e;
   }
-  e = cudaMalloc(p, bytes);
-  if (e == cudaSuccess) g_buf_size[*p] = bytes;
-  return e;
 }
 
 void gbuf_free(void* p, int dev) {
   if (!p) return;
   std::lock_guard<std::mutex> lk(g_buf_mu);
-  auto it = g_buf_size.find(p);
-  if (it != g_buf_size.end() && g_buf_pooled + it->second <= BUF_POOL_MAX) {
-    g_buf_pool[dev].insert({it->second, p});
-    g_buf_pooled += it->second;
-    return;
+  if (!buf_pool(dev).give(p)) cudaFree(p);
+}
+
+cudaError_t device_alloc(void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaSuccess) return e;
+  int dev = 0;
+  if (e == cudaErrorMemoryAllocation && cudaGetDevice(&dev) == cudaSuccess) {
+    {
+      std::lock_guard<std::mutex> lk(g_buf_mu);
+      if (buf_pool(dev).drop()) e = cudaMalloc(p, bytes);
+    }
+    if (e == cudaErrorMemoryAllocation && drop_workspaces(dev)) e = cudaMalloc(p, bytes);
   }
-  if (it != g_buf_size.end()) g_buf_size.erase(it);
-  cudaFree(p);
+  cudaGetLastError();  // (the failed attempts leave theirs behind)
+  if (e != cudaSuccess) *p = nullptr;
+  return e;
+}
+
+cudaError_t device_room(size_t* bytes) {
+  size_t total = 0;
+  int dev = 0;
+  cudaError_t e = cudaMemGetInfo(bytes, &total);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(g_buf_mu);
+  if (e == cudaSuccess) *bytes += buf_pool(dev).pooled();
+  return e;
 }
 
 // Page-locked staging for one-off transfers of pageable host memory (a graph's first upload, a
@@ -643,7 +684,11 @@ static int ensure_ws_bytes(void** p, size_t* cap, size_t want) {
   *p = nullptr;
   *cap = 0;
   size_t alloc = want + want / 4 + 256;
-  DM_CUDA(cudaMalloc(p, alloc));
+  cudaError_t e = device_alloc(p, alloc);
+  if (e == cudaErrorMemoryAllocation) e = device_alloc(p, alloc = want);  // no room to grow into
+  if (e != cudaSuccess)
+    return fail(e == cudaErrorMemoryAllocation ? DM_ENOMEM : DM_ECUDA,
+                std::string("device workspace: ") + cudaGetErrorString(e));
   *cap = alloc;
   return DM_OK;
 }
@@ -938,8 +983,8 @@ static int ensure_index(dm_graph* g, DeviceSlot* s, LaunchCtx& ctx) {
   const size_t bytes = (size_t)total * 16;
   bool fits = total < INDEX_NONE;
   if (fits && bytes > ((size_t)256 << 20)) {
-    size_t free_b = 0, tot_b = 0;
-    DM_CUDA(cudaMemGetInfo(&free_b, &tot_b));
+    size_t free_b = 0;
+    DM_CUDA(device_room(&free_b));
     fits = bytes <= std::min<size_t>((size_t)8 << 30, free_b / 4);
   }
   if (!fits) {
@@ -1817,8 +1862,8 @@ int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_
   const int bit_words = motif_bit_words(g->n);
   const size_t warp_bits = sizeof(uint32_t) * motif_warp_bit_words(k, bit_words, vwarp);
   if (warp_bits * ctx.arena_warps > ((size_t)2 << 30)) {
-    size_t free_b = 0, tot_b = 0;
-    DM_CUDA(cudaMemGetInfo(&free_b, &tot_b));
+    size_t free_b = 0;
+    DM_CUDA(device_room(&free_b));
     const size_t room = std::max<size_t>(ws.bits_cap, std::min<size_t>((size_t)8 << 30, free_b / 4));
     ctx.arena_warps = (int)std::min<size_t>(ctx.arena_warps, std::max<size_t>(8, room / warp_bits));
   }
@@ -1828,7 +1873,7 @@ int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_
     cudaFree(ws.d_bits);
     ws.d_bits = nullptr;
     ws.bits_cap = 0;
-    DM_CUDA(cudaMalloc(&ws.d_bits, bits_bytes));
+    DM_CUDA(device_alloc(reinterpret_cast<void**>(&ws.d_bits), bits_bytes));
     ws.bits_cap = bits_bytes;
     DM_CUDA(cudaMemsetAsync(ws.d_bits, 0, bits_bytes, ctx.stream));
   }

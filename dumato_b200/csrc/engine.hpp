@@ -289,6 +289,10 @@ int check_opts(const dm_opts* o);
 // Device buffers from the library's per-device pool (current device; safe from any thread). A
 // buffer is given back only once nothing on the device uses it any more.
 cudaError_t gbuf_alloc(void** p, size_t bytes);
+// cudaMalloc that releases the pooled buffers and tries again when the device has no room (no error is
+// left behind), and the bytes such allocations can have: free ones and pooled ones.
+cudaError_t device_alloc(void** p, size_t bytes);
+cudaError_t device_room(size_t* bytes);
 void gbuf_free(void* p, int dev);
 // Transfers of pageable host memory through pooled page-locked buffers (engine.cu), on `st`.
 struct Staging {
@@ -328,6 +332,8 @@ constexpr int QUEUE_SHARD_SLOTS = 2048; // slots per shard
 #define DM_CUDA(call)                                                              \
   do {                                                                             \
     cudaError_t e_ = (call);                                                       \
-    if (e_ != cudaSuccess)                                                         \
+    if (e_ != cudaSuccess) {                                                       \
+      cudaGetLastError(); /* (else the next call's launch check would find it) */  \
       return ::dmb::fail(DM_ECUDA, std::string(#call " failed: ") + cudaGetErrorString(e_)); \
+    }                                                                              \
   } while (0)
