@@ -569,22 +569,28 @@ int dm_batch_create(const dm_query* queries, int32_t n, const dm_opts* opts, int
   const size_t warps_fit =
       std::max<size_t>(BATCH_WARPS, budget / std::max(arena_bytes, bits_words * sizeof(uint32_t)));
   b->grid = std::max(1, std::min(b->grid, (int)(warps_fit / BATCH_WARPS)));
+  // the arena, and the motif queries' vertex bitmaps per warp (zeroed here; every task leaves them zero):
+  // for half as many blocks where the device has no room
+  while (true) {
+    const size_t warps = (size_t)b->grid * BATCH_WARPS;
+    b->bits_bytes = bits_words * sizeof(uint32_t) * warps;
+    ce = device_alloc(reinterpret_cast<void**>(&b->d_arena), arena_bytes * warps);
+    if (ce == cudaSuccess && bits_words) ce = device_alloc(reinterpret_cast<void**>(&b->d_bits), b->bits_bytes);
+    if (ce == cudaSuccess) break;
+    cudaFree(b->d_arena);
+    b->d_arena = nullptr;
+    if (ce != cudaErrorMemoryAllocation || b->grid == 1)
+      return fail_release(b, fail(ce == cudaErrorMemoryAllocation ? DM_ENOMEM : DM_ECUDA,
+                                  std::string("dm_batch_create: workspace: ") + cudaGetErrorString(ce)));
+    b->grid /= 2;
+  }
+  if (bits_words && (ce = cudaMemsetAsync(b->d_bits, 0, b->bits_bytes, b->stream)) != cudaSuccess)
+    return fail_release(b, fail(DM_ECUDA, std::string("dm_batch_create: bitmaps: ") + cudaGetErrorString(ce)));
   const int warps = b->grid * BATCH_WARPS;
   // a threshold is a percentage of the warps (>= 100: this query never donates)
   for (int32_t i = 0; i < n; ++i) {
     const int thr = desc[i].trigger;
     desc[i].trigger = thr >= 100 ? 0 : std::max(1, (thr * warps + 99) / 100);
-  }
-  ce = device_alloc(reinterpret_cast<void**>(&b->d_arena), arena_bytes * (size_t)warps);
-  if (ce != cudaSuccess)
-    return fail_release(b, fail(DM_ECUDA, std::string("dm_batch_create: arena: ") + cudaGetErrorString(ce)));
-  // vertex bitmaps of the motif queries, per warp (zeroed here; every task leaves them zero)
-  if (bits_words) {
-    b->bits_bytes = bits_words * sizeof(uint32_t) * (size_t)warps;
-    ce = device_alloc(reinterpret_cast<void**>(&b->d_bits), b->bits_bytes);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(b->d_bits, 0, b->bits_bytes, b->stream);
-    if (ce != cudaSuccess)
-      return fail_release(b, fail(DM_ECUDA, std::string("dm_batch_create: bitmaps: ") + cudaGetErrorString(ce)));
   }
   BatchArgs& a = b->args;
   a.g = GraphView{b->d_row, b->d_deg, b->d_adj, (int32_t)total_v};

@@ -1622,7 +1622,11 @@ int dm_count_near_cliques(dm_graph* g, int32_t n, const dm_opts* o, uint64_t* co
     L.arena_ints = ((size_t)L.list_cap + (size_t)g->near_rows + 63) / 64 * 64;
     const size_t per_warp = L.arena_ints * sizeof(int32_t);
     ctx.arena_warps = (int)std::min<size_t>((size_t)ctx.num_sms * 64, std::max<size_t>(8, ((size_t)8 << 30) / per_warp));
-    if ((rc = ensure_ws_bytes(&ws.d_scratch, &ws.scratch_cap, per_warp * ctx.arena_warps))) return rc;
+    // (a launch with half as many warps where the device has no room, down to one block)
+    while ((rc = ensure_ws_bytes(&ws.d_scratch, &ws.scratch_cap, per_warp * ctx.arena_warps)) == DM_ENOMEM &&
+           ctx.arena_warps > 8)
+      ctx.arena_warps = std::max(8, ctx.arena_warps / 2);
+    if (rc) return rc;
     L.arena = reinterpret_cast<int32_t*>(ws.d_scratch);
   }
   if (items == 0) std::memset(ws.h_out, 0, sizeof(DevCounters));  // no launch
@@ -1743,6 +1747,80 @@ static int motif_census(dm_graph* g, int k, const dm_dictionary* dict, const int
   return DM_OK;
 }
 
+// Vertex bitmaps beyond BITS_KEEP are given back at the end of the call.
+constexpr size_t BITS_KEEP = (size_t)8 << 30;
+struct FreeLargeBits {
+  Workspace& ws;
+  ~FreeLargeBits() {
+    if (ws.bits_cap <= BITS_KEEP) return;
+    cudaFree(ws.d_bits);
+    ws.d_bits = nullptr;
+    ws.bits_cap = 0;
+  }
+};
+
+// The motif kernel's per-warp memory: extension levels and runs (at most 8 GB), and vertex bitmaps, zero
+// between calls, for as many warps as the launch keeps on the device (ctx.arena_warps) - or as
+// there is room for. Past BITS_KEEP a warp is one group (each has bitmaps of its own), and past half of
+// the free memory warps are cut. 5-vertex motifs of a random graph of 24,000,000 / 29,000,000 (43 GB
+// of bitmaps for all warps) took 694 ms in the 712 warps of an 8 GB limit, now 208 (171 of them the
+// kernel, the rest allocating); 60,000,000 / 70,000,000 550 ms. Binary searches instead of bitmaps took
+// 256 and 592. When an allocation fails all the same (another owner), the launch shrinks further, down
+// to one block.
+static int motif_workspace(Workspace& ws, int k, int maxdeg, int bit_words, int n_classes, LaunchCtx& ctx, int* vwarp) {
+  constexpr int BLOCK_WARPS = 8;
+  int rc, limit = INT_MAX;
+  while (true) {
+    int warps = 0;
+    size_t warp_bits = 0;
+    if ((rc = motif_warps(k, *vwarp, n_classes, bit_words, ctx, &warps, &warp_bits))) return rc;
+    const size_t per_warp = motif_arena_stride(k, maxdeg, *vwarp) * sizeof(int2);
+    auto cap = [&](size_t n) { warps = (int)std::min<size_t>(warps, std::max<size_t>(BLOCK_WARPS, n)); };
+    cap(((size_t)8 << 30) / per_warp);
+    if (warp_bits * warps > ((size_t)2 << 30) && warp_bits * warps > ws.bits_cap) {
+      size_t room = 0;
+      DM_CUDA(device_room(&room));
+      room = std::max(ws.bits_cap, (room + ws.bits_cap) / 2);
+      if (warp_bits * warps > std::min(room, BITS_KEEP) && *vwarp < 32) {
+        *vwarp = 32;
+        continue;
+      }
+      // (up to twice BITS_KEEP stay within it: half the warps cost less than allocating every time)
+      cap((warp_bits * warps <= 2 * BITS_KEEP ? std::min(room, BITS_KEEP) : room) / warp_bits);
+    }
+    cap((size_t)limit);
+    const size_t bits_bytes = warp_bits * warps;
+    rc = ensure_ws_bytes(&ws.d_scratch, &ws.scratch_cap, per_warp * warps);
+    cudaError_t e = cudaSuccess;
+    if (!rc && ws.bits_cap < bits_bytes) {
+      cudaFree(ws.d_bits);
+      ws.d_bits = nullptr;
+      ws.bits_cap = 0;
+      e = device_alloc(reinterpret_cast<void**>(&ws.d_bits), bits_bytes);
+      if (e == cudaSuccess) {
+        ws.bits_cap = bits_bytes;
+        DM_CUDA(cudaMemsetAsync(ws.d_bits, 0, bits_bytes, ctx.stream));
+      }
+    }
+    if (!rc && e == cudaSuccess) {
+      ctx.arena_warps = warps;
+      return DM_OK;
+    }
+    if (rc && rc != DM_ENOMEM) return rc;
+    if (e != cudaSuccess && e != cudaErrorMemoryAllocation)
+      return fail(DM_ECUDA, std::string("motif bitmaps: ") + cudaGetErrorString(e));
+    // no room: everything of this call's is freed and half as many warps tried
+    cudaFree(ws.d_scratch);
+    cudaFree(ws.d_bits);
+    ws.d_scratch = nullptr;
+    ws.d_bits = nullptr;
+    ws.scratch_cap = ws.bits_cap = 0;
+    if (warps > BLOCK_WARPS) limit = std::max(BLOCK_WARPS, warps / 2 / BLOCK_WARPS * BLOCK_WARPS);
+    else if (*vwarp < 32) *vwarp = 32;
+    else return fail(DM_ENOMEM, "no device memory for one block of the motif kernel");
+  }
+}
+
 int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_opts* o, uint64_t* class_counts,
                     dm_stats* st) {
   if (!g || !dict || !class_counts) return fail(DM_EINVAL, "dm_count_motifs: null argument");
@@ -1850,33 +1928,11 @@ int dm_count_motifs(dm_graph* g, int32_t k, const dm_dictionary* dict, const dm_
                             sizeof(unsigned long long) * dict->n_classes)))
     return rc;
   DM_CUDA(cudaMemsetAsync(ws.d_hist, 0, sizeof(unsigned long long) * dict->n_classes, ctx.stream));
-  // arena: extension levels and runs per warp
   const int maxdeg = std::max(g->max_degree, 1);
-  const int vwarp = (ctx.vwarp == 8 || ctx.vwarp == 16) ? ctx.vwarp : 32;
-  const size_t per_warp = motif_arena_stride(k, maxdeg, vwarp) * sizeof(int2);
-  const size_t budget = (size_t)8 << 30;
-  // (the kernel keeps at most 32 warps per SM)
-  ctx.arena_warps = (int)std::min<size_t>((size_t)ctx.num_sms * 32, std::max<size_t>(8, budget / per_warp));
-  // vertex bitmaps, zero between calls; past 2 GB they get up to a quarter of the free memory (at
-  // most 8 GB), and the launch as many warps as that holds
   const int bit_words = motif_bit_words(g->n);
-  const size_t warp_bits = sizeof(uint32_t) * motif_warp_bit_words(k, bit_words, vwarp);
-  if (warp_bits * ctx.arena_warps > ((size_t)2 << 30)) {
-    size_t free_b = 0;
-    DM_CUDA(device_room(&free_b));
-    const size_t room = std::max<size_t>(ws.bits_cap, std::min<size_t>((size_t)8 << 30, free_b / 4));
-    ctx.arena_warps = (int)std::min<size_t>(ctx.arena_warps, std::max<size_t>(8, room / warp_bits));
-  }
-  if ((rc = ensure_ws_bytes(&ws.d_scratch, &ws.scratch_cap, per_warp * ctx.arena_warps))) return rc;
-  const size_t bits_bytes = warp_bits * ctx.arena_warps;
-  if (ws.bits_cap < bits_bytes) {
-    cudaFree(ws.d_bits);
-    ws.d_bits = nullptr;
-    ws.bits_cap = 0;
-    DM_CUDA(device_alloc(reinterpret_cast<void**>(&ws.d_bits), bits_bytes));
-    ws.bits_cap = bits_bytes;
-    DM_CUDA(cudaMemsetAsync(ws.d_bits, 0, bits_bytes, ctx.stream));
-  }
+  int vwarp = (ctx.vwarp == 8 || ctx.vwarp == 16) ? ctx.vwarp : 32;
+  FreeLargeBits large_bits{ws};
+  if ((rc = motif_workspace(ws, k, maxdeg, bit_words, dict->n_classes, ctx, &vwarp))) return rc;
   const bool want_log = o && o->subtree_counts;
   if (want_log) {
     if ((rc = ensure_ws_bytes(reinterpret_cast<void**>(&ws.d_per_root), &ws.per_root_cap,

@@ -256,6 +256,8 @@ struct MotifLaunch {
 inline int motif_bit_words(int n) { return (n + 31) / 32 + 1; }
 int motif_launch(const MotifLaunch& L, LaunchCtx& ctx, int* grid);
 size_t motif_warp_bit_words(int k, int bit_words, int vwarp);  // words of vertex bitmaps per warp
+// Warps that a launch keeps on the device at once, and the bytes of bitmaps each needs in global memory.
+int motif_warps(int k, int vwarp, int n_classes, int bit_words, const LaunchCtx& ctx, int* warps, size_t* warp_bits);
 size_t motif_arena_stride(int k, int maxdeg, int vwarp);  // int2 slots per warp
 
 const char* cuda_err_str(cudaError_t e);

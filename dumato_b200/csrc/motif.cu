@@ -115,28 +115,67 @@ size_t motif_arena_stride(int k, int maxdeg, int vwarp) {
   return motif_group_stride(k, maxdeg) * (size_t)(32 / w);
 }
 
+// Launch shape of one kernel: blocks that the device holds at once (within dm_opts.threads), dynamic shared
+// memory, and whether the bitmaps are part of it.
+struct MotifShape {
+  int grid = 0;
+  size_t smem = 0;
+  bool bits_smem = false;
+};
+
 template <int K, int W>
-static int launch_motif(MotifArgs a, LaunchCtx& ctx, int* grid_out) {
+static int motif_shape(int n_classes, int bit_words, const LaunchCtx& ctx, MotifShape* s) {
   const int block = 32 * MOTIF_WARPS;
-  const size_t bits_bytes = (size_t)a.c.bit_words * motif_bit_stride(K) * (32 / W) * sizeof(uint32_t) * MOTIF_WARPS;
-  a.bits_smem = K >= 4 && bits_bytes <= MOTIF_SMEM_BITS_MAX ? 1 : 0;
-  const size_t smem = sizeof(unsigned long long) * ((a.n_classes + 1) & ~1) +
-                      motif_warp_smem<K, W>() * MOTIF_WARPS + (a.bits_smem ? bits_bytes : 0);
-  auto kern = motif_kernel<K, W>;
+  const size_t bits_bytes = (size_t)bit_words * motif_bit_stride(K) * (32 / W) * sizeof(uint32_t) * MOTIF_WARPS;
+  s->bits_smem = K >= 4 && bits_bytes <= MOTIF_SMEM_BITS_MAX;
+  s->smem = sizeof(unsigned long long) * ((n_classes + 1) & ~1) + motif_warp_smem<K, W>() * MOTIF_WARPS +
+            (s->bits_smem ? bits_bytes : 0);
   static LaunchCache cache;
   int occ = 0;
-  DM_CUDA(cached_occupancy(cache, kern, ctx.device, block, smem, &occ));
+  DM_CUDA(cached_occupancy(cache, motif_kernel<K, W>, ctx.device, block, s->smem, &occ));
   if (occ < 1) return fail(DM_EINVAL, "motif kernel does not fit on an SM");
-  int grid = ctx.num_sms * occ;
-  if (ctx.threads > 0) grid = std::max(1, std::min(grid, (ctx.threads + block - 1) / block));
+  s->grid = ctx.num_sms * occ;
+  if (ctx.threads > 0) s->grid = std::max(1, std::min(s->grid, (ctx.threads + block - 1) / block));
+  return DM_OK;
+}
+
+template <int K, int W>
+static int launch_motif(MotifArgs a, LaunchCtx& ctx, int* grid_out) {
+  MotifShape s;
+  int rc = motif_shape<K, W>(a.n_classes, a.c.bit_words, ctx, &s);
+  if (rc) return rc;
+  a.bits_smem = s.bits_smem ? 1 : 0;
+  int grid = s.grid;
   if (grid * MOTIF_WARPS > ctx.arena_warps) grid = std::max(1, ctx.arena_warps / MOTIF_WARPS);
   const int warps = grid * MOTIF_WARPS;
   a.c.lb.hungry_trigger = ctx.threshold >= 100 ? 0 : std::max(1, (ctx.threshold * warps + 99) / 100);
-  kern<<<grid, block, smem, ctx.stream>>>(a);
+  motif_kernel<K, W><<<grid, 32 * MOTIF_WARPS, s.smem, ctx.stream>>>(a);
   ctx.launches++;
   *grid_out = grid;
   DM_CUDA(cudaGetLastError());
   return DM_OK;
+}
+
+template <int K>
+static int warps_motif(int vwarp, int n_classes, int bit_words, const LaunchCtx& ctx, int* warps, size_t* warp_bits) {
+  MotifShape s;
+  const int rc = vwarp == 8    ? motif_shape<K, 8>(n_classes, bit_words, ctx, &s)
+                 : vwarp == 16 ? motif_shape<K, 16>(n_classes, bit_words, ctx, &s)
+                               : motif_shape<K, 32>(n_classes, bit_words, ctx, &s);
+  *warps = s.grid * MOTIF_WARPS;
+  *warp_bits = s.bits_smem ? 0 : sizeof(uint32_t) * motif_warp_bit_words(K, bit_words, vwarp);
+  return rc;
+}
+
+int motif_warps(int k, int vwarp, int n_classes, int bit_words, const LaunchCtx& ctx, int* warps, size_t* warp_bits) {
+  switch (k) {
+    case 3: return warps_motif<3>(vwarp, n_classes, bit_words, ctx, warps, warp_bits);
+    case 4: return warps_motif<4>(vwarp, n_classes, bit_words, ctx, warps, warp_bits);
+    case 5: return warps_motif<5>(vwarp, n_classes, bit_words, ctx, warps, warp_bits);
+    case 6: return warps_motif<6>(vwarp, n_classes, bit_words, ctx, warps, warp_bits);
+    case 7: return warps_motif<7>(vwarp, n_classes, bit_words, ctx, warps, warp_bits);
+    default: return fail(DM_EINVAL, "motif k must be in [3, 7]");
+  }
 }
 
 template <int K>

@@ -67,7 +67,50 @@ def test_pooled_buffers_are_given_back(dm, gpu, tmp_path):
         got, st = dm.count_motifs(g, 5, d)
     g.release_device()
     want, full = dm.count_motifs(g, 5, d)
-    assert np.array_equal(got, want)
+    assert st.grid == full.grid and np.array_equal(got, want)
+
+
+def test_motif_launch_shrinks_to_the_memory_left(dm, gpu, drop_kept):
+    """1.8 GB of bitmaps for all warps at 32 lanes (four times that at 8), 900 MB left."""
+    g = dm.Graph.generate(dm.GEN_ER, 1_000_000, 1_100_000, seed=2)
+    for k in (5, 6):
+        d = dm.Dictionary.generate(k)
+        want, full = dm.count_motifs(g, k, d)
+        for vwarp in (32, 8):
+            g.release_device()
+            drop_kept()
+            with little_memory(900 << 20):
+                got, st = dm.count_motifs(g, k, d, dm.Options(vwarp=vwarp))
+            assert st.grid < full.grid and np.array_equal(got, want), (k, vwarp)
+
+
+def test_batch_shrinks_to_the_memory_left(dm, gpu, drop_kept):
+    d = dm.Dictionary.generate(5)
+    g = dm.Graph.generate(dm.GEN_ER, 1_000_000, 1_100_000, seed=3)
+    h = dense(dm, 300, 0.2)
+    queries = [dm.Query(dm.QUERY_MOTIF, 5, g, d), dm.Query(dm.QUERY_CLIQUE, 5, h)]
+    b = dm.Batch(queries)
+    want, full = b.run()
+    b.close()
+    drop_kept()
+    with little_memory(900 << 20):
+        b = dm.Batch(queries)
+        got, st = b.run()
+        b.close()
+    assert st.grid < full.grid
+    assert np.array_equal(got[0], want[0]) and got[1] == want[1]
+
+
+def test_near_cliques_shrink_to_the_memory_left(dm, gpu, drop_kept):
+    """600 MB of rows for all warps on a complete graph of 700 vertices."""
+    from math import comb
+
+    g = dense(dm, 700, 1.1)
+    want = comb(700, 3) * comb(697, 2)
+    drop_kept()
+    with little_memory(300 << 20):
+        got, st = dm.count_near_cliques(g, 5)
+    assert got == want
 
 
 def test_failed_allocation_leaves_no_error_behind(dm, orc, gpu, drop_kept):
