@@ -506,7 +506,11 @@ Stager::Stager(int device, cudaStream_t st) : dev_(device), st_(st) {
     }
     if (!s_.pinned && !(s_.buf[i] = std::malloc(STAGE_BYTES))) err_ = cudaErrorMemoryAllocation;
   }
-  for (int i = 0; i < 2 && err_ == cudaSuccess; ++i) err_ = cudaEventCreateWithFlags(&s_.ev[i], cudaEventDisableTiming);
+  for (int i = 0; i < 2 && err_ == cudaSuccess; ++i) {
+    err_ = cudaEventCreateWithFlags(&s_.ev[i], cudaEventDisableTiming);
+    for (cudaEvent_t* e : {&s_.beg[i], &s_.end[i]})
+      if (err_ == cudaSuccess) err_ = cudaEventCreate(e);
+  }
 }
 
 Stager::~Stager() {
@@ -521,7 +525,8 @@ Stager::~Stager() {
   }
   for (int i = 0; i < 2; ++i) {
     if (s_.busy[i]) cudaEventSynchronize(s_.ev[i]);
-    if (s_.ev[i]) cudaEventDestroy(s_.ev[i]);
+    for (cudaEvent_t e : {s_.ev[i], s_.beg[i], s_.end[i]})
+      if (e) cudaEventDestroy(e);
     if (s_.pinned) cudaFreeHost(s_.buf[i]);
     else std::free(s_.buf[i]);
   }
@@ -531,7 +536,15 @@ Stager::~Stager() {
 cudaError_t Stager::wait(int i) {
   if (err_ == cudaSuccess && s_.busy[i]) err_ = cudaEventSynchronize(s_.ev[i]);
   s_.busy[i] = false;
+  float ms = 0.f;
+  if (timed_[i] && err_ == cudaSuccess && cudaEventElapsedTime(&ms, s_.beg[i], s_.end[i]) == cudaSuccess) ms_ += ms;
+  timed_[i] = false;
   return err_;
+}
+
+float Stager::copy_ms() {
+  for (int i = 0; i < 2; ++i) wait(i);
+  return ms_;
 }
 
 cudaError_t Stager::sent(int i) {
@@ -540,6 +553,7 @@ cudaError_t Stager::sent(int i) {
   return err_;
 }
 
+// (got: the timed form)
 cudaError_t Stager::upload(void* dst, size_t bytes, const std::function<size_t(void*, size_t)>& fill, size_t* got) {
   size_t off = 0;
   while (off < bytes && err_ == cudaSuccess) {
@@ -549,8 +563,12 @@ cudaError_t Stager::upload(void* dst, size_t bytes, const std::function<size_t(v
     const size_t want = std::min(STAGE_BYTES, bytes - off);
     const size_t n = fill(s_.buf[i], want);
     if (n) {
-      err_ = cudaMemcpyAsync(static_cast<char*>(dst) + off, s_.buf[i], n, cudaMemcpyHostToDevice, st_);
+      if (got) err_ = cudaEventRecord(s_.beg[i], st_);
+      if (err_ == cudaSuccess)
+        err_ = cudaMemcpyAsync(static_cast<char*>(dst) + off, s_.buf[i], n, cudaMemcpyHostToDevice, st_);
+      if (got && err_ == cudaSuccess) err_ = cudaEventRecord(s_.end[i], st_);
       sent(i);
+      timed_[i] = got != nullptr;
       off += n;
     }
     if (n < want) break;

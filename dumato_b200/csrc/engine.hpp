@@ -300,6 +300,7 @@ void gbuf_free(void* p, int dev);
 struct Staging {
   void* buf[2] = {nullptr, nullptr};
   cudaEvent_t ev[2] = {nullptr, nullptr};  // the last copy from or into the buffer
+  cudaEvent_t beg[2] = {nullptr, nullptr}, end[2] = {nullptr, nullptr};  // its times, where it is timed
   bool busy[2] = {false, false};
   bool pinned = true;
 };
@@ -311,10 +312,12 @@ class Stager {
   Stager& operator=(const Stager&) = delete;
   // The source may change as soon as the call returns; the destination is written in stream order.
   cudaError_t upload(void* dst, const void* src, size_t bytes);
-  // fill(buf, n) writes up to n bytes and returns how many (fewer end the upload); *got: the total
+  // fill(buf, n) writes up to n bytes and returns how many (fewer end the upload); *got: the total. These
+  // copies are timed: copy_ms() is their device time, once the stream has been waited for.
   cudaError_t upload(void* dst, size_t bytes, const std::function<size_t(void*, size_t)>& fill, size_t* got);
   // The destination is complete when the call returns.
   cudaError_t download(void* dst, const void* src, size_t bytes);
+  float copy_ms();
 
  private:
   cudaError_t wait(int i);
@@ -323,6 +326,8 @@ class Stager {
   cudaStream_t st_;
   Staging s_;
   int next_ = 0;
+  bool timed_[2] = {false, false};
+  float ms_ = 0.f;
   cudaError_t err_ = cudaSuccess;
 };
 int queue_init_launch(void* queue, int nq, int cap, cudaStream_t st);  // empty donation queue

@@ -92,3 +92,66 @@ def test_device_ingest_staging_edges(dm, gpu, tmp_path, size):
     for _ in range(2):  # staged first upload, then the page-locked one
         assert dm.count_cliques(g, 3)[0] == dm.count_cliques(h, 3)[0]
         g.release_device()
+
+
+SLOW_READS = r"""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <stdio.h>
+#include <unistd.h>
+static FILE* sought;
+size_t fread(void* p, size_t s, size_t n, FILE* f) {
+  static size_t (*real)(void*, size_t, size_t, FILE*);
+  if (!real) real = (size_t(*)(void*, size_t, size_t, FILE*))dlsym(RTLD_NEXT, "fread");
+  if (s * n >= 1 << 20) usleep(150000);
+  return real(p, s, n, f);
+}
+size_t __fread_chk(void* p, size_t room, size_t s, size_t n, FILE* f) { return fread(p, s, n, f); }
+int fseek(FILE* f, long o, int w) {
+  static int (*real)(FILE*, long, int);
+  if (!real) real = (int (*)(FILE*, long, int))dlsym(RTLD_NEXT, "fseek");
+  sought = f;
+  return real(f, o, w);
+}
+int fclose(FILE* f) {
+  static int (*real)(FILE*);
+  if (!real) real = (int (*)(FILE*))dlsym(RTLD_NEXT, "fclose");
+  if (f == sought) sought = NULL;
+  return real(f);
+}
+int setvbuf(FILE* f, char* b, int m, size_t n) {
+  static int (*real)(FILE*, char*, int, size_t);
+  if (!real) real = (int (*)(FILE*, char*, int, size_t))dlsym(RTLD_NEXT, "setvbuf");
+  if (f == sought) fputs("late setvbuf\n", stderr);
+  return real(f, b, m, n);
+}
+"""
+
+
+def test_device_ms_leaves_out_the_reads(dm, gpu, tmp_path):
+    """On a disk that takes 150 ms for each of the file's four pieces the call takes 0.6 s, device_ms
+    does not; and the stream's buffering is chosen before its first use."""
+    import os
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+
+    shim, path = tmp_path / "slow.so", tmp_path / "slow.edgelist"
+    (tmp_path / "slow.c").write_text(SLOW_READS)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(shim), str(tmp_path / "slow.c"), "-ldl"], check=True)
+    rng = np.random.default_rng(4)
+    np.savetxt(path, rng.integers(100_000, 999_999, (1_000_000, 2)), fmt="%d")
+    assert 3 << 22 < path.stat().st_size < 4 << 22
+    code = ("import sys, time, dumato_b200 as dm\n"
+            "for _ in range(3):\n"
+            "    t = time.perf_counter()\n"
+            "    g, ms = dm.Graph.load_edgelist_device(sys.argv[1])\n"
+            "    print(g.info().n_edges, ms, 1e3 * (time.perf_counter() - t))\n")
+    res = subprocess.run([sys.executable, "-c", code, str(path)], cwd=ROOT, capture_output=True, text=True,
+                         timeout=120, env=dict(os.environ, LD_PRELOAD=str(shim)))
+    assert res.returncode == 0, res.stderr
+    assert "late setvbuf" not in res.stderr
+    edges, device_ms, total_ms = map(float, res.stdout.splitlines()[-1].split())
+    assert edges > 990_000
+    assert total_ms >= 600 and 0 < device_ms < 150
