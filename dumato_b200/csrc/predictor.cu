@@ -984,7 +984,10 @@ int dm_predictor_train(dm_predictor* p, const float* X, const float* T, int64_t 
   const float b1 = 0.9f, b2 = 0.999f;
   std::vector<float> bias(2 * (size_t)steps);
   for (int ep = 0; ep < epochs; ++ep) {
-    // (the device still runs the previous epoch: its indices are in the other buffer)
+    // (while the device still runs the previous epoch, whose indices are in the other device buffer. idx
+    // and bias may change: a copy from pageable memory returns once it has left for the driver's own
+    // staging memory. Page-locked buffers of ours with an event each made the host wait for the epoch
+    // before: 300 rows, 4 epochs 132 -> 196 us.)
     for (int64_t i = n - 1; i > 0; --i) {
       s = g_pred_seed_mix(s);
       std::swap(idx[i], idx[s % (uint64_t)(i + 1)]);

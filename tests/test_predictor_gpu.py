@@ -189,3 +189,24 @@ def test_training_matches_float64_adam(dm, gpu, n, batch):
             p = p - lr * (m / (1 - b1 ** steps)) / (np.sqrt(v / (1 - b2 ** steps)) + 1e-8)
     assert np.abs(pr.get_params() - p).max() <= 1e-3 * lr * steps + 1e-6
     assert abs(loss - total / n) <= 1e-4 * max(1.0, total / n)
+
+
+def test_training_of_many_rows(dm, gpu):
+    """Index lists longer than a staging piece (4 MiB), shuffled again on the host while the device trains on
+    the previous order: several epochs equal the launches' form (batches above 4,096) step for step, up
+    to FP32 sums in another order, and a second run of the same."""
+    rng = np.random.default_rng(8)
+    n = 1_500_000
+    X = rng.normal(size=(n, F)).astype(np.float32)
+    T = (X[:, 0] - 0.5 * X[:, 3]).astype(np.float32)
+
+    def train(batch):
+        pr = dm.Predictor(seed=5)
+        loss = pr.train(X, T, epochs=4, batch=batch, lr=1e-3)
+        return pr.get_params(), loss
+
+    (a, la), (b, lb) = train(4096), train(4096)
+    assert np.array_equal(a, b) and abs(la - lb) <= 1e-4 * la  # (the loss alone is added atomically)
+    c, lc = train(4097)
+    # one sample in a batch of 4,097 apart, and steps of 1e-3: the losses of both runs meet
+    assert abs(la - lc) <= 0.05 * max(la, lc)
