@@ -69,7 +69,8 @@ struct CensusArgs {
 // ---------------- in-lists (laid out once per device copy) ----------------
 
 __global__ void __launch_bounds__(256) in_count_kernel(GraphView g, int32_t* __restrict__ deg) {
-  const int r = (blockIdx.x * 256 + threadIdx.x) >> 3, l = threadIdx.x & 7;
+  // (eight threads per rank: beyond 32 bits from 2^29 ranks on)
+  const int r = (int)((blockIdx.x * 256ll + threadIdx.x) >> 3), l = threadIdx.x & 7;
   if (r >= g.n) return;
   const int32_t* L = g.adj + g.row[r];
   for (int i = l; i < g.deg[r]; i += 8) atomicAdd(deg + L[i], 1);
@@ -95,7 +96,8 @@ __global__ void __launch_bounds__(256) in_place_kernel(const int32_t* __restrict
 
 __global__ void __launch_bounds__(256) in_fill_kernel(GraphView g, int32_t* __restrict__ pos,
                                                       InEdge* __restrict__ in) {
-  const int r = (blockIdx.x * 256 + threadIdx.x) >> 3, l = threadIdx.x & 7;
+  // (eight threads per rank: beyond 32 bits from 2^29 ranks on)
+  const int r = (int)((blockIdx.x * 256ll + threadIdx.x) >> 3), l = threadIdx.x & 7;
   if (r >= g.n) return;
   const int b = g.row[r];
   for (int i = l; i < g.deg[r]; i += 8) in[atomicAdd(pos + g.adj[b + i], 1)] = make_int2(r, b + i);
