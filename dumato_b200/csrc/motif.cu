@@ -21,6 +21,7 @@ struct MotifArgs {
   int2* arena;                 // per warp: 32/W group arenas of c.arena_stride int2
   uint32_t* bits;              // per warp: 32/W groups x motif_bit_stride(k) bitmaps of c.bit_words (k >= 4)
   const int32_t* parts;        // optional per-root-entry part word (p | P << 16)
+  int hist_smem;               // block-level class counters in shared memory (else straight to hist)
   int bits_smem;               // the bitmaps live in shared memory (zeroed at launch), not in `bits`
 };
 
@@ -43,14 +44,15 @@ template <int K, int W>
 __global__ void __launch_bounds__(32 * MOTIF_WARPS, motif_min_blocks(K)) motif_kernel(const __grid_constant__ MotifArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   unsigned long long* bhist = reinterpret_cast<unsigned long long*>(smem);
-  unsigned char* wbase = smem + sizeof(unsigned long long) * ((a.n_classes + 1) & ~1);
+  const int n_bhist = a.hist_smem ? a.n_classes : 0;
+  unsigned char* wbase = smem + sizeof(unsigned long long) * ((n_bhist + 1) & ~1);
   const int lane = lane_id();
   const int wib = warp_in_block();
   MotifShared* ws = reinterpret_cast<MotifShared*>(wbase + motif_warp_smem<K, W>() * wib);
   const MotifCtx& c = a.c;
   const size_t warp_bit_words = (size_t)c.bit_words * motif_bit_stride(K) * (32 / W);
   uint32_t* sbits = reinterpret_cast<uint32_t*>(wbase + motif_warp_smem<K, W>() * MOTIF_WARPS);
-  for (int cl = threadIdx.x; cl < a.n_classes; cl += blockDim.x) bhist[cl] = 0;
+  for (int cl = threadIdx.x; cl < n_bhist; cl += blockDim.x) bhist[cl] = 0;
   motif_zero_sweeps<K, W>(ws);
   if (a.bits_smem)
     for (size_t i = threadIdx.x; i < warp_bit_words * MOTIF_WARPS; i += blockDim.x) sbits[i] = 0u;
@@ -90,7 +92,7 @@ __global__ void __launch_bounds__(32 * MOTIF_WARPS, motif_min_blocks(K)) motif_k
       if (!donated && a.parts) part_bounds(__ldg(a.parts + first + ti), bb, ee);
       ++ntasks;
       // block-level class counters, added to the global ones at exit
-      motif_run_task<K, W>(c, ClassHist{reinterpret_cast<unsigned*>(bhist), nullptr}, ws, warp_arena, warp_bits, v0, bb, ee, level, path, nodes);
+      motif_run_task<K, W>(c, ClassHist{a.hist_smem ? reinterpret_cast<unsigned*>(bhist) : nullptr, a.hist}, ws, warp_arena, warp_bits, v0, bb, ee, level, path, nodes);
     }
     if (lane == 0) lb_done(c.lb, count);
   }
@@ -101,7 +103,7 @@ __global__ void __launch_bounds__(32 * MOTIF_WARPS, motif_min_blocks(K)) motif_k
     atomicAdd(&c.lb.ctr->nodes, nodes);
   }
   __syncthreads();
-  for (int cl = threadIdx.x; cl < a.n_classes; cl += blockDim.x)
+  for (int cl = threadIdx.x; cl < n_bhist; cl += blockDim.x)
     if (bhist[cl]) atomicAdd(a.hist + cl, bhist[cl]);
 }
 
@@ -116,20 +118,25 @@ size_t motif_arena_stride(int k, int maxdeg, int vwarp) {
 }
 
 // Launch shape of one kernel: blocks that the device holds at once (within dm_opts.threads), dynamic shared
-// memory, and whether the bitmaps are part of it.
+// memory, and whether the bitmaps and the block's class counters are part of it (a table of any number of
+// classes is counted: one that leaves no room for the warps' state adds to global memory).
 struct MotifShape {
   int grid = 0;
   size_t smem = 0;
   bool bits_smem = false;
+  bool hist_smem = true;
 };
 
 template <int K, int W>
 static int motif_shape(int n_classes, int bit_words, const LaunchCtx& ctx, MotifShape* s) {
   const int block = 32 * MOTIF_WARPS;
   const size_t bits_bytes = (size_t)bit_words * motif_bit_stride(K) * (32 / W) * sizeof(uint32_t) * MOTIF_WARPS;
-  s->bits_smem = K >= 4 && bits_bytes <= MOTIF_SMEM_BITS_MAX;
-  s->smem = sizeof(unsigned long long) * ((n_classes + 1) & ~1) + motif_warp_smem<K, W>() * MOTIF_WARPS +
-            (s->bits_smem ? bits_bytes : 0);
+  constexpr size_t SMEM_MAX = 227 * 1024, state = motif_warp_smem<K, W>() * MOTIF_WARPS;
+  const size_t hist = sizeof(unsigned long long) * (((size_t)n_classes + 1) & ~(size_t)1);
+  s->hist_smem = hist + state <= SMEM_MAX;
+  s->smem = (s->hist_smem ? hist : 0) + state;
+  s->bits_smem = K >= 4 && bits_bytes <= MOTIF_SMEM_BITS_MAX && s->smem + bits_bytes <= SMEM_MAX;
+  if (s->bits_smem) s->smem += bits_bytes;
   static LaunchCache cache;
   int occ = 0;
   DM_CUDA(cached_occupancy(cache, motif_kernel<K, W>, ctx.device, block, s->smem, &occ));
@@ -145,6 +152,7 @@ static int launch_motif(MotifArgs a, LaunchCtx& ctx, int* grid_out) {
   int rc = motif_shape<K, W>(a.n_classes, a.c.bit_words, ctx, &s);
   if (rc) return rc;
   a.bits_smem = s.bits_smem ? 1 : 0;
+  a.hist_smem = s.hist_smem ? 1 : 0;
   int grid = s.grid;
   if (grid * MOTIF_WARPS > ctx.arena_warps) grid = std::max(1, ctx.arena_warps / MOTIF_WARPS);
   const int warps = grid * MOTIF_WARPS;
@@ -208,7 +216,7 @@ int motif_launch(const MotifLaunch& L, LaunchCtx& ctx, int* grid) {
   a.hist = L.hist;
   a.arena = reinterpret_cast<int2*>(L.arena);
   a.parts = L.parts;
-  a.bits_smem = 0;
+  a.bits_smem = a.hist_smem = 0;
   const int w = (L.vwarp == 8 || L.vwarp == 16) ? L.vwarp : 32;
   switch (L.k) {
     case 3: return launch_motif_w<3>(a, w, ctx, grid);

@@ -76,3 +76,19 @@ def test_seven_vertices_of_a_windmill(dm, gpu, vwarp, blades):
     got, _ = dm.count_motifs(g, 7, d, dm.Options(vwarp=vwarp))
     want = [comb(blades, j) * comb(blades - j, 6 - 2 * j) * 2 ** (6 - 2 * j) for j in range(4)]
     assert sorted(int(x) for x in got if x) == sorted(want)
+
+
+@pytest.mark.parametrize("k,vwarp", [(6, 8), (6, 32), (7, 32), (7, 8)])
+def test_tables_with_a_class_per_code(dm, orc, gpu, tmp_path, k, vwarp):
+    """Hand-made tables of 16,384 classes (k = 6), and of 30,000 (k = 7), whose block counters leave no
+    shared memory for the bitmaps, or none for themselves: looked up code by code as the oracle does."""
+    nq = 1 << (k * (k - 1) // 2 - 1)
+    nc = min(nq, 30_000)
+    q2c = (np.arange(nq) % nc).astype(np.int32)
+    p = tmp_path / f"{k}.csv"
+    p.write_text(f"#quick,cg_local\n{nq}\n" + "".join(f"{q},{c}\n" for q, c in enumerate(q2c)) +
+                 f"#cg_local,cg_global\n{nc}\n" + "".join(f"{c},{c}\n" for c in range(nc)))
+    d = dm.Dictionary.load_csv(p)
+    g = graph(dm, "core")
+    want = orc.motifs(orc.OracleGraph.from_pairs(*g.edges()), k, q2c, nc)
+    assert np.array_equal(dm.count_motifs(g, k, d, dm.Options(vwarp=vwarp))[0], want)
