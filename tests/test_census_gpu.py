@@ -83,16 +83,17 @@ def test_census_vs_closed_form_and_enumeration(dm, orc, gpu, name):
         assert np.array_equal(got, again)
 
 
-@pytest.mark.parametrize("n,m,hub", [(230_000, 500_000, 0), (80_000, 150_000, 70_000)])
+@pytest.mark.parametrize("n,m,hub", [(230_000, 500_000, 0), (230_000, 500_000, 9_000), (80_000, 150_000, 70_000)])
 def test_census_counter_windows(dm, orc, gpu, n, m, hub):
-    """More ranks than one window of counters holds; a degree of 65,536 or more (32-bit counters)."""
+    """No vertex for the block counters; a hub whose counters take several windows (16 bits); a degree of
+    65,536 or more (32-bit counters, two windows)."""
     rng = np.random.default_rng(n)
     s, t = rng.integers(0, n, m), rng.integers(0, n, m)
     if hub:
         s, t = np.concatenate([s, np.full(hub, 5)]), np.concatenate([t, 6 + np.arange(hub)])
     g = dm.Graph.from_edges(s, t)
     if hub:
-        assert g.info().max_degree >= 65_536
+        assert (g.info().max_degree >= 65_536) == (hub >= 65_536)
     d = dm.Dictionary.generate(4)
     got, _ = dm.count_motifs(g, 4, d)
     assert types4(dm, orc, got, d) == orc.graphlet4(orc.OracleGraph.from_pairs(*g.edges()))
