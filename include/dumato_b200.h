@@ -101,11 +101,12 @@ typedef struct dm_report {
   double elapsed_ms;           /* host time since the counting kernel was launched */
   int32_t warps;               /* warps of the launch */
   int32_t hungry_warps;        /* warps waiting for work when sampled */
-  int64_t roots_claimed;       /* root tasks dealt to warps so far */
+  int64_t roots_claimed;       /* root tasks dealt to warps so far (near-cliques: roots any of whose
+                                  out-edges is dealt) */
   int64_t roots_total;
   int64_t pending;             /* root and donated tasks not settled */
   uint64_t donations;          /* tasks donated between warps so far */
-  uint64_t progress;           /* work finished (advances while long items run) */
+  uint64_t progress;           /* work finished (advances while long items run; units of the path) */
 } dm_report;
 typedef void (*dm_report_fn)(const dm_report* sample, void* user);
 
@@ -121,7 +122,8 @@ typedef struct dm_opts {
   int32_t vwarp;               /* virtual-warp width 0 (auto), 8, 16 or 32: motifs, the lanes sharing
                                   a task's second vertices per group; cliques, the lanes running one
                                   first-level candidate's DFS on the list path (the bitmap paths run
-                                  one DFS per lane) */
+                                  one DFS per lane). Motifs run with 32 where narrower groups' vertex
+                                  bitmaps exceed 8 GB (dm_stats.vwarp_used tells) */
   int32_t mode;                /* DM_MODE_* */
   int32_t scheduler;           /* DM_SCHED_* */
   int32_t rank;                /* root shard: this process counts roots r with r % world == rank */
@@ -155,7 +157,7 @@ typedef struct dm_opts {
 typedef struct dm_stats {
   double kernel_ms;            /* device time of the counting kernels (CUDA events) */
   double prep_ms;              /* device time of graph upload/orientation/task ordering */
-  uint64_t tasks;              /* root (or donated-prefix) tasks executed */
+  uint64_t tasks;              /* root (or donated-prefix) tasks executed; near-cliques: root tasks */
   uint64_t donations;          /* prefixes donated between warps */
   uint64_t idle_polls;         /* polls by warps that found no work */
   uint64_t nodes;              /* DFS nodes expanded (extend calls) */
@@ -182,8 +184,8 @@ DM_API int dm_graph_load_edgelist(const char* path, dm_graph** out);
    src/main/DuMatoCPU.cu:94-108): the file's bytes are parsed, deduplicated, symmetrised
    and degree-oriented on the device of opts (may be NULL), and the graph is identical to
    dm_graph_load_edgelist's (same CSR, orientation, counts and format errors). Files below
-   2 GiB. *device_ms (may be NULL) receives the device time from the byte upload to the
-   read-back of the CSRs. */
+   2 GiB. *device_ms (may be NULL) receives the device time of the byte upload and of everything
+   from there to the read-back of the CSRs (not the reads of the file between the copies). */
 DM_API int dm_graph_load_edgelist_device(const char* path, const dm_opts* opts, dm_graph** out, double* device_ms);
 DM_API int dm_graph_from_edges(const int32_t* src, const int32_t* dst, int64_t n_pairs,
                         int32_t n_vertices, dm_graph** out);

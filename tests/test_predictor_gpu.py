@@ -192,9 +192,9 @@ def test_training_matches_float64_adam(dm, gpu, n, batch):
 
 
 def test_training_of_many_rows(dm, gpu):
-    """Index lists longer than a staging piece (4 MiB), shuffled again on the host while the device trains on
-    the previous order: several epochs equal the launches' form (batches above 4,096) step for step, up
-    to FP32 sums in another order, and a second run of the same."""
+    """Index lists of 6 MB, shuffled again on the host while the device trains on the previous order: two
+    runs of four epochs give the same weights bit for bit (an order overwritten in flight would not), and
+    the launches' form (batches above 4,096) a loss within 5 %: one sample per batch differs."""
     rng = np.random.default_rng(8)
     n = 1_500_000
     X = rng.normal(size=(n, F)).astype(np.float32)
@@ -208,5 +208,4 @@ def test_training_of_many_rows(dm, gpu):
     (a, la), (b, lb) = train(4096), train(4096)
     assert np.array_equal(a, b) and abs(la - lb) <= 1e-4 * la  # (the loss alone is added atomically)
     c, lc = train(4097)
-    # one sample in a batch of 4,097 apart, and steps of 1e-3: the losses of both runs meet
     assert abs(la - lc) <= 0.05 * max(la, lc)
