@@ -109,7 +109,7 @@ __device__ void batch_motif(const BatchArgs& a, const BatchQuery& q, unsigned ch
   for (int c = lane; c < BATCH_HIST; c += 32) hist[c] = 0ull;
   motif_zero_sweeps<K, W>(ws);
   unsigned long long tn = 0;
-  motif_run_task<K, W>(q.mctx, ClassHist{local ? reinterpret_cast<unsigned*>(hist) : nullptr, q.out}, ws, arena, bits, v0, b, e, level, path, tn);
+  motif_run_task<K, W, false>(q.mctx, ClassHist{local ? reinterpret_cast<unsigned*>(hist) : nullptr, q.out}, ws, arena, bits, v0, b, e, level, path, tn);
   __syncwarp();
   if (local)
     for (int c = lane; c < q.n_classes; c += 32)

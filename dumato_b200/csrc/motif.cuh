@@ -252,7 +252,7 @@ __device__ __noinline__ unsigned long long leaf_ordered(const MotifCtx& c, const
 //
 // Bound by instruction issue: a step of about 40 instructions takes W row entries (an owner
 // search by shuffles, one load of the entry, one lookup in the bitmaps, one ballot).
-template <int K, int W, class Between>
+template <int K, int W, bool ROWS, class Between>
 __device__ __forceinline__ unsigned long long leaf_sweep(const MotifCtx& c, const ClassHist& hist, MotifSweep<K>* sw,
                                                          const int2* E, int n, int lo, const int* lim, int v0,
                                                          unsigned quick_t, const MotifBits<K>& bits, int gl, int gsrc,
@@ -298,7 +298,7 @@ __device__ __forceinline__ unsigned long long leaf_sweep(const MotifCtx& c, cons
     // narrow groups, rows of similar length: a row per lane, which needs no owners (k = 6, random graph of
     // 9,000 / 16,000, 8 lanes: 4.22 -> 3.51 ms; k = 7, 16,000 / 18,000, 16 lanes: 4.46 -> 3.93; k = 5
     // with 16 lanes is no faster by rows)
-    constexpr bool BY_ROW = W == 8 || (W == 16 && K >= 6);
+    constexpr bool BY_ROW = ROWS && (W == 8 || (W == 16 && K >= 6));
     int longest = INT_MAX;
     if constexpr (BY_ROW) {
       longest = len;
@@ -508,9 +508,11 @@ __device__ __forceinline__ void leaf_pairs(const MotifCtx& c, const int32_t* E0,
 
 // Runs one task on the calling warp (all 32 lanes). level 0: second vertices [bb, ee) of v0
 // (task_range encoding); level L >= 1: replay path[0..L-1], then expand positions [bb, ee) of
-// E_L (group 0 only). The sweep counters are zero (motif_zero_sweeps). Adds the task's subgraphs to hist; nodes counts expansions (every
+// E_L (group 0 only). The sweep counters are zero (motif_zero_sweeps). ROWS: narrow groups may sweep a row
+// per lane (the batch kernel, short of registers, leaves that out: k = 4 with 8 lanes 1.15 ms with it,
+// 1.05 without). Adds the task's subgraphs to hist; nodes counts expansions (every
 // lane of a group counts the same nodes; the caller keeps group leaders' counts only).
-template <int K, int W>
+template <int K, int W, bool ROWS = true>
 __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHist& hist, MotifShared* ws,
                                                int2* warp_arena, uint32_t* warp_bits, int v0, int bb, int ee,
                                                int level, const int* path, unsigned long long& nodes) {
@@ -760,7 +762,7 @@ __device__ __forceinline__ void motif_run_task(const MotifCtx& c, const ClassHis
         if (p == K - 3) {
           // the last two vertices in bulk
           int last = first_pos;
-          task_cnt += leaf_sweep<K, W>(c, hist, sw, Ep, m, first_pos, &sg->lim[p], v0, quick_p, bits, gl, gsrc, gmask,
+          task_cnt += leaf_sweep<K, W, ROWS>(c, hist, sw, Ep, m, first_pos, &sg->lim[p], v0, quick_p, bits, gl, gsrc, gmask,
                                        [&](int next) {
                                          const unsigned long long before = nodes;
                                          nodes += (unsigned long long)(next - last);
